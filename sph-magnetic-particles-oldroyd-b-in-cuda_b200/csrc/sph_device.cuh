@@ -39,31 +39,50 @@ __device__ __forceinline__ auto rec_P(const R& r, int q) -> decltype(r.x) {
   if constexpr (DIM == 3) return r.P[q]; else return q < 3 ? r.P[q] : decltype(r.x)(0);
 }
 
-// ---------------------------------------------------------------------------------
-// SPH kernel and its radial derivative (kernel_W.cu:13-59, kernel_gradW.cu:13-53).
-// Written branch-free: the clamped terms are exact zeros where the reference skips
-// them, so the value is the same as the branchy form.
-// ---------------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T sph_w(T r, T rcut_inv, T cw) {
-  T q3 = (r * rcut_inv) * T(3);
-  T t1 = T(3) - q3, t2 = T(2) - q3, t3 = T(1) - q3;
-  T a1 = t1 * t1, a2 = t2 * t2, a3 = t3 * t3;
-  T w = (a1 * a1) * t1;
-  if (q3 < T(2)) w = w - T(6) * ((a2 * a2) * t2);
-  if (q3 < T(1)) w = w + T(15) * ((a3 * a3) * t3);
-  return cw * w;
+// Explicitly rounded operations: the pair sums must give the same bits in every kernel that
+// takes them (one box or many, with or without the minimum image, one or two particles per
+// lane), and the compiler may contract a plain expression differently in each.
+__device__ __forceinline__ double xmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double xadd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float xadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double xfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float xfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// 1 / sqrt(x) of a positive normal x.  FP64: the hardware's seed and one third-order
+// Householder step, y (1 + e (1/2 + 3/8 e)) with e = 1 - x y^2 (the Taylor series of
+// (1 - e)^(-1/2) to second order: the error is 5/16 e^3), without the special cases of the
+// library function, which no pair of distinct particles meets.
+__device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
+__device__ __forceinline__ double inv_sqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
+  return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 
+// c where t >= 0, else 0 (a test of the sign bit; FP64: the constant's high word alone, its
+// low word being zero)
+template <int C>
+__device__ __forceinline__ double where_pos(double t) {
+  return __hiloint2double(__double2hiint(t) < 0 ? 0 : __double2hiint((double)C), 0);
+}
+template <int C>
+__device__ __forceinline__ float where_pos(float t) {
+  return t < 0.0f ? 0.0f : (float)C;
+}
+
+// SPH kernel over its constant, W / cw (kernel_W.cu:13-59; its radial derivative,
+// kernel_gradW.cu:13-53, is in PairRadial): (3 - q)^5 - 6 (2 - q)^5 [q < 2] +
+// 15 (1 - q)^5 [q < 1] with q = 3 r / rcut.  Branch-free: the clamped terms are exact zeros
+// where the reference skips them, so the value is that of the branchy form.
 template <typename T>
-__device__ __forceinline__ T sph_gradw(T r, T rcut_inv, T c_gradw) {
-  T q3 = T(3) * (r * rcut_inv);
-  T t1 = T(3) - q3, t2 = T(2) - q3, t3 = T(1) - q3;
-  T a1 = t1 * t1, a2 = t2 * t2, a3 = t3 * t3;
-  T g = a1 * a1;
-  if (q3 < T(2)) g = g - T(6) * (a2 * a2);
-  if (q3 < T(1)) g = g + T(15) * (a3 * a3);
-  return c_gradw * g;
+__device__ __forceinline__ T sph_w(T r, T rcut_inv3) {
+  const T t1 = xfma(-rcut_inv3, r, T(3)), t2 = xfma(-rcut_inv3, r, T(2)),
+          t3 = xfma(-rcut_inv3, r, T(1));
+  const T a1 = xmul(t1, t1), a2 = xmul(t2, t2), a3 = xmul(t3, t3);
+  return xfma(xmul(where_pos<15>(t3), t3), xmul(a3, a3),
+              xfma(xmul(where_pos<-6>(t2), t2), xmul(a2, a2), xmul(xmul(a1, a1), t1)));
 }
 
 // Minimum image as the reference writes it: subtract L above L/2, add L below -L/2
@@ -467,7 +486,7 @@ __device__ __forceinline__ float4 ld_pos(const float4* a) {
 
 template <typename T, int DIM>
 struct PairParams {
-  T L[3], h[3], rcutsq, rcut_inv, c_gradw, a, b;
+  T L[3], h[3], rcutsq, rcut_inv3, a, b;  // rcut_inv3 = 3 / rcut
   __device__ __forceinline__ void load(const BoxParams& p) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -475,8 +494,7 @@ struct PairParams {
       h[q] = (T)p.halfL[q];
     }
     rcutsq = (T)p.rcutsq;
-    rcut_inv = (T)p.rcut_inv;
-    c_gradw = (T)p.c_gradw;
+    rcut_inv3 = (T)(3.0 * p.rcut_inv);
     a = (T)p.a;
     b = (T)p.b;
   }
@@ -485,75 +503,34 @@ struct PairParams {
 // the target particle i of the pass
 template <typename T, int DIM>
 struct PairOwn {
-  T x, y, z, v[3], invd, press, P[6];
+  T x, y, z, v[3], invd, press;
   int t;
   bool fluid, do_grad, do_force;
 };
 
-// Sums of the float pair terms in mixed precision (density, velocity gradient, forces):
-// kind 1 compensated float sums (Kahan), kind 2 FP64 accumulators of the float terms (kept:
-// more accurate, and at 128^3 the pair pass 2.41 -> 2.39 ms and the density 0.74 -> 0.73 ms,
-// the conversions and FP64 adds running on the otherwise idle FP64 pipe).  FP64 sums stay
-// plain.  S: the accumulator type.
-constexpr int kFloatSums = 2;
+// Sums of a pass over one particle's list.  What is common to every term is left out of the
+// terms and applied when the sums are stored (pair_store): the kernel's factor c_gradw, the
+// particle's own stress term P_i (its part of the force is P_i times the sum s of gw e) and
+// the gradient's -1/d_i.  S: the accumulator type.  The float pair terms of mixed precision
+// are summed in FP64 (more accurate than compensated float sums, and the conversions and
+// FP64 adds run on the otherwise idle FP64 pipe).
 template <typename T>
 struct SumKind {
-  static constexpr int kind = 0;
-  using S = T;
+  using S = double;
 };
-template <>
-struct SumKind<float> {
-  static constexpr int kind = kFloatSums;
-  using S = std::conditional_t<kFloatSums == 2, double, float>;
-};
-template <typename T>
-struct Compensated {
-  static constexpr bool on = SumKind<T>::kind == 1;
-};
-
-// Kahan step: s + c tracks the exact sum of the terms to about one rounding of s.
-__device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
-  const float y = __fsub_rn(x, c);
-  const float t = __fadd_rn(s, y);
-  c = __fsub_rn(__fsub_rn(t, s), y);
-  s = t;
-}
-
 template <typename T, int DIM>
 struct PairAcc {
-  // the sums of float pair terms (mixed precision) are FP64 accumulators, or, in the
-  // compensated form (SumKind kind 1), floats each carrying its rounding error in a second
-  // float (Kahan) that is added back when the sum is stored
   using S = typename SumKind<T>::S;
-  static constexpr bool kComp = Compensated<T>::on;
-  static constexpr bool kTermwise = SumKind<T>::kind != 0;  // a pair's force as one term
-  S g[DIM][DIM];
-  S f[3];
-  T cg[DIM][DIM];
-  T cf[3];
+  S g[DIM][DIM];  // sum of gw e_a v_c
+  S f[DIM];       // force terms but the particle's own stress
+  S s[DIM];       // sum of gw e
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int a = 0; a < DIM; ++a)
+    for (int a = 0; a < DIM; ++a) {
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        g[a][c] = S(0);
-        cg[a][c] = T(0);
-      }
-    f[0] = f[1] = f[2] = S(0);
-    cf[0] = cf[1] = cf[2] = T(0);
-  }
-  // s (with compensation c) += x
-  __device__ __forceinline__ static void add(S& s, T& c, T x) {
-    if constexpr (kComp)
-      kahan_add(s, c, x);
-    else
-      s += (S)x;
-  }
-  __device__ __forceinline__ double grad(int a, int c) const {
-    return kComp ? (double)g[a][c] - (double)cg[a][c] : (double)g[a][c];
-  }
-  __device__ __forceinline__ double force(int a) const {
-    return kComp ? (double)f[a] - (double)cf[a] : (double)f[a];
+      for (int c = 0; c < DIM; ++c) g[a][c] = S(0);
+      f[a] = s[a] = S(0);
+    }
   }
 };
 
@@ -569,8 +546,6 @@ __device__ __forceinline__ void load_own(const Dev& d, int i, int ti, const Rec&
   o.v[2] = (T)rec_vz<DIM>(ri);
   o.invd = ri.invd;
   o.press = (T)d.press[i];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) o.P[q] = rec_P<DIM>(ri, q);
   o.t = type_of(ti);
   o.fluid = o.t == 0;
   // gradient: every particle in kPairGradvAll; in the fused pass fluid particles (whose
@@ -590,89 +565,72 @@ __device__ __forceinline__ T pair_sep(const PairParams<T, DIM>& pp, int wall,
   return norm2(r[0], r[1], r[2], DIM == 3);
 }
 
-// 1/|r|, the kernel slope gw = dW/dr at |r| and the unit vector e = r / |r|.
+// 1/|r| and the vector s = (dW/dr / c_gradw) r / |r|; w = |s| / |r|.
 template <typename T, int DIM>
 struct PairRadial {
-  T rinv, gw, e[3];
+  T rinv, w, s[DIM];
   __device__ __forceinline__ void eval(const PairParams<T, DIM>& pp, T r2, const T r[3]) {
-    rinv = rsqrt(r2);  // r and 1/r from one reciprocal square root
-    const T rr = r2 * rinv;
-    gw = sph_gradw<T>(rr, pp.rcut_inv, pp.c_gradw);
-    e[0] = r[0] * rinv;
-    e[1] = r[1] * rinv;
-    e[2] = DIM == 3 ? r[2] * rinv : T(0);
+    rinv = inv_sqrt(r2);
+    const T rr = xmul(r2, rinv);
+    // (3 - q)^4 - 6 (2 - q)^4 [q < 2] + 15 (1 - q)^4 [q < 1], q = 3 |r| / rcut
+    const T t1 = xfma(-pp.rcut_inv3, rr, T(3)), t2 = xfma(-pp.rcut_inv3, rr, T(2)),
+            t3 = xfma(-pp.rcut_inv3, rr, T(1));
+    const T a1 = xmul(t1, t1), a2 = xmul(t2, t2), a3 = xmul(t3, t3);
+    const T gw = xfma(xmul(where_pos<15>(t3), a3), a3,
+                      xfma(xmul(where_pos<-6>(t2), a2), a2, xmul(a1, a1)));
+    w = xmul(gw, rinv);
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) s[a] = xmul(w, r[a]);
   }
 };
 
-// Velocity-gradient term, g_ac += -(1/d_i) gw e_a v_c (kernel_vel_gradients.cu:334-337,
-// 632-640).
+// Velocity-gradient term, g_ac += gw e_a v_c (kernel_vel_gradients.cu:334-337, 632-640).
 template <typename T, int DIM>
-__device__ __forceinline__ void pair_grad_add(const PairOwn<T, DIM>& o, const PairRadial<T, DIM>& g,
-                                              const T v[3], PairAcc<T, DIM>& acc) {
-  const T s = -o.invd * g.gw;
+__device__ __forceinline__ void pair_grad_add(const PairRadial<T, DIM>& g, const T v[3],
+                                              PairAcc<T, DIM>& acc) {
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) {
-    const T se = s * g.e[a];
+  for (int a = 0; a < DIM; ++a)
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
-      if constexpr (PairAcc<T, DIM>::kTermwise)
-        PairAcc<T, DIM>::add(acc.g[a][c], acc.cg[a][c], se * v[c]);
+      if constexpr (sizeof(T) == 8)
+        acc.g[a][c] = xfma(g.s[a], v[c], acc.g[a][c]);
       else
-        acc.g[a][c] += se * v[c];
+        acc.g[a][c] = xadd(acc.g[a][c], (double)xmul(g.s[a], v[c]));
     }
-  }
 }
 
-// Force term from the partners' stress terms Pi, Pj (P/d^2 - nkT c/d^2) and inverse
-// densities di, dj: the reversible part -gw (Pi + Pj).e and the viscous part
-// a gw/(di dj r) v + b gw/(di dj r) (e.v) e (kernel_forces.cu:426-440, 826-850).
+// Force term (kernel_forces.cu:426-440, 826-850) from the partner's stress Pj
+// (P/d^2 - nkT c/d^2) and dd = 1/(d_i d_j): the reversible part -gw Pj.e (the target's own
+// stress is applied to the sum s) and the viscous part
+// a gw dd/r v + b gw dd/r (e.v) e.
 template <typename T, int DIM>
 __device__ __forceinline__ void pair_force_add(const PairParams<T, DIM>& pp,
-                                               const PairRadial<T, DIM>& g, const T v[3],
-                                               const T Pi[6], const T Pj[6], T di, T dj,
+                                               const PairRadial<T, DIM>& g, const T r[3],
+                                               const T v[3], const T Pj[6], T dd,
                                                PairAcc<T, DIM>& acc) {
-  const T gw = g.gw;
-  const T* e = g.e;
-  const T aux = gw * di * dj * g.rinv;
-  const T aux1 = pp.a * aux;
-  if constexpr (PairAcc<T, DIM>::kTermwise) {
-    // the pair's force as one term per component, then one compensated (or FP64) add
-    const T axx = -gw * (Pi[0] + Pj[0]);
-    const T axy = -gw * (Pi[1] + Pj[1]);
-    const T ayy = -gw * (Pi[2] + Pj[2]);
-    T ev = e[0] * v[0] + e[1] * v[1];
-    T t0 = axx * e[0] + axy * e[1], t1 = axy * e[0] + ayy * e[1], t2 = T(0);
-    if (DIM == 3) {
-      const T axz = -gw * (Pi[3] + Pj[3]);
-      const T ayz = -gw * (Pi[4] + Pj[4]);
-      const T azz = -gw * (Pi[5] + Pj[5]);
-      ev += e[2] * v[2];
-      t0 += axz * e[2];
-      t1 += ayz * e[2];
-      t2 = axz * e[0] + ayz * e[1] + azz * e[2];
+  const T m = xmul(g.w, dd);
+  const T aux1 = xmul(pp.a, m);
+  T rv = xfma(r[1], v[1], xmul(r[0], v[0]));
+  if (DIM == 3) rv = xfma(r[2], v[2], rv);
+  const T aux2 = xmul(xmul(xmul(pp.b, m), rv), xmul(g.rinv, g.rinv));
+  // rows of the symmetric stress: xx xy xz, xy yy yz, xz yz zz
+  constexpr int kRow[3][3] = {{0, 1, 3}, {1, 2, 4}, {3, 4, 5}};
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    if constexpr (sizeof(T) == 8) {
+      T f = acc.f[a];
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) f = xfma(-Pj[kRow[a][c]], g.s[c], f);
+      acc.f[a] = xfma(aux2, r[a], xfma(aux1, v[a], f));
+      acc.s[a] = xadd(acc.s[a], g.s[a]);
+    } else {
+      // the pair's force as one float term, then one FP64 add
+      T t = xmul(Pj[kRow[a][0]], g.s[0]);
+#pragma unroll
+      for (int c = 1; c < DIM; ++c) t = xfma(Pj[kRow[a][c]], g.s[c], t);
+      acc.f[a] = xadd(acc.f[a], (double)xfma(aux2, r[a], xfma(aux1, v[a], -t)));
+      acc.s[a] = xadd(acc.s[a], (double)g.s[a]);
     }
-    const T aux2 = pp.b * aux * ev;
-    PairAcc<T, DIM>::add(acc.f[0], acc.cf[0], t0 + (aux1 * v[0] + aux2 * e[0]));
-    PairAcc<T, DIM>::add(acc.f[1], acc.cf[1], t1 + (aux1 * v[1] + aux2 * e[1]));
-    if (DIM == 3) PairAcc<T, DIM>::add(acc.f[2], acc.cf[2], t2 + (aux1 * v[2] + aux2 * e[2]));
-  } else {
-    // -gw (Pi + Pj).e and the viscous terms folded into the sums by fused multiply-adds
-    const T ngw = -gw;
-    T ev = e[0] * v[0] + e[1] * v[1];
-    T t0 = (Pi[0] + Pj[0]) * e[0] + (Pi[1] + Pj[1]) * e[1];
-    T t1 = (Pi[1] + Pj[1]) * e[0] + (Pi[2] + Pj[2]) * e[1];
-    T t2 = T(0);
-    if (DIM == 3) {
-      const T sxz = Pi[3] + Pj[3], syz = Pi[4] + Pj[4];
-      ev += e[2] * v[2];
-      t0 += sxz * e[2];
-      t1 += syz * e[2];
-      t2 = sxz * e[0] + syz * e[1] + (Pi[5] + Pj[5]) * e[2];
-    }
-    const T aux2 = pp.b * aux * ev;
-    acc.f[0] = fma(aux2, e[0], fma(aux1, v[0], fma(ngw, t0, acc.f[0])));
-    acc.f[1] = fma(aux2, e[1], fma(aux1, v[1], fma(ngw, t1, acc.f[1])));
-    if (DIM == 3) acc.f[2] = fma(aux2, e[2], fma(aux1, v[2], fma(ngw, t2, acc.f[2])));
   }
 }
 
@@ -703,39 +661,30 @@ __device__ __forceinline__ void pair_term(const BoxParams& p, const PairParams<T
   }
   PairRadial<T, DIM> g;
   g.eval(pp, r2, r);
-  if (pair_grad) pair_grad_add<T, DIM>(o, g, v, acc);
+  if (pair_grad) pair_grad_add<T, DIM>(g, v, acc);
   if (pair_force) {
-    T Pi[6], Pj[6], di, dj;
+    T Pj[6], dd;
     if (o.fluid && fluid_j) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        Pi[q] = o.P[q];
-        Pj[q] = rec_P<DIM>(rj, q);
-      }
-      di = o.invd;
-      dj = rj.invd;
+      for (int q = 0; q < 6; ++q) Pj[q] = rec_P<DIM>(rj, q);
+      dd = xmul(o.invd, (T)rj.invd);
     } else if (o.fluid) {
       // j mirrors i's density and pressure, keeps its own c (kernel_forces.cu:217-233)
-      const T dsq = o.invd * o.invd;
+      const T dsq = xmul(o.invd, o.invd);
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
-        Pi[q] = o.P[q];
         const T diag = (q == 0 || q == 2 || q == 5) ? o.press : T(0);
-        Pj[q] = (diag + rec_P<DIM>(rj, q)) * dsq;
+        Pj[q] = xmul(xadd(diag, rec_P<DIM>(rj, q)), dsq);
       }
-      di = o.invd;
-      dj = o.invd;
+      dd = dsq;
     } else {
-      // i takes j's density, pressure and c (kernel_forces.cu:320-336)
+      // i takes j's density, pressure and c (kernel_forces.cu:320-336): twice j's stress, and
+      // none of its own at the end of the pass
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        Pj[q] = rec_P<DIM>(rj, q);
-        Pi[q] = rec_P<DIM>(rj, q);
-      }
-      di = rj.invd;
-      dj = rj.invd;
+      for (int q = 0; q < 6; ++q) Pj[q] = xmul(T(2), rec_P<DIM>(rj, q));
+      dd = xmul((T)rj.invd, (T)rj.invd);
     }
-    pair_force_add<T, DIM>(pp, g, v, Pi, Pj, di, dj, acc);
+    pair_force_add<T, DIM>(pp, g, r, v, Pj, dd, acc);
   }
 }
 
@@ -758,12 +707,12 @@ __device__ __forceinline__ void pair_fluid_x1(const BoxParams& p, const PairPara
   const T v[3] = {o.v[0] - (T)rj.vx, o.v[1] - (T)rj.vy, o.v[2] - (T)rec_vz<DIM>(rj)};
   PairRadial<T, DIM> g;
   g.eval(pp, r2, r);
-  if constexpr (FluidTerms<MODE>::kGrad) pair_grad_add<T, DIM>(o, g, v, acc);
+  if constexpr (FluidTerms<MODE>::kGrad) pair_grad_add<T, DIM>(g, v, acc);
   if constexpr (FluidTerms<MODE>::kForce) {
     T Pj[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) Pj[q] = rec_P<DIM>(rj, q);
-    pair_force_add<T, DIM>(pp, g, v, o.P, Pj, o.invd, (T)rj.invd, acc);
+    pair_force_add<T, DIM>(pp, g, r, v, Pj, xmul(o.invd, (T)rj.invd), acc);
   }
 }
 
@@ -779,28 +728,44 @@ __device__ __forceinline__ void vv2_fluid(const BoxParams& p, double mass, doubl
   if (DIM == 3) v.z = __fma_rn(hm, fz, v.z);
 }
 
-// stored gradient, forces with the body force, and dc/dt of particle i
+// stored gradient, forces with the body force, and dc/dt of particle i, from the pass's sums
+// and the factors left out of them (see PairAcc)
 template <typename T, int DIM, int MODE, bool EXT>
 __device__ __forceinline__ void pair_store(const Dev& d, int i, const BoxParams& p,
                                            const PairOwn<T, DIM>& o,
                                            const PairAcc<T, DIM>& acc) {
+  using Rec = typename RecFor<T, DIM>::type;
   const int Np2 = d.Npad;
+  const double cg = -((double)o.invd * p.c_gradw);
+  double G[DIM][DIM];
+#pragma unroll
+  for (int a = 0; a < DIM; ++a)
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) G[a][c] = cg * acc.g[a][c];
   if (MODE == kPairGradvAll || (MODE == kPairFused && d.gradv != nullptr && o.do_grad)) {
     // storage order xx xy xz yx yy yz zx zy zz
-    d.gradv[0 * Np2 + i] = acc.grad(0, 0);
-    d.gradv[1 * Np2 + i] = acc.grad(0, 1);
-    d.gradv[3 * Np2 + i] = acc.grad(1, 0);
-    d.gradv[4 * Np2 + i] = acc.grad(1, 1);
-    if (DIM == 3) {
-      d.gradv[2 * Np2 + i] = acc.grad(0, DIM - 1);
-      d.gradv[5 * Np2 + i] = acc.grad(1, DIM - 1);
-      d.gradv[6 * Np2 + i] = acc.grad(DIM - 1, 0);
-      d.gradv[7 * Np2 + i] = acc.grad(DIM - 1, 1);
-      d.gradv[8 * Np2 + i] = acc.grad(DIM - 1, DIM - 1);
-    }
+#pragma unroll
+    for (int a = 0; a < DIM; ++a)
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) d.gradv[(3 * a + c) * Np2 + i] = G[a][c];
   }
   if (MODE == kPairGradvAll) return;
-  double fx = acc.force(0), fy = acc.force(1), fz = acc.force(2);
+  double F[3] = {acc.f[0], acc.f[1], DIM == 3 ? acc.f[DIM - 1] : 0.0};
+  if (o.fluid) {
+    const Rec* rec = reinterpret_cast<const Rec*>(d.rec);
+    const double Pxx = rec[i].P[0], Pxy = rec[i].P[1], Pyy = rec[i].P[2];
+    F[0] = __fma_rn(-Pxy, acc.s[1], __fma_rn(-Pxx, acc.s[0], F[0]));
+    F[1] = __fma_rn(-Pyy, acc.s[1], __fma_rn(-Pxy, acc.s[0], F[1]));
+    if constexpr (DIM == 3) {
+      const double Pxz = rec[i].P[3], Pyz = rec[i].P[4], Pzz = rec[i].P[5];
+      F[0] = __fma_rn(-Pxz, acc.s[2], F[0]);
+      F[1] = __fma_rn(-Pyz, acc.s[2], F[1]);
+      F[2] = __fma_rn(-Pzz, acc.s[2],
+                      __fma_rn(-Pyz, acc.s[1], __fma_rn(-Pxz, acc.s[0], F[2])));
+    }
+  }
+  double fx = __dmul_rn(p.c_gradw, F[0]), fy = __dmul_rn(p.c_gradw, F[1]),
+         fz = __dmul_rn(p.c_gradw, F[2]);
   if (EXT && o.fluid) {
     const double4 xd = d.pos[i];
     const double m = xd.w;
@@ -832,8 +797,8 @@ __device__ __forceinline__ void pair_store(const Dev& d, int i, const BoxParams&
     double dc[6];
     const double cxx = d.conf[i], cxy = d.conf[Np2 + i], cyy = d.conf[2 * Np2 + i];
     if (DIM == 2) {
-      const double gxx = acc.grad(0, 0), gxy = acc.grad(0, 1), gyx = acc.grad(1, 0),
-                   gyy = acc.grad(1, 1);
+      const double gxx = G[0][0], gxy = G[0][1], gyx = G[1][0],
+                   gyy = G[1][1];
       const double Axx = cxx * gxx + cxy * gyx, Axy = cxx * gxy + cxy * gyy;
       const double Ayx = cxy * gxx + cyy * gyx, Ayy = cxy * gxy + cyy * gyy;
       dc[0] = 2.0 * Axx + tinv * (1.0 - cxx);
@@ -845,10 +810,10 @@ __device__ __forceinline__ void pair_store(const Dev& d, int i, const BoxParams&
       dc[5] = 0.0;
     } else {
       const double cxz = d.conf[3 * Np2 + i], cyz = d.conf[4 * Np2 + i], czz = d.conf[5 * Np2 + i];
-      const double gxx = acc.grad(0, 0), gxy = acc.grad(0, 1), gxz = acc.grad(0, DIM - 1);
-      const double gyx = acc.grad(1, 0), gyy = acc.grad(1, 1), gyz = acc.grad(1, DIM - 1);
-      const double gzx = acc.grad(DIM - 1, 0), gzy = acc.grad(DIM - 1, 1),
-                   gzz = acc.grad(DIM - 1, DIM - 1);
+      const double gxx = G[0][0], gxy = G[0][1], gxz = G[0][DIM - 1];
+      const double gyx = G[1][0], gyy = G[1][1], gyz = G[1][DIM - 1];
+      const double gzx = G[DIM - 1][0], gzy = G[DIM - 1][1],
+                   gzz = G[DIM - 1][DIM - 1];
       const double Axx = cxx * gxx + cxy * gyx + cxz * gzx;
       const double Axy = cxx * gxy + cxy * gyy + cxz * gzy;
       const double Axz = cxx * gxz + cxy * gyz + cxz * gzz;

@@ -290,19 +290,19 @@ __global__ void k_reorder(Dev d) {
   if (k == d.Ntot - 1 || d.keys[k + 1] != key) d.cell_end[key] = k - slot0;
 }
 
-// Density contribution of one list entry (kernel_densities.cu:52-163 with kernel_W.cu):
-// the exact distance test, then W(r) with r from one reciprocal square root; the
-// particle itself (r2 = 0) contributes W(0).  WRAP: see min_image.
+// Density contribution of one list entry over cw (kernel_densities.cu:52-163 with
+// kernel_W.cu): the exact distance test, then W(r) with r from one reciprocal square root;
+// the particle itself (r2 = 0) contributes W(0).  WRAP: see min_image.
 template <typename T, int DIM, bool WRAP = true>
 __device__ __forceinline__ T density_term(const typename V4<T>::type& xi,
                                           const typename V4<T>::type& xj, const T L[3],
-                                          const T h[3], int wall, T rcutsq, T rcut_inv, T cw) {
+                                          const T h[3], int wall, T rcutsq, T rcut_inv3) {
   T rx = xi.x - xj.x, ry = xi.y - xj.y, rz = DIM == 3 ? xi.z - xj.z : T(0);
   min_image<T, DIM, WRAP>(rx, ry, rz, L, h, wall);
   const T r2 = norm2(rx, ry, rz, DIM == 3);
   if (!(r2 < rcutsq)) return T(0);
-  const T r = r2 > T(0) ? r2 * rsqrt(r2) : T(0);
-  return sph_w<T>(r, rcut_inv, cw);
+  const T r = r2 > T(0) ? xmul(r2, inv_sqrt(r2)) : T(0);
+  return sph_w<T>(r, rcut_inv3);
 }
 
 // Density, pressure (kernel_pressures.cu:13-23) and the neighbour record of slot i.
@@ -771,13 +771,12 @@ __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>
   const T L[3] = {(T)p.L[0], (T)p.L[1], (T)p.L[2]};
   const T h[3] = {(T)p.halfL[0], (T)p.halfL[1], (T)p.halfL[2]};
   const T rcutsq = (T)p.rcutsq;
-  const T rcut_inv = (T)p.rcut_inv, cw = (T)p.cw;
+  const T rcut_inv3 = (T)(3.0 * p.rcut_inv);
   const V xi = ld_pos<DIM>(P + i);
   const int n = d.nbr_cnt[i];
   NbrIter it;
   it.init(d, i);
   typename SumKind<T>::S dens = 0;
-  T comp = T(0);  // Kahan compensation of a float sum
   for (int k = 0; k < n; k += kAhead) {
     int j[kAhead];
     V x[kAhead];
@@ -788,14 +787,11 @@ __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
       if (j[u] < 0) break;
-      const T w = density_term<T, DIM, WRAP>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv, cw);
-      if constexpr (Compensated<T>::on)
-        kahan_add(dens, comp, w);
-      else
-        dens = dens + w;
+      const T w = density_term<T, DIM, WRAP>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv3);
+      dens = dens + w;
     }
   }
-  return (double)dens - (double)comp;
+  return __dmul_rn(p.cw, dens);
 }
 
 // Whole warps (lanes past the end mirror the last slot and store nothing), so that a warp
@@ -879,7 +875,7 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
   const T L[3] = {(T)p.L[0], (T)p.L[1], (T)p.L[2]};
   const T h[3] = {(T)p.halfL[0], (T)p.halfL[1], (T)p.halfL[2]};
   const T rcutsq = (T)p.rcutsq;
-  const T rcut_inv = (T)p.rcut_inv, cw = (T)p.cw;
+  const T rcut_inv3 = (T)(3.0 * p.rcut_inv);
   const int beg = d.cell_begin[cell], end = d.cell_begin[cell + 1];
   for (int t0 = 0; t0 < end - beg; t0 += 32) {
     const int i = beg + t0 + lane;
@@ -891,13 +887,9 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
     // the next list entry not yet summed (-1: none left)
     int jn = n > 0 ? it.next() : -1;
     typename SumKind<T>::S dens = 0;
-  T comp = T(0);  // Kahan compensation of a float sum
     auto add = [&](const V& xj) {
-      const T wv = density_term<T, DIM>(xi, xj, L, h, p.wall, rcutsq, rcut_inv, cw);
-      if constexpr (Compensated<T>::on)
-        kahan_add(dens, comp, wv);
-      else
-        dens = dens + wv;
+      const T wv = density_term<T, DIM>(xi, xj, L, h, p.wall, rcutsq, rcut_inv3);
+      dens = dens + wv;
     };
     int k = 0;
     for (int ph = 0; ph < kPh; ++ph) {
@@ -962,7 +954,7 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
       add(ld_pos<DIM>(P + jn));
       jn = k + 1 < n ? it.next() : -1;
     }
-    if (active) density_epilogue<T, DIM>(d, i, p, (double)dens - (double)comp);
+    if (active) density_epilogue<T, DIM>(d, i, p, __dmul_rn(p.cw, dens));
   }
 }
 
@@ -1024,8 +1016,8 @@ struct PairShape {
 // The pair constants of a one-box context, viewed as PairParams (same layout).
 template <typename T, int DIM>
 __device__ __forceinline__ const PairParams<T, DIM>& one_box_params(const Dev& d) {
-  static_assert(sizeof(PairParams<double, DIM>) == 11 * sizeof(double) &&
-                    sizeof(PairParams<float, DIM>) == 11 * sizeof(float),
+  static_assert(sizeof(PairParams<double, DIM>) == 10 * sizeof(double) &&
+                    sizeof(PairParams<float, DIM>) == 10 * sizeof(float),
                 "PairParams layout");
   if constexpr (sizeof(T) == 8)
     return *reinterpret_cast<const PairParams<T, DIM>*>(d.pc.L);
