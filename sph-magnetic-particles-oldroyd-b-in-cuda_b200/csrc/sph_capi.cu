@@ -864,11 +864,15 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
       k.hf[a] = (float)q.halfL[a];
     }
     k.rcutsq = q.rcutsq;
+    k.rcut_inv = q.rcut_inv;
     k.rcut_inv3 = 3.0 * q.rcut_inv;
+    k.c_gradw = q.c_gradw;
     k.a = q.a;
     k.b = q.b;
     k.rcutsqf = (float)q.rcutsq;
+    k.rcut_invf = (float)q.rcut_inv;
     k.rcut_inv3f = (float)(3.0 * q.rcut_inv);
+    k.c_gradwf = (float)q.c_gradw;
     k.af = (float)q.a;
     k.bf = (float)q.b;
   }

@@ -43,17 +43,13 @@ __device__ __forceinline__ auto rec_P(const R& r, int q) -> decltype(r.x) {
 // takes them (one box or many, with or without the minimum image, one or two particles per
 // lane), and the compiler may contract a plain expression differently in each.
 __device__ __forceinline__ double xmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double xadd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float xadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double xfma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float xfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 // 1 / sqrt(x) of a positive normal x.  FP64: the hardware's seed and one third-order
 // Householder step, y (1 + e (1/2 + 3/8 e)) with e = 1 - x y^2 (the Taylor series of
 // (1 - e)^(-1/2) to second order: the error is 5/16 e^3), without the special cases of the
 // library function, which no pair of distinct particles meets.
-__device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double inv_sqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -61,28 +57,39 @@ __device__ __forceinline__ double inv_sqrt(double x) {
   return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 
-// c where t >= 0, else 0 (a test of the sign bit; FP64: the constant's high word alone, its
-// low word being zero)
+// c where t >= 0, else 0 (a test of the sign bit; the constant's low word is zero)
 template <int C>
 __device__ __forceinline__ double where_pos(double t) {
   return __hiloint2double(__double2hiint(t) < 0 ? 0 : __double2hiint((double)C), 0);
 }
-template <int C>
-__device__ __forceinline__ float where_pos(float t) {
-  return t < 0.0f ? 0.0f : (float)C;
-}
-
-// SPH kernel over its constant, W / cw (kernel_W.cu:13-59; its radial derivative,
-// kernel_gradW.cu:13-53, is in PairRadial): (3 - q)^5 - 6 (2 - q)^5 [q < 2] +
-// 15 (1 - q)^5 [q < 1] with q = 3 r / rcut.  Branch-free: the clamped terms are exact zeros
-// where the reference skips them, so the value is that of the branchy form.
-template <typename T>
-__device__ __forceinline__ T sph_w(T r, T rcut_inv3) {
-  const T t1 = xfma(-rcut_inv3, r, T(3)), t2 = xfma(-rcut_inv3, r, T(2)),
-          t3 = xfma(-rcut_inv3, r, T(1));
-  const T a1 = xmul(t1, t1), a2 = xmul(t2, t2), a3 = xmul(t3, t3);
+// SPH kernel (kernel_W.cu:13-59; its radial derivative, kernel_gradW.cu:13-53, is in
+// PairRadial): cw ((3 - q)^5 - 6 (2 - q)^5 [q < 2] + 15 (1 - q)^5 [q < 1]), q = 3 r / rcut.
+// Branch-free: the clamped terms are exact zeros where the reference skips them, so the value
+// is that of the branchy form.  FP64: without cw, which the density sum is multiplied by.
+__device__ __forceinline__ double sph_w(double r, double rcut_inv3) {
+  const double t1 = xfma(-rcut_inv3, r, 3.0), t2 = xfma(-rcut_inv3, r, 2.0),
+               t3 = xfma(-rcut_inv3, r, 1.0);
+  const double a1 = xmul(t1, t1), a2 = xmul(t2, t2), a3 = xmul(t3, t3);
   return xfma(xmul(where_pos<15>(t3), t3), xmul(a3, a3),
               xfma(xmul(where_pos<-6>(t2), t2), xmul(a2, a2), xmul(xmul(a1, a1), t1)));
+}
+__device__ __forceinline__ float sph_w(float r, float rcut_inv, float cw) {
+  float q3 = (r * rcut_inv) * 3.0f;
+  float t1 = 3.0f - q3, t2 = 2.0f - q3, t3 = 1.0f - q3;
+  float a1 = t1 * t1, a2 = t2 * t2, a3 = t3 * t3;
+  float w = (a1 * a1) * t1;
+  if (q3 < 2.0f) w = w - 6.0f * ((a2 * a2) * t2);
+  if (q3 < 1.0f) w = w + 15.0f * ((a3 * a3) * t3);
+  return cw * w;
+}
+__device__ __forceinline__ float sph_gradw(float r, float rcut_inv, float c_gradw) {
+  float q3 = 3.0f * (r * rcut_inv);
+  float t1 = 3.0f - q3, t2 = 2.0f - q3, t3 = 1.0f - q3;
+  float a1 = t1 * t1, a2 = t2 * t2, a3 = t3 * t3;
+  float g = a1 * a1;
+  if (q3 < 2.0f) g = g - 6.0f * (a2 * a2);
+  if (q3 < 1.0f) g = g + 15.0f * (a3 * a3);
+  return c_gradw * g;
 }
 
 // Minimum image as the reference writes it: subtract L above L/2, add L below -L/2
@@ -486,7 +493,7 @@ __device__ __forceinline__ float4 ld_pos(const float4* a) {
 
 template <typename T, int DIM>
 struct PairParams {
-  T L[3], h[3], rcutsq, rcut_inv3, a, b;  // rcut_inv3 = 3 / rcut
+  T L[3], h[3], rcutsq, rcut_inv, rcut_inv3, c_gradw, a, b;  // rcut_inv3 = 3 / rcut
   __device__ __forceinline__ void load(const BoxParams& p) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -494,7 +501,9 @@ struct PairParams {
       h[q] = (T)p.halfL[q];
     }
     rcutsq = (T)p.rcutsq;
+    rcut_inv = (T)p.rcut_inv;
     rcut_inv3 = (T)(3.0 * p.rcut_inv);
+    c_gradw = (T)p.c_gradw;
     a = (T)p.a;
     b = (T)p.b;
   }
@@ -504,32 +513,28 @@ struct PairParams {
 template <typename T, int DIM>
 struct PairOwn {
   T x, y, z, v[3], invd, press;
+  float P[6];  // mixed precision: the particle's stress term (FP64 applies it to the sums)
   int t;
   bool fluid, do_grad, do_force;
 };
 
-// Sums of a pass over one particle's list.  What is common to every term is left out of the
-// terms and applied when the sums are stored (pair_store): the kernel's factor c_gradw, the
-// particle's own stress term P_i (its part of the force is P_i times the sum s of gw e) and
-// the gradient's -1/d_i.  S: the accumulator type.  The float pair terms of mixed precision
-// are summed in FP64 (more accurate than compensated float sums, and the conversions and
-// FP64 adds run on the otherwise idle FP64 pipe).
-template <typename T>
-struct SumKind {
-  using S = double;
-};
+// Sums of a pass over one particle's list, in FP64 accumulators.
+// FP64: what is common to every term is left out of the terms and applied when the sums are
+// stored (pair_store): the kernel's factor c_gradw, the particle's own stress term P_i (its
+// part of the force is P_i times the sum s of gw e) and the gradient's -1/d_i.
+// Mixed precision: whole terms, evaluated in float (more accurate than compensated float
+// sums, and the conversions and FP64 adds run on the otherwise idle FP64 pipe).
 template <typename T, int DIM>
 struct PairAcc {
-  using S = typename SumKind<T>::S;
-  S g[DIM][DIM];  // sum of gw e_a v_c
-  S f[DIM];       // force terms but the particle's own stress
-  S s[DIM];       // sum of gw e
+  double g[DIM][DIM];  // FP64: sum of gw e_a v_c; mixed: the gradient
+  double f[DIM];       // the force (FP64: but the particle's own stress)
+  double s[DIM];       // FP64: sum of gw e
   __device__ __forceinline__ void zero() {
 #pragma unroll
     for (int a = 0; a < DIM; ++a) {
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) g[a][c] = S(0);
-      f[a] = s[a] = S(0);
+      for (int c = 0; c < DIM; ++c) g[a][c] = 0.0;
+      f[a] = s[a] = 0.0;
     }
   }
 };
@@ -546,6 +551,10 @@ __device__ __forceinline__ void load_own(const Dev& d, int i, int ti, const Rec&
   o.v[2] = (T)rec_vz<DIM>(ri);
   o.invd = ri.invd;
   o.press = (T)d.press[i];
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int q = 0; q < 6; ++q) o.P[q] = rec_P<DIM>(ri, q);
+  }
   o.t = type_of(ti);
   o.fluid = o.t == 0;
   // gradient: every particle in kPairGradvAll; in the fused pass fluid particles (whose
@@ -565,73 +574,120 @@ __device__ __forceinline__ T pair_sep(const PairParams<T, DIM>& pp, int wall,
   return norm2(r[0], r[1], r[2], DIM == 3);
 }
 
-// 1/|r| and the vector s = (dW/dr / c_gradw) r / |r|; w = |s| / |r|.
+// The radial part of a pair's terms.  FP64: 1/|r| and the vector s = (dW/dr / c_gradw) r / |r|,
+// w = |s| / |r|.  Mixed: 1/|r|, the slope gw = dW/dr and the unit vector e = r / |r|.
 template <typename T, int DIM>
-struct PairRadial {
-  T rinv, w, s[DIM];
-  __device__ __forceinline__ void eval(const PairParams<T, DIM>& pp, T r2, const T r[3]) {
+struct PairRadial;
+template <int DIM>
+struct PairRadial<double, DIM> {
+  double rinv, w, s[DIM];
+  __device__ __forceinline__ void eval(const PairParams<double, DIM>& pp, double r2,
+                                       const double r[3]) {
     rinv = inv_sqrt(r2);
-    const T rr = xmul(r2, rinv);
+    const double rr = xmul(r2, rinv);
     // (3 - q)^4 - 6 (2 - q)^4 [q < 2] + 15 (1 - q)^4 [q < 1], q = 3 |r| / rcut
-    const T t1 = xfma(-pp.rcut_inv3, rr, T(3)), t2 = xfma(-pp.rcut_inv3, rr, T(2)),
-            t3 = xfma(-pp.rcut_inv3, rr, T(1));
-    const T a1 = xmul(t1, t1), a2 = xmul(t2, t2), a3 = xmul(t3, t3);
-    const T gw = xfma(xmul(where_pos<15>(t3), a3), a3,
-                      xfma(xmul(where_pos<-6>(t2), a2), a2, xmul(a1, a1)));
+    const double t1 = xfma(-pp.rcut_inv3, rr, 3.0), t2 = xfma(-pp.rcut_inv3, rr, 2.0),
+                 t3 = xfma(-pp.rcut_inv3, rr, 1.0);
+    const double a1 = xmul(t1, t1), a2 = xmul(t2, t2), a3 = xmul(t3, t3);
+    const double gw = xfma(xmul(where_pos<15>(t3), a3), a3,
+                           xfma(xmul(where_pos<-6>(t2), a2), a2, xmul(a1, a1)));
     w = xmul(gw, rinv);
 #pragma unroll
     for (int a = 0; a < DIM; ++a) s[a] = xmul(w, r[a]);
   }
 };
+template <int DIM>
+struct PairRadial<float, DIM> {
+  float rinv, gw, e[3];
+  __device__ __forceinline__ void eval(const PairParams<float, DIM>& pp, float r2,
+                                       const float r[3]) {
+    rinv = rsqrt(r2);  // r and 1/r from one reciprocal square root
+    const float rr = r2 * rinv;
+    gw = sph_gradw(rr, pp.rcut_inv, pp.c_gradw);
+    e[0] = r[0] * rinv;
+    e[1] = r[1] * rinv;
+    e[2] = DIM == 3 ? r[2] * rinv : 0.0f;
+  }
+};
 
-// Velocity-gradient term, g_ac += gw e_a v_c (kernel_vel_gradients.cu:334-337, 632-640).
-template <typename T, int DIM>
-__device__ __forceinline__ void pair_grad_add(const PairRadial<T, DIM>& g, const T v[3],
-                                              PairAcc<T, DIM>& acc) {
+// Velocity-gradient term (kernel_vel_gradients.cu:334-337, 632-640): FP64 g_ac += gw e_a v_c,
+// mixed g_ac += -(1/d_i) gw e_a v_c.
+template <int DIM>
+__device__ __forceinline__ void pair_grad_add(const PairOwn<double, DIM>&,
+                                              const PairRadial<double, DIM>& g, const double v[3],
+                                              PairAcc<double, DIM>& acc) {
 #pragma unroll
   for (int a = 0; a < DIM; ++a)
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      if constexpr (sizeof(T) == 8)
-        acc.g[a][c] = xfma(g.s[a], v[c], acc.g[a][c]);
-      else
-        acc.g[a][c] = xadd(acc.g[a][c], (double)xmul(g.s[a], v[c]));
-    }
+    for (int c = 0; c < DIM; ++c) acc.g[a][c] = xfma(g.s[a], v[c], acc.g[a][c]);
+}
+template <int DIM>
+__device__ __forceinline__ void pair_grad_add(const PairOwn<float, DIM>& o,
+                                              const PairRadial<float, DIM>& g, const float v[3],
+                                              PairAcc<float, DIM>& acc) {
+  const float s = -o.invd * g.gw;
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    const float se = s * g.e[a];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) acc.g[a][c] += (double)(se * v[c]);
+  }
 }
 
-// Force term (kernel_forces.cu:426-440, 826-850) from the partner's stress Pj
-// (P/d^2 - nkT c/d^2) and dd = 1/(d_i d_j): the reversible part -gw Pj.e (the target's own
-// stress is applied to the sum s) and the viscous part
-// a gw dd/r v + b gw dd/r (e.v) e.
-template <typename T, int DIM>
-__device__ __forceinline__ void pair_force_add(const PairParams<T, DIM>& pp,
-                                               const PairRadial<T, DIM>& g, const T r[3],
-                                               const T v[3], const T Pj[6], T dd,
-                                               PairAcc<T, DIM>& acc) {
-  const T m = xmul(g.w, dd);
-  const T aux1 = xmul(pp.a, m);
-  T rv = xfma(r[1], v[1], xmul(r[0], v[0]));
+// Force term (kernel_forces.cu:426-440, 826-850) from the partners' stress terms Pi, Pj
+// (P/d^2 - nkT c/d^2) and inverse densities di, dj: the reversible part -gw (Pi + Pj).e and the
+// viscous part a gw/(di dj r) v + b gw/(di dj r) (e.v) e.  FP64: without Pi (see PairAcc).
+template <int DIM>
+__device__ __forceinline__ void pair_force_add(const PairParams<double, DIM>& pp,
+                                               const PairRadial<double, DIM>& g,
+                                               const double r[3], const double v[3],
+                                               const double*, const double Pj[6], double di,
+                                               double dj, PairAcc<double, DIM>& acc) {
+  const double m = xmul(g.w, xmul(di, dj));
+  const double aux1 = xmul(pp.a, m);
+  double rv = xfma(r[1], v[1], xmul(r[0], v[0]));
   if (DIM == 3) rv = xfma(r[2], v[2], rv);
-  const T aux2 = xmul(xmul(xmul(pp.b, m), rv), xmul(g.rinv, g.rinv));
+  const double aux2 = xmul(xmul(xmul(pp.b, m), rv), xmul(g.rinv, g.rinv));
   // rows of the symmetric stress: xx xy xz, xy yy yz, xz yz zz
   constexpr int kRow[3][3] = {{0, 1, 3}, {1, 2, 4}, {3, 4, 5}};
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
-    if constexpr (sizeof(T) == 8) {
-      T f = acc.f[a];
+    double f = acc.f[a];
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) f = xfma(-Pj[kRow[a][c]], g.s[c], f);
-      acc.f[a] = xfma(aux2, r[a], xfma(aux1, v[a], f));
-      acc.s[a] = xadd(acc.s[a], g.s[a]);
-    } else {
-      // the pair's force as one float term, then one FP64 add
-      T t = xmul(Pj[kRow[a][0]], g.s[0]);
-#pragma unroll
-      for (int c = 1; c < DIM; ++c) t = xfma(Pj[kRow[a][c]], g.s[c], t);
-      acc.f[a] = xadd(acc.f[a], (double)xfma(aux2, r[a], xfma(aux1, v[a], -t)));
-      acc.s[a] = xadd(acc.s[a], (double)g.s[a]);
-    }
+    for (int c = 0; c < DIM; ++c) f = xfma(-Pj[kRow[a][c]], g.s[c], f);
+    acc.f[a] = xfma(aux2, r[a], xfma(aux1, v[a], f));
+    acc.s[a] = xadd(acc.s[a], g.s[a]);
   }
+}
+template <int DIM>
+__device__ __forceinline__ void pair_force_add(const PairParams<float, DIM>& pp,
+                                               const PairRadial<float, DIM>& g, const float*,
+                                               const float v[3], const float Pi[6],
+                                               const float Pj[6], float di, float dj,
+                                               PairAcc<float, DIM>& acc) {
+  const float gw = g.gw;
+  const float* e = g.e;
+  const float aux = gw * di * dj * g.rinv;
+  const float aux1 = pp.a * aux;
+  // the pair's force as one float term per component, then one FP64 add
+  const float axx = -gw * (Pi[0] + Pj[0]);
+  const float axy = -gw * (Pi[1] + Pj[1]);
+  const float ayy = -gw * (Pi[2] + Pj[2]);
+  float ev = e[0] * v[0] + e[1] * v[1];
+  float t0 = axx * e[0] + axy * e[1], t1 = axy * e[0] + ayy * e[1], t2 = 0.0f;
+  if (DIM == 3) {
+    const float axz = -gw * (Pi[3] + Pj[3]);
+    const float ayz = -gw * (Pi[4] + Pj[4]);
+    const float azz = -gw * (Pi[5] + Pj[5]);
+    ev += e[2] * v[2];
+    t0 += axz * e[2];
+    t1 += ayz * e[2];
+    t2 = axz * e[0] + ayz * e[1] + azz * e[2];
+  }
+  const float aux2 = pp.b * aux * ev;
+  acc.f[0] += (double)(t0 + (aux1 * v[0] + aux2 * e[0]));
+  acc.f[1] += (double)(t1 + (aux1 * v[1] + aux2 * e[1]));
+  if constexpr (DIM == 3) acc.f[2] += (double)(t2 + (aux1 * v[2] + aux2 * e[2]));
 }
 
 // One (i, j) pair.  tj: the neighbour's particle type.  WRAP: see min_image.
@@ -661,30 +717,40 @@ __device__ __forceinline__ void pair_term(const BoxParams& p, const PairParams<T
   }
   PairRadial<T, DIM> g;
   g.eval(pp, r2, r);
-  if (pair_grad) pair_grad_add<T, DIM>(g, v, acc);
+  if (pair_grad) pair_grad_add<DIM>(o, g, v, acc);
   if (pair_force) {
-    T Pj[6], dd;
+    T Pi[6], Pj[6], di, dj;
     if (o.fluid && fluid_j) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) Pj[q] = rec_P<DIM>(rj, q);
-      dd = xmul(o.invd, (T)rj.invd);
+      for (int q = 0; q < 6; ++q) {
+        Pi[q] = o.P[q];
+        Pj[q] = rec_P<DIM>(rj, q);
+      }
+      di = o.invd;
+      dj = rj.invd;
     } else if (o.fluid) {
       // j mirrors i's density and pressure, keeps its own c (kernel_forces.cu:217-233)
-      const T dsq = xmul(o.invd, o.invd);
+      const T dsq = o.invd * o.invd;
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
+        Pi[q] = o.P[q];
         const T diag = (q == 0 || q == 2 || q == 5) ? o.press : T(0);
-        Pj[q] = xmul(xadd(diag, rec_P<DIM>(rj, q)), dsq);
+        Pj[q] = (diag + rec_P<DIM>(rj, q)) * dsq;
       }
-      dd = dsq;
+      di = o.invd;
+      dj = o.invd;
     } else {
-      // i takes j's density, pressure and c (kernel_forces.cu:320-336): twice j's stress, and
-      // none of its own at the end of the pass
+      // i takes j's density, pressure and c (kernel_forces.cu:320-336); FP64: twice j's
+      // stress, and none of its own at the end of the pass
 #pragma unroll
-      for (int q = 0; q < 6; ++q) Pj[q] = xmul(T(2), rec_P<DIM>(rj, q));
-      dd = xmul((T)rj.invd, (T)rj.invd);
+      for (int q = 0; q < 6; ++q) {
+        Pj[q] = (sizeof(T) == 8 ? T(2) : T(1)) * rec_P<DIM>(rj, q);
+        Pi[q] = rec_P<DIM>(rj, q);
+      }
+      di = rj.invd;
+      dj = rj.invd;
     }
-    pair_force_add<T, DIM>(pp, g, r, v, Pj, dd, acc);
+    pair_force_add<DIM>(pp, g, r, v, Pi, Pj, di, dj, acc);
   }
 }
 
@@ -707,12 +773,15 @@ __device__ __forceinline__ void pair_fluid_x1(const BoxParams& p, const PairPara
   const T v[3] = {o.v[0] - (T)rj.vx, o.v[1] - (T)rj.vy, o.v[2] - (T)rec_vz<DIM>(rj)};
   PairRadial<T, DIM> g;
   g.eval(pp, r2, r);
-  if constexpr (FluidTerms<MODE>::kGrad) pair_grad_add<T, DIM>(g, v, acc);
+  if constexpr (FluidTerms<MODE>::kGrad) pair_grad_add<DIM>(o, g, v, acc);
   if constexpr (FluidTerms<MODE>::kForce) {
-    T Pj[6];
+    T Pi[6], Pj[6];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) Pj[q] = rec_P<DIM>(rj, q);
-    pair_force_add<T, DIM>(pp, g, r, v, Pj, xmul(o.invd, (T)rj.invd), acc);
+    for (int q = 0; q < 6; ++q) {
+      Pi[q] = o.P[q];
+      Pj[q] = rec_P<DIM>(rj, q);
+    }
+    pair_force_add<DIM>(pp, g, r, v, Pi, Pj, o.invd, (T)rj.invd, acc);
   }
 }
 
@@ -736,7 +805,7 @@ __device__ __forceinline__ void pair_store(const Dev& d, int i, const BoxParams&
                                            const PairAcc<T, DIM>& acc) {
   using Rec = typename RecFor<T, DIM>::type;
   const int Np2 = d.Npad;
-  const double cg = -((double)o.invd * p.c_gradw);
+  const double cg = sizeof(T) == 8 ? -(o.invd * p.c_gradw) : 1.0;
   double G[DIM][DIM];
 #pragma unroll
   for (int a = 0; a < DIM; ++a)
@@ -751,7 +820,7 @@ __device__ __forceinline__ void pair_store(const Dev& d, int i, const BoxParams&
   }
   if (MODE == kPairGradvAll) return;
   double F[3] = {acc.f[0], acc.f[1], DIM == 3 ? acc.f[DIM - 1] : 0.0};
-  if (o.fluid) {
+  if (sizeof(T) == 8 && o.fluid) {
     const Rec* rec = reinterpret_cast<const Rec*>(d.rec);
     const double Pxx = rec[i].P[0], Pxy = rec[i].P[1], Pyy = rec[i].P[2];
     F[0] = __fma_rn(-Pxy, acc.s[1], __fma_rn(-Pxx, acc.s[0], F[0]));
@@ -764,8 +833,8 @@ __device__ __forceinline__ void pair_store(const Dev& d, int i, const BoxParams&
                       __fma_rn(-Pyz, acc.s[1], __fma_rn(-Pxz, acc.s[0], F[2])));
     }
   }
-  double fx = __dmul_rn(p.c_gradw, F[0]), fy = __dmul_rn(p.c_gradw, F[1]),
-         fz = __dmul_rn(p.c_gradw, F[2]);
+  const double cf = sizeof(T) == 8 ? p.c_gradw : 1.0;
+  double fx = __dmul_rn(cf, F[0]), fy = __dmul_rn(cf, F[1]), fz = __dmul_rn(cf, F[2]);
   if (EXT && o.fluid) {
     const double4 xd = d.pos[i];
     const double m = xd.w;

@@ -155,8 +155,8 @@ static_assert(sizeof(RecF2) == 32, "RecF2 layout");
 // value, so these live in the constant bank, where the pair pass's arithmetic reads them as
 // operands instead of holding them in registers (PairParams has the same layout).
 struct PairConsts {
-  double L[3], h[3], rcutsq, rcut_inv3, a, b;  // rcut_inv3 = 3 / rcut
-  float Lf[3], hf[3], rcutsqf, rcut_inv3f, af, bf;
+  double L[3], h[3], rcutsq, rcut_inv, rcut_inv3, c_gradw, a, b;  // rcut_inv3 = 3 / rcut
+  float Lf[3], hf[3], rcutsqf, rcut_invf, rcut_inv3f, c_gradwf, af, bf;
 };
 
 // Device pointers, passed to kernels by value.

@@ -290,19 +290,22 @@ __global__ void k_reorder(Dev d) {
   if (k == d.Ntot - 1 || d.keys[k + 1] != key) d.cell_end[key] = k - slot0;
 }
 
-// Density contribution of one list entry over cw (kernel_densities.cu:52-163 with
-// kernel_W.cu): the exact distance test, then W(r) with r from one reciprocal square root;
-// the particle itself (r2 = 0) contributes W(0).  WRAP: see min_image.
+// Density contribution of one list entry (kernel_densities.cu:52-163 with kernel_W.cu): the
+// exact distance test, then W(r) with r from one reciprocal square root; the particle itself
+// (r2 = 0) contributes W(0).  FP64: over cw, and rcut_inv is 3 / rcut.  WRAP: see min_image.
 template <typename T, int DIM, bool WRAP = true>
 __device__ __forceinline__ T density_term(const typename V4<T>::type& xi,
                                           const typename V4<T>::type& xj, const T L[3],
-                                          const T h[3], int wall, T rcutsq, T rcut_inv3) {
+                                          const T h[3], int wall, T rcutsq, T rcut_inv, T cw) {
   T rx = xi.x - xj.x, ry = xi.y - xj.y, rz = DIM == 3 ? xi.z - xj.z : T(0);
   min_image<T, DIM, WRAP>(rx, ry, rz, L, h, wall);
   const T r2 = norm2(rx, ry, rz, DIM == 3);
   if (!(r2 < rcutsq)) return T(0);
-  const T r = r2 > T(0) ? xmul(r2, inv_sqrt(r2)) : T(0);
-  return sph_w<T>(r, rcut_inv3);
+  if constexpr (sizeof(T) == 8) {
+    return sph_w(r2 > 0.0 ? xmul(r2, inv_sqrt(r2)) : 0.0, rcut_inv);
+  } else {
+    return sph_w(r2 > 0.0f ? r2 * rsqrt(r2) : 0.0f, rcut_inv, cw);
+  }
 }
 
 // Density, pressure (kernel_pressures.cu:13-23) and the neighbour record of slot i.
@@ -771,12 +774,13 @@ __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>
   const T L[3] = {(T)p.L[0], (T)p.L[1], (T)p.L[2]};
   const T h[3] = {(T)p.halfL[0], (T)p.halfL[1], (T)p.halfL[2]};
   const T rcutsq = (T)p.rcutsq;
-  const T rcut_inv3 = (T)(3.0 * p.rcut_inv);
+  const T rcut_inv = (T)((sizeof(T) == 8 ? 3.0 : 1.0) * p.rcut_inv), cw = (T)p.cw;
+  const double cdens = sizeof(T) == 8 ? p.cw : 1.0;  // the factor left out of the terms
   const V xi = ld_pos<DIM>(P + i);
   const int n = d.nbr_cnt[i];
   NbrIter it;
   it.init(d, i);
-  typename SumKind<T>::S dens = 0;
+  double dens = 0;
   for (int k = 0; k < n; k += kAhead) {
     int j[kAhead];
     V x[kAhead];
@@ -787,11 +791,11 @@ __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
       if (j[u] < 0) break;
-      const T w = density_term<T, DIM, WRAP>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv3);
+      const T w = density_term<T, DIM, WRAP>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv, cw);
       dens = dens + w;
     }
   }
-  return __dmul_rn(p.cw, dens);
+  return __dmul_rn(cdens, dens);
 }
 
 // Whole warps (lanes past the end mirror the last slot and store nothing), so that a warp
@@ -875,7 +879,8 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
   const T L[3] = {(T)p.L[0], (T)p.L[1], (T)p.L[2]};
   const T h[3] = {(T)p.halfL[0], (T)p.halfL[1], (T)p.halfL[2]};
   const T rcutsq = (T)p.rcutsq;
-  const T rcut_inv3 = (T)(3.0 * p.rcut_inv);
+  const T rcut_inv = (T)((sizeof(T) == 8 ? 3.0 : 1.0) * p.rcut_inv), cw = (T)p.cw;
+  const double cdens = sizeof(T) == 8 ? p.cw : 1.0;  // the factor left out of the terms
   const int beg = d.cell_begin[cell], end = d.cell_begin[cell + 1];
   for (int t0 = 0; t0 < end - beg; t0 += 32) {
     const int i = beg + t0 + lane;
@@ -886,9 +891,9 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
     it.init(d, active ? i : beg);
     // the next list entry not yet summed (-1: none left)
     int jn = n > 0 ? it.next() : -1;
-    typename SumKind<T>::S dens = 0;
+    double dens = 0;
     auto add = [&](const V& xj) {
-      const T wv = density_term<T, DIM>(xi, xj, L, h, p.wall, rcutsq, rcut_inv3);
+      const T wv = density_term<T, DIM>(xi, xj, L, h, p.wall, rcutsq, rcut_inv, cw);
       dens = dens + wv;
     };
     int k = 0;
@@ -954,7 +959,7 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
       add(ld_pos<DIM>(P + jn));
       jn = k + 1 < n ? it.next() : -1;
     }
-    if (active) density_epilogue<T, DIM>(d, i, p, __dmul_rn(p.cw, dens));
+    if (active) density_epilogue<T, DIM>(d, i, p, __dmul_rn(cdens, dens));
   }
 }
 
@@ -1016,8 +1021,8 @@ struct PairShape {
 // The pair constants of a one-box context, viewed as PairParams (same layout).
 template <typename T, int DIM>
 __device__ __forceinline__ const PairParams<T, DIM>& one_box_params(const Dev& d) {
-  static_assert(sizeof(PairParams<double, DIM>) == 10 * sizeof(double) &&
-                    sizeof(PairParams<float, DIM>) == 10 * sizeof(float),
+  static_assert(sizeof(PairParams<double, DIM>) == 12 * sizeof(double) &&
+                    sizeof(PairParams<float, DIM>) == 12 * sizeof(float),
                 "PairParams layout");
   if constexpr (sizeof(T) == 8)
     return *reinterpret_cast<const PairParams<T, DIM>*>(d.pc.L);
