@@ -5,7 +5,11 @@
 // The 256 x 256 layers (forward, input gradient and weight gradient) run on the tensor
 // cores through sph_tc_gemm.cuh (tcgen05, accumulators in TMEM); the 6-wide input layer
 // and the 4-wide output layer are a few hundred multiply-adds per sample and run on the
-// CUDA cores.  Every reduction has a fixed order: training is bit-reproducible.
+// CUDA cores.  One kernel takes 128 samples of a head through all four layers, one takes
+// them back through them (k_forward, k_backward); the weight gradients of both 256 x 256
+// layers are one GEMM launch, and one kernel sums their slices, updates the parameters and
+// rounds the new weights (k_update).  Every reduction has a fixed order: training is
+// bit-reproducible.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -14,6 +18,7 @@
 #include <cstring>
 #include <algorithm>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "sph_mlp.h"
@@ -37,32 +42,390 @@ constexpr int OFF_B4 = OFF_W4 + OUT * HID;
 constexpr int NPARAM = OFF_B4 + OUT;
 static_assert(NPARAM == SPH_MLP_NPARAMS, "parameter count");
 
-__device__ __forceinline__ float gelu(float z) {
-  return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
-}
-__device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) +
-         z * expf(-0.5f * z * z) * 0.39894228040143268f;
+// ---- the network's passes: one CTA carries 128 samples of one head through its layers ----
+//
+// The 128 x 256 activations live in shared memory as the next layer's A operand (four K
+// chunks of 64 in the canonical layout); the 256 x 256 weights stream through a second
+// region, four chunks of 32 KB, each layer's copied while the CUDA cores work on the layer
+// before.  16 warps: warp w takes TMEM lanes (samples) 32 (w % 4) .. + 31 and columns
+// 64 (w / 4) .. + 63, so a thread holds 64 neurons of one sample, the K chunk w / 4.
+//
+// R > 1: a CTA takes 128 / R samples, each in R rows of the operand (the tensor cores are nearly
+// idle), and a thread 64 / R neurons of its row's sample, so that a batch of few tiles (8 per
+// head at 1024 samples) spreads its GELUs over R times as many SMs.  R is chosen so that the
+// tiles fit one wave (net_rep).
+// What bounds it is the GELU arithmetic (erff) of 3 x 256 neurons per sample on the CUDA
+// cores, 36 instructions each (77 M of them for 20,011 points and 5 heads: issue half of the
+// cycles), and the weights each tile reads from L2 (256 KB).  Measured there, prediction by
+// all heads: 2.29 ms with a kernel per layer, the activations in memory between them and 1024
+// samples per pass, 0.18 ms so.  A training step (5 heads, batch 1024): 373 us in 15 launches,
+// 115 us in 5.
+constexpr int kNetThreads = 512;
+constexpr int kNetA = tc::kTileM * HID * 2;       // bytes of the activations
+constexpr int kNetChunkA = tc::kTileM * tc::kChunkK * 2;
+constexpr int kNetChunkW = HID * tc::kChunkK * 2;
+constexpr int kNetW = HID * HID * 2;              // bytes of one layer's weights
+constexpr int kNetChunks = HID / tc::kChunkK;
+static_assert(kNetChunks == 4 && kNetThreads == 128 * kNetChunks, "a K chunk per four warps");
+struct NetSmall {
+  float w1[HID][8];   // W1 row and its bias: w[0..5], b, 0
+  float w4[HID][4];   // W4 by column
+  float b2[HID], b3[HID], b4[4];
+  float4 red[kNetChunks][tc::kTileM];  // output sums of the four column groups
+  uint64_t bar;
+  uint32_t tmem;
+};
+constexpr int kNetSmem = kNetA + kNetW + (int)sizeof(NetSmall);
+static_assert(kNetSmem <= 227 * 1024, "shared memory of one CTA");
+
+// Copies a 256 x 256 bf16 matrix (rows of 256) into the four chunks at dst, asynchronously:
+// eight lanes fill the eight 16-byte rows of a core matrix (no bank conflicts), four such
+// groups take 64 consecutive bytes of each row.
+__device__ __forceinline__ void net_load_weights(uint8_t* dst, const __nv_bfloat16* w) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int q = warp; q < (HID / 8) * (HID / 32); q += kNetThreads / 32) {
+    const int row = (q >> 3) * 8 + (lane & 7), k8 = (q & 7) * 4 + (lane >> 3);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                     tc::smem_u32(dst + (k8 >> 3) * kNetChunkW + tc::core_offset(row, k8 & 7))),
+                 "l"(w + (size_t)row * HID + k8 * 8)
+                 : "memory");
+  }
 }
 
-// Epilogues of the tensor-core GEMM (one thread = one row of the 128 x N tile).
-enum Epi { kEpiStore = 0, kEpiForward = 1, kEpiBackward = 2 };
-struct EpiArgs {
-  float* C;                 // kEpiStore: FP32 result, ldc = N
-  long long strideC;
-  long long strideSplit;    // kEpiStore with split K: distance between the slices' results
-  const float* bias;        // kEpiForward: + bias[col], then GELU
-  long long strideBias;
-  const float* Zin;         // kEpiBackward: GELU'(Zin) of the layer below
-  long long strideZ;
-  float* Zout;              // kEpiForward: pre-activation (FP32) kept for the backward pass
-  __nv_bfloat16* H;         // activation (bf16), row-major
-  __nv_bfloat16* Ht;        // the same, transposed (column-major), leading dimension M
-  long long strideH;
+// Starts the layer's product: accumulator (128 x 256, FP32, TMEM) = A . W^T, once every thread's
+// shared-memory writes and copies have landed.  Returns false if its completion was not
+// observed in time (after a second bounded wait, which lets the MMAs that write TMEM finish).
+__device__ __forceinline__ bool net_product(uint8_t* smem, NetSmall* s, uint32_t parity) {
+  tc::cp_async_wait_all();
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (threadIdx.x == 0) {
+    const uint32_t idesc = tc::idesc_bf16_f32(tc::kTileM, HID);
+    const uint32_t sa = tc::smem_u32(smem), sw = sa + kNetA;
+#pragma unroll
+    for (int c = 0; c < kNetChunks; ++c)
+#pragma unroll
+      for (int q = 0; q < tc::kChunkK / 16; ++q)
+        tc::mma_bf16(s->tmem, tc::smem_desc(sa + c * kNetChunkA + q * 256),
+                     tc::smem_desc(sw + c * kNetChunkW + q * 256), idesc, c > 0 || q > 0 ? 1 : 0);
+    tc::mma_commit(&s->bar);
+  }
+  const bool ok = __syncthreads_and(tc::mbar_wait(&s->bar, parity) ? 1 : 0) != 0;
+  if (!ok) tc::mbar_wait(&s->bar, parity);
+  tc::fence_after_sync();
+  return ok;
+}
+
+__device__ __forceinline__ void net_open(NetSmall* s) {
+  if (threadIdx.x < 32) tc::tmem_alloc(&s->tmem, tc::kTmemCols);
+  if (threadIdx.x == 0) tc::mbar_init(&s->bar, 1);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+}
+__device__ __forceinline__ void net_close(NetSmall* s, bool ok, int* err) {
+  tc::cp_async_wait_all();
+  if (!ok && threadIdx.x == 0) atomicExch(err, 1);
+  tc::fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    tc::fence_after_sync();
+    tc::tmem_free(s->tmem, tc::kTmemCols);
+  }
+}
+
+// Stores 8 activations of a sample, columns 8 k8 .. + 7 of chunk c, into its rows of the A
+// operand.
+template <int R>
+__device__ __forceinline__ void net_store8(uint8_t* smem, int c, int sample, int k8,
+                                           const __nv_bfloat16 (&h)[8]) {
+#pragma unroll
+  for (int d = 0; d < R; ++d)
+    *reinterpret_cast<uint4*>(smem + c * kNetChunkA +
+                              tc::core_offset(sample + d * (tc::kTileM / R), k8)) =
+        *reinterpret_cast<const uint4*>(h);
+}
+
+// Reads this thread's 64 / R accumulator columns 16 at a time, the next 16 in flight while
+// `use(k8, v)` works on the ones before (v: 8 columns from 8 k8 on).
+template <int R, typename F>
+__device__ __forceinline__ void net_columns(uint32_t tm, F use) {
+  constexpr int kN = 4 / R;  // groups of 16 columns
+  uint32_t r[2][16];
+  tc::tmem_ld16_start(tm, r[0]);
+  tc::tmem_ld16_finish(r[0]);
+#pragma unroll
+  for (int k = 0; k < kN; ++k) {
+    if (k + 1 < kN) tc::tmem_ld16_start(tm + 16 * (k + 1), r[(k + 1) & 1]);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = __uint_as_float(r[k & 1][8 * p + q]);
+      use(2 * k + p, v);
+    }
+    if (k + 1 < kN) tc::tmem_ld16_finish(r[(k + 1) & 1]);
+  }
+}
+
+struct NetArgs {
+  const float* x;       // n x IN
+  const float* y;       // targets (training)
+  const float* params;  // every head's FP32 parameters
+  const __nv_bfloat16 *w1b, *wa, *wb, *w4b;  // forward: W2, W3; backward: W3^T, W2^T
+  int n, heads;         // samples (a multiple of 128), heads
+  float* out;           // heads x n x OUT
+  // training: slopes GELU'(z) of the three layers, by tile, column group of 4 and sample
+  // (float4 index ((head * tiles + tile) * 64 + column / 4) * 128 + sample); activations and
+  // their gradients transposed (heads x 256 x n); dL/dout; squared errors
+  float *g1, *g2, *g3;
+  __nv_bfloat16 *t1, *t2, *t3;
+  float *dout, *sqerr;
+  int* err;
 };
 
-template <int EPI>
-__global__ void __launch_bounds__(128, 1) k_gemm(GemmArgs g, EpiArgs e) {
+// z = W1 x + b1, then h = GELU(W2 GELU(z) + b2), GELU(W3 h + b3), out = W4 h + b4.  A CTA takes
+// consecutive tiles of 128 samples (mostly of one head).  TRAIN: also writes what the backward
+// pass needs, with the targets' squared errors and dL/dout.
+template <bool TRAIN, int R>
+__global__ void __launch_bounds__(kNetThreads, 1) k_forward(NetArgs a) {
+  constexpr int kS = tc::kTileM / R;  // samples per tile
+  extern __shared__ __align__(1024) uint8_t smem[];
+  NetSmall* s = reinterpret_cast<NetSmall*>(smem + kNetA + kNetW);
+  uint8_t* wsm = smem + kNetA;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int arow = 32 * (warp & 3) + lane, grp = warp >> 2;  // operand row, K chunk
+  const int row = arow % kS, sub8 = arow / kS * (8 / R);     // sample, first 8 columns of its own
+  const int tiles = a.n / kS, total = tiles * a.heads;
+  const int t0 = (int)((long long)blockIdx.x * total / gridDim.x);
+  const int t1 = (int)((long long)(blockIdx.x + 1) * total / gridDim.x);
+  if (t0 >= t1) return;
+  net_open(s);
+  const uint32_t tm = s->tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 * grp + 8 * sub8;
+  net_load_weights(wsm, a.wa + (size_t)(t0 / tiles) * HID * HID);
+  int loaded = -1;
+  uint32_t parity = 0;
+  bool ok = true;
+  for (int t = t0; t < t1; ++t) {
+    const int head = t / tiles, b = (t % tiles) * kS + row;
+    if (head != loaded) {
+      __syncthreads();  // the last tile's readers
+      const float* P = a.params + (size_t)head * NPARAM;
+      for (int j = threadIdx.x; j < HID; j += kNetThreads) {
+#pragma unroll
+        for (int i = 0; i < IN; ++i)
+          s->w1[j][i] = __bfloat162float(a.w1b[(size_t)head * HID * IN + j * IN + i]);
+        s->w1[j][6] = P[OFF_B1 + j];
+        s->b2[j] = P[OFF_B2 + j];
+        s->b3[j] = P[OFF_B3 + j];
+#pragma unroll
+        for (int o = 0; o < OUT; ++o)
+          s->w4[j][o] = __bfloat162float(a.w4b[(size_t)head * OUT * HID + o * HID + j]);
+      }
+      if (threadIdx.x < OUT) s->b4[threadIdx.x] = P[OFF_B4 + threadIdx.x];
+      loaded = head;
+      __syncthreads();
+    }
+    const size_t gbase = ((size_t)t * 64 + 16 * grp) * kS + row;          // slopes, float4
+    const size_t tbase = ((size_t)head * HID + 64 * grp) * a.n + b;       // transposed
+    float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    // 8 neurons: pre-activations z -> activations into the A operand (and the backward
+    // pass's arrays); last: the output layer's sums instead of an operand
+    auto activate = [&](const float (&z)[8], int k, float* g, __nv_bfloat16* ht, bool last) {
+      const int k8 = sub8 + k;
+      __nv_bfloat16 h[8];
+      float sl[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float e = erff(z[q] * 0.70710678118654752f);
+        h[q] = __float2bfloat16(0.5f * z[q] * (1.0f + e));
+        if (TRAIN)
+          sl[q] = 0.5f * (1.0f + e) + z[q] * expf(-0.5f * z[q] * z[q]) * 0.39894228040143268f;
+        if (!TRAIN && last) {
+          const float4 w = *reinterpret_cast<const float4*>(s->w4[64 * grp + 8 * k8 + q]);
+          const float hq = __bfloat162float(h[q]);
+          o4.x = fmaf(w.x, hq, o4.x);
+          o4.y = fmaf(w.y, hq, o4.y);
+          o4.z = fmaf(w.z, hq, o4.z);
+          o4.w = fmaf(w.w, hq, o4.w);
+        }
+      }
+      if (!last || TRAIN) net_store8<R>(smem, grp, row, k8, h);
+      if (TRAIN) {
+        float4* gp = reinterpret_cast<float4*>(g) + gbase + (size_t)(2 * k8) * kS;
+        gp[0] = make_float4(sl[0], sl[1], sl[2], sl[3]);
+        gp[kS] = make_float4(sl[4], sl[5], sl[6], sl[7]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) ht[tbase + (size_t)(8 * k8 + q) * a.n] = h[q];
+      }
+    };
+    {
+      float x[IN];
+#pragma unroll
+      for (int i = 0; i < IN; ++i) x[i] = a.x[(size_t)b * IN + i];  // any float alignment
+#pragma unroll 1
+      for (int k = 0; k < 8 / R; ++k) {
+        float z[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float* w = s->w1[64 * grp + 8 * (sub8 + k) + q];
+          const float4 u = *reinterpret_cast<const float4*>(w);
+          const float4 v = *reinterpret_cast<const float4*>(w + 4);
+          z[q] = fmaf(v.y, x[5], fmaf(v.x, x[4], fmaf(u.w, x[3], fmaf(u.z, x[2],
+                 fmaf(u.y, x[1], fmaf(u.x, x[0], v.z))))));
+        }
+        activate(z, k, a.g1, a.t1, false);
+      }
+    }
+    ok = net_product(smem, s, parity);
+    parity ^= 1;
+    if (!ok) break;
+    net_load_weights(wsm, a.wb + (size_t)head * HID * HID);
+    net_columns<R>(tm, [&](int k, const float (&v)[8]) {
+      float z[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) z[q] = v[q] + s->b2[64 * grp + 8 * (sub8 + k) + q];
+      activate(z, k, a.g2, a.t2, false);
+    });
+    ok = net_product(smem, s, parity);
+    parity ^= 1;
+    if (!ok) break;
+    if (t + 1 < t1) net_load_weights(wsm, a.wa + (size_t)((t + 1) / tiles) * HID * HID);
+    net_columns<R>(tm, [&](int k, const float (&v)[8]) {
+      float z[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) z[q] = v[q] + s->b3[64 * grp + 8 * (sub8 + k) + q];
+      activate(z, k, a.g3, a.t3, true);
+    });
+    const size_t at = (size_t)head * a.n + b;
+    if (!TRAIN) {
+      s->red[grp][arow] = o4;
+      __syncthreads();
+      if (grp == 0 && arow < kS) {
+        float4 g4[kNetChunks];  // the sums of the sample's columns 64 c .. + 63
+#pragma unroll
+        for (int c = 0; c < kNetChunks; ++c) {
+          g4[c] = s->red[c][row];
+#pragma unroll
+          for (int d = 1; d < R; ++d) {
+            const float4 u = s->red[c][row + d * kS];
+            g4[c] = make_float4(g4[c].x + u.x, g4[c].y + u.y, g4[c].z + u.z, g4[c].w + u.w);
+          }
+        }
+        float* o = a.out + at * OUT;  // any float alignment
+        o[0] = ((g4[0].x + g4[1].x) + (g4[2].x + g4[3].x)) + s->b4[0];
+        o[1] = ((g4[0].y + g4[1].y) + (g4[2].y + g4[3].y)) + s->b4[1];
+        o[2] = ((g4[0].z + g4[1].z) + (g4[2].z + g4[3].z)) + s->b4[2];
+        o[3] = ((g4[0].w + g4[1].w) + (g4[2].w + g4[3].w)) + s->b4[3];
+      }
+    } else {
+      // output `grp` of the sample, summed over the neurons in their order
+      __syncthreads();
+      float* red = reinterpret_cast<float*>(s->red);
+      if (arow < kS) {
+      float acc = 0.0f;
+      for (int c = 0; c < kNetChunks; ++c)
+#pragma unroll 2
+        for (int k8 = 0; k8 < 8; ++k8) {
+          const uint4 u = *reinterpret_cast<const uint4*>(smem + c * kNetChunkA + tc::core_offset(row, k8));
+          const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 h = __bfloat1622float2(h2[q]);
+            acc = fmaf(s->w4[64 * c + 8 * k8 + 2 * q][grp], h.x, acc);
+            acc = fmaf(s->w4[64 * c + 8 * k8 + 2 * q + 1][grp], h.y, acc);
+          }
+        }
+      const float r = acc + s->b4[grp], e = r - a.y[(size_t)b * OUT + grp];
+      a.dout[at * OUT + grp] = 2.0f * e / (float)(a.n * OUT);
+      red[4 * row + grp] = e;
+      }
+      __syncthreads();
+      if (grp == 0 && arow < kS) {
+        float se = 0.0f;
+#pragma unroll
+        for (int o = 0; o < OUT; ++o) se += red[4 * row + o] * red[4 * row + o];
+        a.sqerr[at] = se;
+      }
+    }
+  }
+  net_close(s, ok, a.err);
+}
+
+// dz3 = (W4^T dout) GELU'(z3), dz2 = (dz3 W3) GELU'(z2), dz1 = (dz2 W2) GELU'(z1), each written
+// transposed (t3, t2, t1).
+template <int R>
+__global__ void __launch_bounds__(kNetThreads, 1) k_backward(NetArgs a) {
+  constexpr int kS = tc::kTileM / R;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  NetSmall* s = reinterpret_cast<NetSmall*>(smem + kNetA + kNetW);
+  uint8_t* wsm = smem + kNetA;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int arow = 32 * (warp & 3) + lane, grp = warp >> 2;
+  const int row = arow % kS, sub8 = arow / kS * (8 / R);
+  const int tiles = a.n / kS;
+  const int t = blockIdx.x, head = t / tiles, b = (t % tiles) * kS + row;
+  net_open(s);
+  const uint32_t tm = s->tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 * grp + 8 * sub8;
+  net_load_weights(wsm, a.wa + (size_t)head * HID * HID);
+  for (int j = threadIdx.x; j < HID; j += kNetThreads)
+#pragma unroll
+    for (int o = 0; o < OUT; ++o)
+      s->w4[j][o] = __bfloat162float(a.w4b[(size_t)head * OUT * HID + o * HID + j]);
+  __syncthreads();
+  const size_t gbase = ((size_t)t * 64 + 16 * grp) * kS + row;
+  const size_t tbase = ((size_t)head * HID + 64 * grp) * a.n + b;
+  auto back = [&](const float (&v)[8], int k, const float* g, __nv_bfloat16* dzt, bool last) {
+    const int k8 = sub8 + k;
+    const float4* gp = reinterpret_cast<const float4*>(g) + gbase + (size_t)(2 * k8) * kS;
+    const float4 u = gp[0], w = gp[kS];
+    const float sl[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+    __nv_bfloat16 h[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      h[q] = __float2bfloat16(v[q] * sl[q]);
+      dzt[tbase + (size_t)(8 * k8 + q) * a.n] = h[q];
+    }
+    if (!last) net_store8<R>(smem, grp, row, k8, h);
+  };
+  const float4 d = reinterpret_cast<const float4*>(a.dout)[(size_t)head * a.n + b];
+#pragma unroll 1
+  for (int k = 0; k < 8 / R; ++k) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4 w = *reinterpret_cast<const float4*>(s->w4[64 * grp + 8 * (sub8 + k) + q]);
+      v[q] = fmaf(d.w, w.w, fmaf(d.z, w.z, fmaf(d.y, w.y, fmaf(d.x, w.x, 0.0f))));
+    }
+    back(v, k, a.g3, a.t3, false);
+  }
+  bool ok = net_product(smem, s, 0);
+  if (ok) {
+    net_load_weights(wsm, a.wb + (size_t)head * HID * HID);
+    net_columns<R>(tm, [&](int k, const float (&v)[8]) { back(v, k, a.g2, a.t2, false); });
+    ok = net_product(smem, s, 1);
+  }
+  if (ok) {
+    net_columns<R>(tm, [&](int k, const float (&v)[8]) { back(v, k, a.g1, a.t1, true); });
+  }
+  net_close(s, ok, a.err);
+}
+
+// Weight gradients of both 256 x 256 layers, K = the batch split over `splits` CTAs per output
+// tile (2 tiles per head and layer leave most SMs idle otherwise): blockIdx.z = layer * splits
+// + slice, slices summed in order by k_update.
+// Two CTAs share an SM (2 x 96 KB of stages, 2 x 256 TMEM columns).
+constexpr int kWgradSmem = 2 * tc::kStageBytes;
+constexpr int kMaxSplits = 8;  // slices of the K = batch reduction, at most
+struct WgradArgs {
+  const __nv_bfloat16 *dz[2], *h[2];  // transposed, heads x 256 x B
+  float* ws;                          // (layer * splits + slice) x heads x 256 x 256
+  int B, splits;
+  int* err;
+};
+__global__ void __launch_bounds__(128, 2) k_wgrad(WgradArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t bar[2];
   __shared__ uint32_t tmem_sh;
@@ -76,46 +439,29 @@ __global__ void __launch_bounds__(128, 1) k_gemm(GemmArgs g, EpiArgs e) {
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_sh;
-  const bool ok = __syncthreads_and(tc::gemm_mainloop(g, smem, bar, tmem));
+  const int layer = (int)blockIdx.z / a.splits;
+  GemmArgs g;
+  g.A = layer ? a.dz[1] : a.dz[0];
+  g.B = layer ? a.h[1] : a.h[0];
+  g.strideA = g.strideB = (long long)a.B * HID;
+  g.lda = g.ldb = a.B;
+  g.M = g.N = g.ntile = HID;
+  g.K = a.B;
+  g.err = a.err;
+  const bool ok = __syncthreads_and(
+      tc::gemm_mainloop(g, smem, bar, tmem, (int)blockIdx.z % a.splits, a.splits));
   if (ok) {
-    const int head = blockIdx.y;
-    const int row = tc::tile_m0(g) + threadIdx.x, n0 = tc::tile_n0(g);
-    const int N = g.N, M = g.M;
-    for (int t0 = 0; t0 < g.ntile; t0 += 16) {
+    const int row = tc::tile_m0(g) + threadIdx.x;
+    float* c = a.ws + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * HID + row) * HID;
+    for (int c0 = 0; c0 < HID; c0 += 16) {
       float v[16];
-      tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)t0, v);
-      const int c0 = n0 + t0;  // output column
-      if (EPI == kEpiStore) {
-        float* c = e.C + blockIdx.z * e.strideSplit + head * e.strideC + (size_t)row * N + c0;
+      tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-        for (int q = 0; q < 16; q += 4)
-          *reinterpret_cast<float4*>(c + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-      } else {
-        __nv_bfloat16 hv[16];
-        if (EPI == kEpiForward) {
-          const float* bias = e.bias + head * e.strideBias + c0;
-          float* z = e.Zout + head * e.strideZ + (size_t)row * N + c0;
-#pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            const float zz = v[q] + bias[q];
-            z[q] = zz;
-            hv[q] = __float2bfloat16(gelu(zz));
-          }
-        } else {
-          const float* z = e.Zin + head * e.strideZ + (size_t)row * N + c0;
-#pragma unroll
-          for (int q = 0; q < 16; ++q) hv[q] = __float2bfloat16(v[q] * gelu_grad(z[q]));
-        }
-        __nv_bfloat16* h = e.H + head * e.strideH + (size_t)row * N + c0;
-#pragma unroll
-        for (int q = 0; q < 16; q += 8) *reinterpret_cast<uint4*>(h + q) = *reinterpret_cast<uint4*>(hv + q);
-        __nv_bfloat16* ht = e.Ht + head * e.strideH;
-#pragma unroll
-        for (int q = 0; q < 16; ++q) ht[(size_t)(c0 + q) * M + row] = hv[q];
-      }
+      for (int q = 0; q < 16; q += 4)
+        *reinterpret_cast<float4*>(c + c0 + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
     }
   } else if (threadIdx.x == 0) {
-    atomicExch(g.err, 1);
+    atomicExch(a.err, 1);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -125,185 +471,178 @@ __global__ void __launch_bounds__(128, 1) k_gemm(GemmArgs g, EpiArgs e) {
   }
 }
 
-// Sum of the split-K slices of a weight gradient in slice order (a fixed order: training
-// stays bit-reproducible): C[h * strideC + i] = sum over s of ws[(s * heads + h) * MN + i].
-__global__ void k_sum_splits(const float* __restrict__ ws, int splits, int heads, int MN,
-                             float* __restrict__ C, long long strideC) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, h = blockIdx.y;
-  if (i >= MN) return;
-  float acc = ws[(size_t)h * MN + i];
-  for (int s = 1; s < splits; ++s) acc += ws[((size_t)s * heads + h) * MN + i];
-  C[h * strideC + i] = acc;
-}
-
-// ---- CUDA-core layers (6-wide input, 4-wide output) ----
-
-// z1 = W1 x + b1, h1 = GELU(z1): thread per (sample, neuron), head = blockIdx.y.
-__global__ void k_layer1(const float* __restrict__ x, int B, const float* __restrict__ params,
-                         const __nv_bfloat16* __restrict__ w1b, float* Z1, __nv_bfloat16* H1,
-                         __nv_bfloat16* H1t) {
-  const int head = blockIdx.y;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= B * HID) return;
-  const int b = t / HID, j = t % HID;
-  const float* P = params + (size_t)head * NPARAM;
-  const __nv_bfloat16* w = w1b + (size_t)head * HID * IN + j * IN;
-  float z = P[OFF_B1 + j];
+// The gradients that are not 256 x 256: dW4[.][j], dW1[j][.], db1[j], db2[j], db3[j] of neuron j
+// and db4.  A lane per gradient, 16 per neuron, 16 neurons per block; every gradient is one
+// chain s = v u + s over the batch in order, with v one of the neuron's (transposed) activations
+// or gradients and u one of dout, x or 1, staged for the whole block 128 samples at a time.
+// What bounds it is the chain itself, 1024 dependent multiply-adds; a thread per gradient that
+// fetched both factors for each sample took 172 us of a 373 us step at batch 1024 (5 heads).
+constexpr int kSgNeurons = 16, kSgBatch = 128;
+__global__ void __launch_bounds__(256) k_small_grads(const float* __restrict__ dout,
+                                                     const __nv_bfloat16* __restrict__ h3t,
+                                                     const __nv_bfloat16* __restrict__ dz1t,
+                                                     const __nv_bfloat16* __restrict__ dz2t,
+                                                     const __nv_bfloat16* __restrict__ dz3t,
+                                                     const float* __restrict__ x, int B,
+                                                     float* grads) {
+  __shared__ float su[kSgBatch][16];                                  // dout (4), x (6), 1
+  __shared__ __align__(16) __nv_bfloat16 sv[kSgNeurons][5][kSgBatch + 8];  // h3, dz1, dz2, dz3, 1
+  const int head = blockIdx.y, q = threadIdx.x & 15, nj = threadIdx.x >> 4;
+  const int j0 = blockIdx.x * kSgNeurons, j = j0 + nj;
+  // chain q of the neuron: dW4 0..3, dW1 4..9, db1..3 10..12, db4 (two neurons' last lanes)
+  const int o4 = (j & 1) * 3 + q - 13;  // db4 output of lanes 13..15 of neurons 0 and 1
+  const int src = q < 4 ? 0 : q < 11 ? 1 : q == 11 ? 2 : q == 12 ? 3 : 4;
+  const int col = q < 10 ? q : q < 13 ? 10 : min(o4, 3);
+  for (int k = threadIdx.x; k < kSgNeurons * (kSgBatch + 8); k += 256)
+    sv[k / (kSgBatch + 8)][4][k % (kSgBatch + 8)] = __float2bfloat16(1.0f);
+  const __nv_bfloat16* const arrays[4] = {h3t, dz1t, dz2t, dz3t};
+  // staged by this thread: 8 factors u (column tc of samples tr + 16 m) and 8 samples of each of
+  // its neuron's arrays, fetched while the samples before are summed
+  const int tc = threadIdx.x & 15, tr = threadIdx.x >> 4;
+  float ru[8];
+  uint4 rv[4];
+  auto fetch = [&](int b0) {
 #pragma unroll
-  for (int i = 0; i < IN; ++i) z = fmaf(__bfloat162float(w[i]), x[(size_t)b * IN + i], z);
-  const size_t o = (size_t)head * B * HID;
-  Z1[o + (size_t)b * HID + j] = z;
-  const __nv_bfloat16 h = __float2bfloat16(gelu(z));
-  H1[o + (size_t)b * HID + j] = h;
-  H1t[o + (size_t)j * B + b] = h;
-}
-
-// out = W4 h3 + b4 and, with targets, the squared error and dL/dout: thread per sample.
-__global__ void k_layer4(const __nv_bfloat16* __restrict__ H3, int B,
-                         const float* __restrict__ params, const __nv_bfloat16* __restrict__ w4b,
-                         const float* __restrict__ y, float* out, float* dout, float* sqerr) {
-  const int head = blockIdx.y;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  const float* P = params + (size_t)head * NPARAM;
-  const __nv_bfloat16* h = H3 + (size_t)head * B * HID + (size_t)b * HID;
-  const __nv_bfloat16* w = w4b + (size_t)head * OUT * HID;
-  float acc[OUT];
+    for (int m = 0; m < 8; ++m) {
+      const int b = b0 + tr + 16 * m;
+      ru[m] = tc < OUT ? dout[((size_t)head * B + b) * OUT + tc]
+              : tc < OUT + IN ? x[(size_t)b * IN + tc - OUT] : 1.0f;
+    }
 #pragma unroll
-  for (int o = 0; o < OUT; ++o) acc[o] = 0.0f;
-  for (int k = 0; k < HID; ++k) {
-    const float hk = __bfloat162float(h[k]);
+    for (int m = 0; m < 4; ++m)
+      rv[m] = *reinterpret_cast<const uint4*>(arrays[m] + ((size_t)head * HID + j0 + tr) * B + b0 +
+                                              8 * tc);
+  };
+  fetch(0);
+  float s = 0.0f;
+  for (int b0 = 0; b0 < B; b0 += kSgBatch) {
+    __syncthreads();
 #pragma unroll
-    for (int o = 0; o < OUT; ++o) acc[o] = fmaf(__bfloat162float(w[o * HID + k]), hk, acc[o]);
-  }
-  float se = 0.0f;
+    for (int m = 0; m < 8; ++m) su[tr + 16 * m][tc] = ru[m];
 #pragma unroll
-  for (int o = 0; o < OUT; ++o) {
-    const float v = acc[o] + P[OFF_B4 + o];
-    out[((size_t)head * B + b) * OUT + o] = v;
-    if (y) {
-      const float r = v - y[(size_t)b * OUT + o];
-      se += r * r;
-      dout[((size_t)head * B + b) * OUT + o] = 2.0f * r / (float)(B * OUT);
+    for (int m = 0; m < 4; ++m) *reinterpret_cast<uint4*>(&sv[tr][m][8 * tc]) = rv[m];
+    __syncthreads();
+    if (b0 + kSgBatch < B) fetch(b0 + kSgBatch);
+#pragma unroll 2
+    for (int b = 0; b < kSgBatch; b += 8) {
+      const uint4 u = *reinterpret_cast<const uint4*>(&sv[nj][src][b]);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const float2 v = __bfloat1622float2(h2[p]);
+        s = fmaf(v.x, su[b + 2 * p][col], s);
+        s = fmaf(v.y, su[b + 2 * p + 1][col], s);
+      }
     }
   }
-  if (y) sqerr[(size_t)head * B + b] = se;
-}
-
-// dz3 = (W4^T dout) * GELU'(z3): thread per (sample, neuron).
-__global__ void k_layer4_back(const float* __restrict__ dout, int B,
-                              const __nv_bfloat16* __restrict__ w4b, const float* __restrict__ Z3,
-                              __nv_bfloat16* DZ3, __nv_bfloat16* DZ3t) {
-  const int head = blockIdx.y;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= B * HID) return;
-  const int b = t / HID, k = t % HID;
-  const float* d = dout + ((size_t)head * B + b) * OUT;
-  const __nv_bfloat16* w = w4b + (size_t)head * OUT * HID;
-  float g = 0.0f;
-#pragma unroll
-  for (int o = 0; o < OUT; ++o) g = fmaf(d[o], __bfloat162float(w[o * HID + k]), g);
-  const size_t off = (size_t)head * B * HID;
-  const __nv_bfloat16 v = __float2bfloat16(g * gelu_grad(Z3[off + (size_t)b * HID + k]));
-  DZ3[off + (size_t)b * HID + k] = v;
-  DZ3t[off + (size_t)k * B + b] = v;
-}
-
-// Small weight gradients, fixed summation order over the batch: thread per output
-// element.  dW4[o][k] = sum_b dout[b][o] h3[b][k], db4[o] = sum_b dout[b][o];
-// dW1[j][i] = sum_b dz1[b][j] x[b][i], db1[j] = sum_b dz1[b][j];
-// db (hidden) = column sums of a bf16 dz.
-__global__ void k_small_grads(const float* __restrict__ dout, const __nv_bfloat16* __restrict__ H3,
-                              const __nv_bfloat16* __restrict__ DZ1,
-                              const __nv_bfloat16* __restrict__ DZ2,
-                              const __nv_bfloat16* __restrict__ DZ3, const float* __restrict__ x,
-                              int B, float* grads) {
-  const int head = blockIdx.y;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   float* G = grads + (size_t)head * NPARAM;
-  const size_t hoff = (size_t)head * B * HID;
-  // task ranges: dW4 (OUT*HID), db4 (OUT), dW1 (HID*IN), db1, db2, db3 (HID each)
-  int r = t;
-  if (r < OUT * HID) {
-    const int o = r / HID, k = r % HID;
-    float s = 0.0f;
-    for (int b = 0; b < B; ++b)
-      s = fmaf(dout[((size_t)head * B + b) * OUT + o], __bfloat162float(H3[hoff + (size_t)b * HID + k]), s);
-    G[OFF_W4 + r] = s;
-    return;
-  }
-  r -= OUT * HID;
-  if (r < OUT) {
-    float s = 0.0f;
-    for (int b = 0; b < B; ++b) s += dout[((size_t)head * B + b) * OUT + r];
-    G[OFF_B4 + r] = s;
-    return;
-  }
-  r -= OUT;
-  if (r < HID * IN) {
-    const int j = r / IN, i = r % IN;
-    float s = 0.0f;
-    for (int b = 0; b < B; ++b)
-      s = fmaf(__bfloat162float(DZ1[hoff + (size_t)b * HID + j]), x[(size_t)b * IN + i], s);
-    G[OFF_W1 + r] = s;
-    return;
-  }
-  r -= HID * IN;
-  if (r < 3 * HID) {
-    const int which = r / HID, j = r % HID;
-    const __nv_bfloat16* DZ = which == 0 ? DZ1 : which == 1 ? DZ2 : DZ3;
-    float s = 0.0f;
-    for (int b = 0; b < B; ++b) s += __bfloat162float(DZ[hoff + (size_t)b * HID + j]);
-    G[(which == 0 ? OFF_B1 : which == 1 ? OFF_B2 : OFF_B3) + j] = s;
-  }
+  if (q < 4) G[OFF_W4 + q * HID + j] = s;
+  else if (q < 10) G[OFF_W1 + j * IN + q - 4] = s;
+  else if (q < 13) G[(q == 10 ? OFF_B1 : q == 11 ? OFF_B2 : OFF_B3) + j] = s;
+  else if (j < 2 && o4 < OUT) G[OFF_B4 + o4] = s;
 }
-constexpr int kSmallTasks = OUT * HID + OUT + HID * IN + 3 * HID;
 
-// Adam on the FP32 master parameters (all heads, all tensors in one flat array).
-__global__ void k_adam(float* params, const float* grads, float* m, float* v, int n, float lr,
-                       float b1, float b2, float eps, float bc1, float bc2) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const float g = grads[t];
-  const float mt = b1 * m[t] + (1.0f - b1) * g;
-  const float vt = b2 * v[t] + (1.0f - b2) * g * g;
+struct AdamArgs {
+  float lr, b1, b2, eps, bc1, bc2;
+};
+__device__ __forceinline__ float adam(float* params, float* m, float* v, size_t t, float g,
+                                      const AdamArgs& a) {
+  const float mt = fmaf(1.0f - a.b1, g, __fmul_rn(a.b1, m[t]));
+  const float vt = fmaf(__fmul_rn(1.0f - a.b2, g), g, __fmul_rn(a.b2, v[t]));
   m[t] = mt;
   v[t] = vt;
-  params[t] -= lr * (mt / bc1) / (sqrtf(vt / bc2) + eps);
+  const float p = params[t] - a.lr * (mt / a.bc1) / (sqrtf(vt / a.bc2) + a.eps);
+  params[t] = p;
+  return p;
 }
 
-// bf16 copies of the weights used by the kernels: W1, W4 as they are, W2 and W3 also
-// transposed (operand B of the input-gradient GEMMs).
-__global__ void k_cast_weights(const float* params, int heads, __nv_bfloat16* w1b,
-                               __nv_bfloat16* w2b, __nv_bfloat16* w2tb, __nv_bfloat16* w3b,
-                               __nv_bfloat16* w3tb, __nv_bfloat16* w4b) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int per = HID * HID;
-  if (t >= heads * per) return;
-  const int head = t / per, e = t % per, r = e / HID, c = e % HID;
-  const float* P = params + (size_t)head * NPARAM;
-  const size_t o = (size_t)head * per;
-  w2b[o + e] = __float2bfloat16(P[OFF_W2 + e]);
-  w2tb[o + (size_t)c * HID + r] = __float2bfloat16(P[OFF_W2 + e]);
-  w3b[o + e] = __float2bfloat16(P[OFF_W3 + e]);
-  w3tb[o + (size_t)c * HID + r] = __float2bfloat16(P[OFF_W3 + e]);
-  if (e < HID * IN) w1b[(size_t)head * HID * IN + e] = __float2bfloat16(P[OFF_W1 + e]);
-  if (e < OUT * HID) w4b[(size_t)head * OUT * HID + e] = __float2bfloat16(P[OFF_W4 + e]);
-}
-
-// Per-head sum of squared errors in fixed order (one block per head).
-__global__ void k_loss(const float* sqerr, int B, float* loss) {
-  __shared__ float sh[256];
-  const int head = blockIdx.x;
-  float s = 0.0f;
-  for (int b = threadIdx.x; b < B; b += blockDim.x) s += sqerr[(size_t)head * B + b];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-    if ((int)threadIdx.x < k) sh[threadIdx.x] += sh[threadIdx.x + k];
+// What is done with a head's parameters, 32 x 32 tiles of W2 and W3 per block and the others in
+// the last blocks: SUM: the weight gradients' slices summed in slice order into grads; ADAM: the
+// update of the FP32 master parameters; CAST: the bf16 copies the kernels use (W1, W4 as they
+// are, W2 and W3 also transposed, through shared memory).
+struct UpdateArgs {
+  float *params, *grads, *m, *v;
+  const float* sqerr;  // SUM: the last block of a head also sums its squared errors, B of them
+  float* loss;
+  int B;
+  const float* ws;
+  int splits;
+  __nv_bfloat16 *w1b, *w2b, *w2tb, *w3b, *w3tb, *w4b;
+  AdamArgs adam;
+};
+constexpr int kUpdTiles = 2 * (HID / 32) * (HID / 32);
+constexpr int kUpdSmall = NPARAM - 2 * HID * HID;  // the other parameters of a head
+constexpr int kUpdBlocks = kUpdTiles + (kUpdSmall + 1023) / 1024;
+template <bool SUM, bool ADAM, bool CAST>
+__global__ void __launch_bounds__(256) k_update(UpdateArgs a) {
+  __shared__ __nv_bfloat16 tile[32][34];
+  const int head = blockIdx.y;
+  const size_t base = (size_t)head * NPARAM;
+  if (SUM && blockIdx.x == kUpdBlocks) {
+    // the head's loss, in a fixed order
+    __shared__ float sh[256];
+    float s = 0.0f;
+    for (int b = threadIdx.x; b < a.B; b += 256) s += a.sqerr[(size_t)head * a.B + b];
+    sh[threadIdx.x] = s;
     __syncthreads();
+    for (int k = 128; k > 0; k >>= 1) {
+      if ((int)threadIdx.x < k) sh[threadIdx.x] += sh[threadIdx.x + k];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) a.loss[head] = sh[0] / (float)(a.B * OUT);
+    return;
   }
-  if (threadIdx.x == 0) loss[head] = sh[0] / (float)(B * OUT);
+  if ((int)blockIdx.x < kUpdTiles) {
+    const int layer = blockIdx.x / (kUpdTiles / 2), k = blockIdx.x % (kUpdTiles / 2);
+    const int r0 = (k / (HID / 32)) * 32, c0 = (k % (HID / 32)) * 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const size_t wo = (size_t)head * HID * HID;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = (r0 + w + 8 * q) * HID + c0 + lane;
+      const size_t t = base + (layer ? OFF_W3 : OFF_W2) + e;
+      float g = 0.0f;
+      if (SUM) {
+        const float* ws = a.ws + ((size_t)(layer * a.splits) * gridDim.y + head) * HID * HID + e;
+        float part[kMaxSplits];
+#pragma unroll
+        for (int sl = 0; sl < kMaxSplits; ++sl)
+          part[sl] = sl < a.splits ? ws[(size_t)sl * gridDim.y * HID * HID] : 0.0f;
+        g = part[0];
+#pragma unroll
+        for (int sl = 1; sl < kMaxSplits; ++sl)
+          if (sl < a.splits) g += part[sl];
+        a.grads[t] = g;
+      }
+      const float p = ADAM ? adam(a.params, a.m, a.v, t, g, a.adam) : CAST ? a.params[t] : 0.0f;
+      if (CAST) {
+        const __nv_bfloat16 h = __float2bfloat16(p);
+        (layer ? a.w3b : a.w2b)[wo + e] = h;
+        tile[lane][w + 8 * q] = h;
+      }
+    }
+    if (CAST) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        (layer ? a.w3tb : a.w2tb)[wo + (size_t)(c0 + w + 8 * q) * HID + r0 + lane] =
+            tile[w + 8 * q][lane];
+    }
+    return;
+  }
+  for (int u = 0; u < 4 && (ADAM || CAST); ++u) {
+    const int k = ((int)blockIdx.x - kUpdTiles) * 1024 + u * 256 + (int)threadIdx.x;
+    if (k >= kUpdSmall) return;
+    // the parameters in order, without W2 and W3
+    const int off = k < OFF_W2 ? k : k < OFF_W2 + HID ? k + HID * HID : k + 2 * HID * HID;
+    const size_t t = base + off;
+    const float p = ADAM ? adam(a.params, a.m, a.v, t, a.grads[t], a.adam) : CAST ? a.params[t] : 0.0f;
+    if (CAST) {
+      if (off < OFF_B1) a.w1b[(size_t)head * HID * IN + off] = __float2bfloat16(p);
+      if (off >= OFF_W4 && off < OFF_B4)
+        a.w4b[(size_t)head * OUT * HID + off - OFF_W4] = __float2bfloat16(p);
+    }
+  }
 }
 
 // C = A . B^T in FP32 (the tensor-core GEMM with a plain store epilogue).
@@ -322,7 +661,7 @@ __global__ void __launch_bounds__(128, 1) k_gemm_f32(GemmArgs g, float* C, int l
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_sh;
-  const bool ok = __syncthreads_and(tc::gemm_mainloop(g, smem, bar, tmem));
+  const bool ok = __syncthreads_and(tc::gemm_mainloop(g, smem, bar, tmem, 0, 1));
   if (ok) {
     const int row = tc::tile_m0(g) + threadIdx.x;
     float* c = C + blockIdx.y * strideC + (size_t)row * ldc + tc::tile_n0(g);
@@ -358,12 +697,12 @@ struct sph_mlp {
   float *params = nullptr, *grads = nullptr, *m = nullptr, *v = nullptr;
   __nv_bfloat16 *w1b = nullptr, *w2b = nullptr, *w2tb = nullptr, *w3b = nullptr, *w3tb = nullptr,
                 *w4b = nullptr;
-  float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr;
-  __nv_bfloat16 *h1 = nullptr, *h1t = nullptr, *h2 = nullptr, *h2t = nullptr, *h3 = nullptr,
-                *h3t = nullptr, *dz1 = nullptr, *dz1t = nullptr, *dz2 = nullptr, *dz2t = nullptr,
-                *dz3 = nullptr, *dz3t = nullptr;
-  float *out = nullptr, *dout = nullptr, *sqerr = nullptr, *loss = nullptr;
-  float* ws = nullptr;  // split-K slices of a weight gradient (kMaxSplits x heads x HID x HID)
+  // slopes GELU'(z) and the transposed activations and gradients of one batch
+  float *g1 = nullptr, *g2 = nullptr, *g3 = nullptr;
+  __nv_bfloat16 *h1t = nullptr, *h2t = nullptr, *h3t = nullptr, *dz1t = nullptr, *dz2t = nullptr,
+                *dz3t = nullptr;
+  float *dout = nullptr, *sqerr = nullptr, *loss = nullptr;
+  float* ws = nullptr;  // weight-gradient slices (2 x kMaxSplits x heads x HID x HID)
   int* err = nullptr;
   long long step = 0;
 };
@@ -413,119 +752,105 @@ void init_params(std::vector<float>& P, int heads, unsigned long long seed) {
     }
 }
 
-template <int EPI>
-int gemm_launch(sph_mlp* c, const __nv_bfloat16* A, long long sA, int lda, const __nv_bfloat16* B,
-                long long sB, int ldb, int M, int N, int K, const EpiArgs& e, int splits = 1) {
-  GemmArgs g;
-  g.A = A;
-  g.B = B;
-  g.strideA = sA;
-  g.strideB = sB;
-  g.lda = lda;
-  g.ldb = ldb;
-  g.M = M;
-  g.N = N;
-  g.K = K;
-  // forward and input-gradient GEMMs whose row tiles alone leave SMs idle (a 1024-sample
-  // batch: 8 row tiles x 5 heads = 40 CTAs): two column tiles per row tile
-  g.ntile = (EPI != kEpiStore && N == 256 && (M / tc::kTileM) * c->heads < c->nsm) ? 128 : N;
-  g.err = c->err;
-  k_gemm<EPI><<<dim3(M / tc::kTileM * (N / g.ntile), c->heads, splits), 128, tc::kSmemBytes,
-                 c->stream>>>(g, e);
-  return cudaGetLastError() != cudaSuccess;
+// Rows of the operand per sample: 4 or 2 where all tiles then still run at once.
+int net_rep(const sph_mlp* c, int n) {
+  const int tiles = n / tc::kTileM * c->heads;
+  return 4 * tiles <= c->nsm ? 4 : 2 * tiles <= c->nsm ? 2 : 1;
 }
 
-// Weight gradient dW = dZ^T H (M = N = HID, K = the batch) into grads + off of every head.
-// The K = batch reduction is split over up to kMaxSplits CTAs per output tile (2 tiles per
-// head leave most SMs idle otherwise); the slices are summed in order by k_sum_splits.
-constexpr int kMaxSplits = 8;
-int weight_grad(sph_mlp* c, const __nv_bfloat16* dzt, const __nv_bfloat16* ht, int B, int off) {
-  const long long act = (long long)B * HID;
+NetArgs net_args(const sph_mlp* c, const float* x, int n) {
+  NetArgs a{};
+  a.x = x;
+  a.params = c->params;
+  a.w1b = c->w1b;
+  a.w4b = c->w4b;
+  a.n = n;
+  a.heads = c->heads;
+  a.g1 = c->g1;
+  a.g2 = c->g2;
+  a.g3 = c->g3;
+  a.dout = c->dout;
+  a.sqerr = c->sqerr;
+  a.err = c->err;
+  return a;
+}
+
+int wgrad_splits(int B) {
   int splits = kMaxSplits;
   while (splits > 1 && B % (tc::kChunkK * splits) != 0) splits /= 2;
-  EpiArgs e{};
-  if (splits == 1) {
-    e.C = c->grads + off;
-    e.strideC = NPARAM;
-    return gemm_launch<kEpiStore>(c, dzt, act, B, ht, act, B, HID, HID, B, e);
-  }
-  const int MN = HID * HID;
-  e.C = c->ws;
-  e.strideC = MN;
-  e.strideSplit = (long long)c->heads * MN;
-  if (gemm_launch<kEpiStore>(c, dzt, act, B, ht, act, B, HID, HID, B, e, splits)) return 1;
-  k_sum_splits<<<dim3((MN + 255) / 256, c->heads), 256, 0, c->stream>>>(c->ws, splits, c->heads,
-                                                                          MN, c->grads + off, NPARAM);
-  return cudaGetLastError() != cudaSuccess;
+  return splits;
 }
 
-// Forward pass of every head on B samples (x: B x IN, device); with y (B x OUT) also the
-// squared errors and dL/dout.
-int forward(sph_mlp* c, const float* x, const float* y, int B) {
-  const int H = c->heads;
-  const long long act = (long long)B * HID;
-  k_layer1<<<dim3((B * HID + 255) / 256, H), 256, 0, c->stream>>>(x, B, c->params, c->w1b, c->z1,
-                                                                   c->h1, c->h1t);
-  if (cudaGetLastError() != cudaSuccess) return 1;
-  EpiArgs e{};
-  e.strideBias = NPARAM;
-  e.strideZ = act;
-  e.strideH = act;
-  e.bias = c->params + OFF_B2;
-  e.Zout = c->z2;
-  e.H = c->h2;
-  e.Ht = c->h2t;
-  if (gemm_launch<kEpiForward>(c, c->h1, act, HID, c->w2b, (long long)HID * HID, HID, B, HID, HID, e))
-    return 1;
-  e.bias = c->params + OFF_B3;
-  e.Zout = c->z3;
-  e.H = c->h3;
-  e.Ht = c->h3t;
-  if (gemm_launch<kEpiForward>(c, c->h2, act, HID, c->w3b, (long long)HID * HID, HID, B, HID, HID, e))
-    return 1;
-  k_layer4<<<dim3((B + 127) / 128, H), 128, 0, c->stream>>>(c->h3, B, c->params, c->w4b, y, c->out,
-                                                            c->dout, c->sqerr);
-  return cudaGetLastError() != cudaSuccess;
+UpdateArgs update_args(const sph_mlp* c, int splits, int B = 0) {
+  UpdateArgs u{};
+  u.sqerr = c->sqerr;
+  u.loss = c->loss;
+  u.B = B;
+  u.params = c->params;
+  u.grads = c->grads;
+  u.m = c->m;
+  u.v = c->v;
+  u.ws = c->ws;
+  u.splits = splits;
+  u.w1b = c->w1b;
+  u.w2b = c->w2b;
+  u.w2tb = c->w2tb;
+  u.w3b = c->w3b;
+  u.w3tb = c->w3tb;
+  u.w4b = c->w4b;
+  return u;
 }
 
-// Backward pass after forward(x, y): gradients of the mean squared error of every head.
-int backward(sph_mlp* c, const float* x, int B) {
-  const int H = c->heads;
-  const long long act = (long long)B * HID;
-  k_layer4_back<<<dim3((B * HID + 255) / 256, H), 256, 0, c->stream>>>(c->dout, B, c->w4b, c->z3,
-                                                                       c->dz3, c->dz3t);
+// Gradients of the mean squared error of every head on B samples, but for the sum of the
+// weight gradients' slices (k_update<true, ...>), whose number is returned in *splits.
+template <bool TRAIN>
+void forward_launch(const sph_mlp* c, const NetArgs& f, int rep) {
+  const int grid = std::min(f.n / tc::kTileM * f.heads * rep, c->nsm);
+  if (rep == 4) k_forward<TRAIN, 4><<<grid, kNetThreads, kNetSmem, c->stream>>>(f);
+  else if (rep == 2) k_forward<TRAIN, 2><<<grid, kNetThreads, kNetSmem, c->stream>>>(f);
+  else k_forward<TRAIN, 1><<<grid, kNetThreads, kNetSmem, c->stream>>>(f);
+}
+
+int backprop(sph_mlp* c, const float* x, const float* y, int B, int* splits) {
+  const int rep = net_rep(c, B), tiles = B / tc::kTileM * c->heads * rep;
+  NetArgs f = net_args(c, x, B);
+  f.y = y;
+  f.wa = c->w2b;
+  f.wb = c->w3b;
+  f.t1 = c->h1t;
+  f.t2 = c->h2t;
+  f.t3 = c->h3t;
+  forward_launch<true>(c, f, rep);
   if (cudaGetLastError() != cudaSuccess) return 1;
-  EpiArgs e{};
-  e.strideC = NPARAM;
-  e.strideZ = act;
-  e.strideH = act;
-  // dW3 = dz3^T h2, then dz2 = (dz3 W3) * GELU'(z2)
-  if (weight_grad(c, c->dz3t, c->h2t, B, OFF_W3)) return 1;
-  e.Zin = c->z2;
-  e.H = c->dz2;
-  e.Ht = c->dz2t;
-  if (gemm_launch<kEpiBackward>(c, c->dz3, act, HID, c->w3tb, (long long)HID * HID, HID, B, HID,
-                                HID, e))
-    return 1;
-  // dW2 = dz2^T h1, then dz1 = (dz2 W2) * GELU'(z1)
-  if (weight_grad(c, c->dz2t, c->h1t, B, OFF_W2)) return 1;
-  e.Zin = c->z1;
-  e.H = c->dz1;
-  e.Ht = c->dz1t;
-  if (gemm_launch<kEpiBackward>(c, c->dz2, act, HID, c->w2tb, (long long)HID * HID, HID, B, HID,
-                                HID, e))
-    return 1;
-  k_small_grads<<<dim3((kSmallTasks + 127) / 128, H), 128, 0, c->stream>>>(
-      c->dout, c->h3, c->dz1, c->dz2, c->dz3, x, B, c->grads);
+  NetArgs r = net_args(c, x, B);
+  r.wa = c->w3tb;
+  r.wb = c->w2tb;
+  r.t1 = c->dz1t;
+  r.t2 = c->dz2t;
+  r.t3 = c->dz3t;
+  if (rep == 4) k_backward<4><<<tiles, kNetThreads, kNetSmem, c->stream>>>(r);
+  else if (rep == 2) k_backward<2><<<tiles, kNetThreads, kNetSmem, c->stream>>>(r);
+  else k_backward<1><<<tiles, kNetThreads, kNetSmem, c->stream>>>(r);
   if (cudaGetLastError() != cudaSuccess) return 1;
-  k_loss<<<H, 256, 0, c->stream>>>(c->sqerr, B, c->loss);
+  // dW2 = dz2^T h1, dW3 = dz3^T h2
+  WgradArgs w{};
+  w.dz[0] = c->dz2t;
+  w.h[0] = c->h1t;
+  w.dz[1] = c->dz3t;
+  w.h[1] = c->h2t;
+  w.ws = c->ws;
+  w.B = B;
+  w.splits = *splits = wgrad_splits(B);
+  w.err = c->err;
+  k_wgrad<<<dim3(HID / tc::kTileM, c->heads, 2 * w.splits), 128, kWgradSmem, c->stream>>>(w);
+  if (cudaGetLastError() != cudaSuccess) return 1;
+  k_small_grads<<<dim3(HID / kSgNeurons, c->heads), 256, 0, c->stream>>>(
+      c->dout, c->h3t, c->dz1t, c->dz2t, c->dz3t, x, B, c->grads);
   return cudaGetLastError() != cudaSuccess;
 }
 
 int cast_weights(sph_mlp* c) {
-  const int n = c->heads * HID * HID;
-  k_cast_weights<<<(n + 255) / 256, 256, 0, c->stream>>>(c->params, c->heads, c->w1b, c->w2b,
-                                                         c->w2tb, c->w3b, c->w3tb, c->w4b);
+  k_update<false, false, true><<<dim3(kUpdBlocks, c->heads), 256, 0, c->stream>>>(update_args(c, 1));
   return cudaGetLastError() != cudaSuccess;
 }
 
@@ -605,21 +930,24 @@ sph_status sph_mlp_create(int heads, int max_batch, unsigned long long seed, int
   ok = ok && mlp_alloc(c, &c->w1b, (size_t)heads * HID * IN) && mlp_alloc(c, &c->w2b, hh) &&
        mlp_alloc(c, &c->w2tb, hh) && mlp_alloc(c, &c->w3b, hh) && mlp_alloc(c, &c->w3tb, hh) &&
        mlp_alloc(c, &c->w4b, (size_t)heads * OUT * HID);
-  ok = ok && mlp_alloc(c, &c->z1, act) && mlp_alloc(c, &c->z2, act) && mlp_alloc(c, &c->z3, act);
-  for (__nv_bfloat16** p : {&c->h1, &c->h1t, &c->h2, &c->h2t, &c->h3, &c->h3t, &c->dz1, &c->dz1t,
-                            &c->dz2, &c->dz2t, &c->dz3, &c->dz3t})
+  for (float** p : {&c->g1, &c->g2, &c->g3}) ok = ok && mlp_alloc(c, p, act);
+  for (__nv_bfloat16** p : {&c->h1t, &c->h2t, &c->h3t, &c->dz1t, &c->dz2t, &c->dz3t})
     ok = ok && mlp_alloc(c, p, act);
-  ok = ok && mlp_alloc(c, &c->out, (size_t)heads * max_batch * OUT) &&
-       mlp_alloc(c, &c->dout, (size_t)heads * max_batch * OUT) &&
+  ok = ok && mlp_alloc(c, &c->dout, (size_t)heads * max_batch * OUT) &&
        mlp_alloc(c, &c->sqerr, (size_t)heads * max_batch) && mlp_alloc(c, &c->loss, heads) &&
-       mlp_alloc(c, &c->ws, (size_t)kMaxSplits * heads * HID * HID) && mlp_alloc(c, &c->err, 1);
+       mlp_alloc(c, &c->ws, 2 * (size_t)kMaxSplits * hh) && mlp_alloc(c, &c->err, 1);
   if (!ok) {
     mlp_free(c);
     return SPH_ERR_NOMEM;
   }
-  for (const void* k : {(const void*)k_gemm<kEpiStore>, (const void*)k_gemm<kEpiForward>,
-                        (const void*)k_gemm<kEpiBackward>})
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes) !=
+  const std::pair<const void*, int> kernels[] = {
+      {(const void*)k_forward<false, 1>, kNetSmem}, {(const void*)k_forward<false, 2>, kNetSmem},
+      {(const void*)k_forward<false, 4>, kNetSmem}, {(const void*)k_forward<true, 1>, kNetSmem},
+      {(const void*)k_forward<true, 2>, kNetSmem},  {(const void*)k_forward<true, 4>, kNetSmem},
+      {(const void*)k_backward<1>, kNetSmem},       {(const void*)k_backward<2>, kNetSmem},
+      {(const void*)k_backward<4>, kNetSmem},       {(const void*)k_wgrad, kWgradSmem}};
+  for (const auto& k : kernels)
+    if (cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, k.second) !=
         cudaSuccess) {
       mlp_free(c);
       return SPH_ERR_CUDA;
@@ -666,7 +994,11 @@ sph_status sph_mlp_gradients(sph_mlp* c, const float* x, const float* y, int bat
                              float* grads_host, float* loss_host) {
   if (!c || !x || !y || !batch_ok(c, batch)) return SPH_ERR_STATE;
   cudaSetDevice(c->device);
-  if (forward(c, x, y, batch) || backward(c, x, batch)) return SPH_ERR_CUDA;
+  int splits = 1;
+  if (backprop(c, x, y, batch, &splits)) return SPH_ERR_CUDA;
+  k_update<true, false, false><<<dim3(kUpdBlocks + 1, c->heads), 256, 0, c->stream>>>(
+      update_args(c, splits, batch));
+  if (cudaGetLastError() != cudaSuccess) return SPH_ERR_CUDA;
   if (grads_host && cudaMemcpyAsync(grads_host, c->grads, (size_t)c->heads * NPARAM * sizeof(float),
                                     cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
     return SPH_ERR_CUDA;
@@ -680,15 +1012,16 @@ sph_status sph_mlp_train_step(sph_mlp* c, const float* x, const float* y, int ba
                               float* loss_host) {
   if (!c || !x || !y || !batch_ok(c, batch)) return SPH_ERR_STATE;
   cudaSetDevice(c->device);
-  if (forward(c, x, y, batch) || backward(c, x, batch)) return SPH_ERR_CUDA;
+  int splits = 1;
+  if (backprop(c, x, y, batch, &splits)) return SPH_ERR_CUDA;
   c->step++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float bc1 = 1.0f - (float)std::pow((double)b1, (double)c->step);
   const float bc2 = 1.0f - (float)std::pow((double)b2, (double)c->step);
-  const int n = c->heads * NPARAM;
-  k_adam<<<(n + 255) / 256, 256, 0, c->stream>>>(c->params, c->grads, c->m, c->v, n, lr, b1, b2,
-                                                 1e-8f, bc1, bc2);
-  if (cudaGetLastError() != cudaSuccess || cast_weights(c)) return SPH_ERR_CUDA;
+  UpdateArgs u = update_args(c, splits, batch);
+  u.adam = {lr, b1, b2, 1e-8f, bc1, bc2};
+  k_update<true, true, true><<<dim3(kUpdBlocks + 1, c->heads), 256, 0, c->stream>>>(u);
+  if (cudaGetLastError() != cudaSuccess) return SPH_ERR_CUDA;
   if (loss_host && cudaMemcpyAsync(loss_host, c->loss, (size_t)c->heads * sizeof(float),
                                    cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
     return SPH_ERR_CUDA;
@@ -699,15 +1032,12 @@ sph_status sph_mlp_train_step(sph_mlp* c, const float* x, const float* y, int ba
 sph_status sph_mlp_predict(sph_mlp* c, const float* x, int n, float* out) {
   if (!c || !x || !out || n <= 0 || n % tc::kTileM != 0) return SPH_ERR_STATE;
   cudaSetDevice(c->device);
-  for (int s = 0; s < n; s += c->max_batch) {
-    const int B = std::min(c->max_batch, n - s);
-    if (forward(c, x + (size_t)s * IN, nullptr, B)) return SPH_ERR_CUDA;
-    for (int h = 0; h < c->heads; ++h)
-      if (cudaMemcpyAsync(out + ((size_t)h * n + s) * OUT, c->out + (size_t)h * B * OUT,
-                          (size_t)B * OUT * sizeof(float), cudaMemcpyDeviceToDevice,
-                          c->stream) != cudaSuccess)
-        return SPH_ERR_CUDA;
-  }
+  NetArgs f = net_args(c, x, n);
+  f.wa = c->w2b;
+  f.wb = c->w3b;
+  f.out = out;
+  forward_launch<false>(c, f, net_rep(c, n));
+  if (cudaGetLastError() != cudaSuccess) return SPH_ERR_CUDA;
   return finish(c);
 }
 

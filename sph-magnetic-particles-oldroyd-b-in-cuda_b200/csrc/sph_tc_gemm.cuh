@@ -127,6 +127,27 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
 }
 
+// The same in two halves: the load started, and its registers ready.
+__device__ __forceinline__ void tmem_ld16_start(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16_finish(uint32_t (&r)[16]) {
+  // the registers pass through the wait, so that no use of them can be moved before it
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                 "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                 "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+
 // Operands of one GEMM launch; head h uses A + h * strideA, B + h * strideB (elements).
 struct GemmArgs {
   const __nv_bfloat16* A;
@@ -151,8 +172,10 @@ __device__ __forceinline__ int tile_n0(const GemmArgs& g) {
 // once (completed by cp_async_wait_all).
 __device__ __forceinline__ void load_chunk(uint8_t* dst, const __nv_bfloat16* src, int ld, int r0,
                                            int rows, int k0) {
+  // eight lanes fill the eight 16-byte rows of a core matrix (no bank conflicts), a warp four
+  // of them along K (64 consecutive bytes of each row)
   for (int idx = threadIdx.x; idx < rows * (kChunkK / 8); idx += blockDim.x) {
-    const int r = idx >> 3, k8 = idx & 7;
+    const int u = idx >> 5, r = (u >> 1) * 8 + (idx & 7), k8 = (u & 1) * 4 + ((idx >> 3) & 3);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
                      smem_u32(dst + core_offset(r, k8))),
                  "l"(src + (size_t)(r0 + r) * ld + k0 + k8 * 8)
@@ -164,8 +187,8 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }
 
 // The main loop: leaves the 128 x ntile FP32 accumulator of this CTA's tile in TMEM columns
-// [tmem, tmem + ntile).  With gridDim.z > 1 the CTA takes K slice blockIdx.z of gridDim.z equal
-// slices (split K; K / gridDim.z a multiple of 64).  Two stages: the copies of chunk c + 1
+// [tmem, tmem + ntile).  With split K the CTA takes K slice `slice` of `splits` equal slices
+// (K / splits a multiple of 64).  Two stages: the copies of chunk c + 1
 // are in flight while the MMAs of chunk c run; bar[s] counts the MMA completions of stage s
 // (a stage is refilled only after the MMAs that read it are done).  Returns false if an
 // MMA completion was not observed in time.
@@ -173,11 +196,11 @@ constexpr int kStageA = kTileM * kChunkK * 2;
 constexpr int kStageBytes = kStageA + kMaxN * kChunkK * 2;
 static_assert(2 * kStageBytes <= kSmemBytes, "two stages of A and B chunks");
 __device__ __forceinline__ bool gemm_mainloop(const GemmArgs& g, uint8_t* smem, uint64_t* bar,
-                                              uint32_t tmem) {
+                                              uint32_t tmem, int slice, int splits) {
   const int head = blockIdx.y;
   const int m0 = tile_m0(g), n0 = tile_n0(g);
-  const int kslice = g.K / (int)gridDim.z;
-  const int kb = (int)blockIdx.z * kslice;
+  const int kslice = g.K / splits;
+  const int kb = slice * kslice;
   const int nch = kslice / kChunkK;
   const __nv_bfloat16* A = g.A + head * g.strideA;
   const __nv_bfloat16* B = g.B + head * g.strideB;
