@@ -24,8 +24,6 @@ struct sph_ctx {
   Dev d{};
   cudaStream_t stream = nullptr;
   std::vector<void*> allocs;
-  int key_bits = 1;
-  SortScratch sort{};
   double* ke_partial = nullptr;
   double* obs_partial = nullptr;  // 2 per KE chunk
   double* obs_acc = nullptr;      // nboxes x SPH_NUM_OBS running sums
@@ -107,12 +105,6 @@ Launch launcher(sph_ctx* c) {
   return L;
 }
 
-int bits_for(int n) {
-  int b = 1;
-  while ((1 << b) < n) ++b;
-  return b;
-}
-
 void swap_state(sph_ctx* c, bool with_forces) {
   std::swap(c->d.pos, c->d.pos_b);
   std::swap(c->d.vel, c->d.vel_b);
@@ -124,6 +116,7 @@ void swap_state(sph_ctx* c, bool with_forces) {
     std::swap(c->d.dcdt, c->d.dcdt_b);
   }
   c->parity ^= 1;
+  c->d.parity = c->parity;
 }
 
 // Neighbour-list capacity: chunks with hits per particle.  A particle's candidates come
@@ -167,11 +160,15 @@ bool alloc_lists(sph_ctx* c, int cap) {
 // Reads the device error flags and their record (err_info, kErrInfoLen ints) without
 // clearing them.  Blocks on the stream.
 bool read_device_status(sph_ctx* c, unsigned* st, int* info) {
-  return cudaMemcpyAsync(st, c->d.status, sizeof(unsigned), cudaMemcpyDeviceToHost,
+  unsigned both[2] = {0u, 0u};
+  const bool ok =
+         cudaMemcpyAsync(both, c->d.status, sizeof(both), cudaMemcpyDeviceToHost,
                          c->stream) == cudaSuccess &&
          cudaMemcpyAsync(info, c->d.err_info, kErrInfoLen * sizeof(int), cudaMemcpyDeviceToHost,
                          c->stream) == cudaSuccess &&
          cudaStreamSynchronize(c->stream) == cudaSuccess;
+  *st = both[0] | both[1];
+  return ok;
 }
 
 long long failed_step(const int* info) {
@@ -200,7 +197,7 @@ sph_status check_device(sph_ctx* c) {
   int info[kErrInfoLen] = {0};
   if (!read_device_status(c, &st, info)) return cuda_fail(c, "device status");
   if (st == 0) return SPH_OK;
-  cudaMemsetAsync(c->d.status, 0, sizeof(unsigned), c->stream);
+  cudaMemsetAsync(c->d.status, 0, 2 * sizeof(unsigned), c->stream);
   return status_of(c, st, info, "");
 }
 
@@ -223,10 +220,13 @@ sph_status grow_capacity(sph_ctx* c, int needed) {
 }
 
 // ---- phases (all asynchronous) ----
-int ph_search(sph_ctx* c) {
+// moving: the search of a whole step, with the particles' half-kick and drift and the step's
+// magnetic moment in its kernels
+int ph_search(sph_ctx* c, bool moving = false) {
   Launch L = launcher(c);
   const bool permute = c->forces_live;
-  if (launch_hash(L) || launch_sort(L, c->key_bits, c->sort) || launch_reorder(L, permute))
+  if ((moving ? launch_vv1_hash(L) : launch_hash(L)) || launch_cell_sort(L, moving) ||
+      launch_reorder(L, permute))
     return 1;
   swap_state(c, permute);
   L = launcher(c);
@@ -236,8 +236,9 @@ int ph_search(sph_ctx* c) {
   return 0;
 }
 
-// fold: the fused pair pass also applies the step's second half-kick to fluid particles
-// (the step graph); the method-by-method path keeps V_Verlet_step2 separate
+// fold: also the step's second half-kick (fluid particles in the fused pair pass, colloids with
+// their forces) and its count (the step graph); the method-by-method path keeps V_Verlet_step2
+// separate
 int ph_forces(sph_ctx* c, bool fold = false) {
   Launch L = launcher(c);
   L.d.gradv = nullptr;  // the fused pass keeps the gradient in registers
@@ -249,7 +250,7 @@ int ph_forces(sph_ctx* c, bool fold = false) {
   if (launch_wall_forces(L)) return 1;
   bool pairs = false;
   for (const HostBox& hb : c->boxes) pairs = pairs || hb.p.N_colloids >= 2;
-  if (launch_colloid_forces(L, pairs ? 1 : 0)) return 1;
+  if (launch_colloid_forces(L, pairs ? 1 : 0, fold ? 1 : 0)) return 1;
   c->forces_live = true;
   c->gradv_valid = false;
   return 0;
@@ -263,17 +264,17 @@ int ph_vv1(sph_ctx* c) {
   return 0;
 }
 
-int ph_vv2(sph_ctx* c, bool folded = false) {
+int ph_vv2(sph_ctx* c) {
   Launch L = launcher(c);
-  if (launch_vv2(L, !folded) || launch_count_step(L)) return 1;
+  if (launch_vv2(L) || launch_count_step(L)) return 1;
   return 0;
 }
 
 // One full step: VV1, search, m(t), forces, VV2 (main.cu:358-432)
 int ph_step(sph_ctx* c) {
-  if (ph_vv1(c) || ph_search(c)) return 1;
-  if (launch_advance_time(launcher(c), 0)) return 1;
-  if (ph_forces(c, true) || ph_vv2(c, true)) return 1;
+  if (launch_vv1_colloids(launcher(c))) return 1;
+  c->forces_live = false;
+  if (ph_search(c, true) || ph_forces(c, true)) return 1;
   c->forces_live = true;
   return 0;
 }
@@ -335,7 +336,7 @@ sph_status search_checked(sph_ctx* c) {
   int info[kErrInfoLen] = {0};
   if (!read_device_status(c, &st, info)) return cuda_fail(c, "device status");
   if (st == 0) return SPH_OK;
-  cudaMemsetAsync(c->d.status, 0, sizeof(unsigned), c->stream);
+  cudaMemsetAsync(c->d.status, 0, 2 * sizeof(unsigned), c->stream);
   if (info[kErrPhase] == kPhaseHash) {
     // the hash stopped the search before its reorder: the state is still in the previous
     // order, in the buffers the host swapped away from
@@ -431,7 +432,7 @@ sph_status settle_call(sph_ctx* c) {
       c->call_open = false;
       return SPH_OK;
     }
-    cudaMemsetAsync(c->d.status, 0, sizeof(unsigned), c->stream);
+    cudaMemsetAsync(c->d.status, 0, 2 * sizeof(unsigned), c->stream);
     // the host's view of the stopped call: completed steps and the buffer parity of the
     // reorders that did run (the failing step's own reorder ran if its list build reported)
     const long long done = failed_step(info);
@@ -450,8 +451,7 @@ sph_status settle_call(sph_ctx* c) {
                        where + "; the state is that step's after its half-kick and drift");
     }
     sph_status s = regrow_lists(c);
-    if (s == SPH_OK && (launch_advance_time(launcher(c), 0) || ph_forces(c, true) ||
-                        ph_vv2(c, true)))
+    if (s == SPH_OK && (launch_advance_time(launcher(c), 0) || ph_forces(c, true)))
       s = cuda_fail(c, "resumed step");
     if (s != SPH_OK) {
       c->call_open = false;
@@ -700,7 +700,6 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
   d.nwallseg = nwall;
   d.Nlist_coll = nlist;
   const int list_cap = o.nbr_capacity > 0 ? o.nbr_capacity : derived_capacity(c->boxes, c->dim);
-  c->key_bits = bits_for(std::max(Ctot, 2));
   const size_t Np = d.Npad;
   bool ok = true;
   BoxParams* dbox = nullptr;
@@ -725,8 +724,9 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
     d.rec = r;
   }
   ok = ok && dalloc(c, &d.nbr_cnt, Np) && dalloc(c, &d.nbr_nch, Np);
-  ok = ok && dalloc(c, &d.key_by_gid, Np) && dalloc(c, &d.keys, Np) && dalloc(c, &d.vals, Np);
-  ok = ok && dalloc(c, &d.keys_alt, Np) && dalloc(c, &d.vals_alt, Np);
+  ok = ok && dalloc(c, &d.keys, Np) && dalloc(c, &d.vals, Np);
+  ok = ok && dalloc(c, &d.moved, Np) && dalloc(c, &d.bucket, Np);
+  ok = ok && dalloc(c, &d.cell_count, Ctot + 1) && dalloc(c, &d.scan_sums, Ctot / 4096 + 2);
   ok = ok && dalloc(c, &d.cell_begin, Ctot + 1) && dalloc(c, &d.cell_start, Ctot);
   ok = ok && dalloc(c, &d.cell_end, Ctot) && dalloc(c, &d.cell_box, Ctot);
   ok = ok && alloc_lists(c, list_cap);
@@ -735,19 +735,18 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
   d.nwallchunks = nwchunk;
   ok = ok && dalloc(c, &d.wall_chunk, nwchunk + 1) && dalloc(c, &d.wall_seg_chunk, nwall + 1);
   ok = ok && dalloc(c, &d.wall_part, 3 * (size_t)std::max(nwchunk, 1));
+  ok = ok && dalloc(c, &d.wall_of_chunk, nwchunk) && dalloc(c, &d.wall_done, nwall);
   ok = ok && dalloc(c, &d.colloids_list, nlist) && dalloc(c, &d.coll_seg, ncoll + 1);
   ok = ok && dalloc(c, &d.coll_box, ncoll) && dalloc(c, &d.xc, 3 * (size_t)std::max(nlist, 1));
   ok = ok && dalloc(c, &d.cs, (size_t)kCollFields * std::max(ncoll, 1));
   ok = ok && dalloc(c, &d.ccell, ncoll) && dalloc(c, &d.cindex, ncoll);
   ok = ok && dalloc(c, &d.ccell_start, ncc) && dalloc(c, &d.ccell_end, ncc);
   ok = ok && dalloc(c, &d.mag, 3 * nboxes) && dalloc(c, &d.ke, nboxes);
-  ok = ok && dalloc(c, &d.step, 1) && dalloc(c, &d.status, 1) &&
+  ok = ok && dalloc(c, &d.step, 1) && dalloc(c, &d.status, 2) &&
        dalloc(c, &d.err_info, kErrInfoLen);
   // positions not yet looked at by a search: the pair passes keep the minimum image
   if (ok) cudaMemsetAsync(d.err_info + kPosOutside, 1, sizeof(int), c->stream);
   ok = ok && dalloc(c, &c->scratch, Np) && dalloc(c, &c->iscratch, Np);
-  c->sort.hist_len = (int)sort_hist_len(Ntot, c->key_bits);
-  ok = ok && dalloc(c, &c->sort.hist, (size_t)c->sort.hist_len);
   // kinetic-energy chunks
   std::vector<int> kchunk{0}, kbox{0};
   for (const HostBox& hb : c->boxes) {
@@ -840,11 +839,12 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
     }
   }
   // chunks of the walls lists for the wall-force reduction
-  std::vector<int> wchunk{0}, wsegchunk{0};
+  std::vector<int> wchunk{0}, wsegchunk{0}, wofchunk;
   for (size_t sgm = 0; sgm + 1 < wseg.size(); ++sgm) {
     for (int j = wseg[sgm]; j < wseg[sgm + 1]; j += kWallChunk)
       wchunk.push_back(std::min(j + kWallChunk, wseg[sgm + 1]));
     wsegchunk.push_back((int)wchunk.size() - 1);
+    wofchunk.resize(wchunk.size() - 1, (int)sgm);
   }
   if ((int)wchunk.size() - 1 != nwchunk || (int)wsegchunk.size() - 1 != nwall) ok = false;
   if (nboxes >= (1 << (31 - kTypeBits))) ok = false;
@@ -889,6 +889,7 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
   up(d.wall_seg, wseg.data(), wseg.size() * sizeof(int));
   up(d.wall_chunk, wchunk.data(), wchunk.size() * sizeof(int));
   up(d.wall_seg_chunk, wsegchunk.data(), wsegchunk.size() * sizeof(int));
+  up(d.wall_of_chunk, wofchunk.data(), wofchunk.size() * sizeof(int));
   up(d.colloids_list, cl.data(), cl.size() * sizeof(int));
   up(d.coll_seg, cseg.data(), cseg.size() * sizeof(int));
   up(d.coll_box, cbox.data(), cbox.size() * sizeof(int));
@@ -1177,12 +1178,13 @@ sph_status sph_profile_phases(sph_ctx* c, int nsteps, double* ms) {
   for (int s = 0; s < nsteps && !bad; ++s) {
     Launch L = launcher(c);
     cudaEventRecord(ev[0], c->stream);
-    bad |= launch_vv1_colloids(L) | launch_vv1_particles(L);
+    // the particles' half-kick and drift are in the hash's kernel, as in the step graph
+    bad |= launch_vv1_colloids(L);
     c->forces_live = false;
     cudaEventRecord(ev[1], c->stream);
-    bad |= launch_hash(L);
+    bad |= launch_vv1_hash(L);
     cudaEventRecord(ev[2], c->stream);
-    bad |= launch_sort(L, c->key_bits, c->sort);
+    bad |= launch_cell_sort(L, true);
     cudaEventRecord(ev[3], c->stream);
     bad |= launch_reorder(L, false);
     swap_state(c, false);
@@ -1191,7 +1193,6 @@ sph_status sph_profile_phases(sph_ctx* c, int nsteps, double* ms) {
     bad |= launch_build_lists_dim(L, c->dim);
     cudaEventRecord(ev[5], c->stream);
     if (c->d.ncoll > 0) bad |= launch_colloid_cells_n(L, c->nboxes, c->max_coll);
-    bad |= launch_advance_time(L, 0);
     cudaEventRecord(ev[6], c->stream);
     Launch Lf = L;
     Lf.d.gradv = nullptr;
@@ -1202,9 +1203,9 @@ sph_status sph_profile_phases(sph_ctx* c, int nsteps, double* ms) {
     cudaEventRecord(ev[8], c->stream);
     bad |= launch_wall_forces(Lf);
     cudaEventRecord(ev[9], c->stream);
-    bad |= launch_colloid_forces(Lf, pairs ? 1 : 0);
+    // with the colloids' half-kick; the pair pass counts the step
+    bad |= launch_colloid_forces(Lf, pairs ? 1 : 0, 1);
     cudaEventRecord(ev[10], c->stream);
-    bad |= launch_vv2(L, false) | launch_count_step(L);
     cudaEventRecord(ev[11], c->stream);
     cudaEventSynchronize(ev[11]);
     for (int k = 0; k < SPH_NUM_PHASES; ++k) {

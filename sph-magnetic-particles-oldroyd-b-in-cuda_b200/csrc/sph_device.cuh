@@ -178,10 +178,12 @@ __device__ __forceinline__ bool own_cell(const BoxParams& p, double x, double y,
   return true;
 }
 
-// Reports a failure.  The first report of any kind also records the step counter and the
-// phase; the first report of a bad position records the particle's global id.
+// Reports a failure (WORD 1: found by the hash).  The first report of any kind also records the
+// step counter and the phase; the first report of a bad position records the particle's global
+// id.
+template <int WORD = 0>
 __device__ __forceinline__ void raise_status(const Dev& d, unsigned bit, int info, int phase) {
-  const unsigned old = atomicOr(d.status, bit);
+  const unsigned old = atomicOr(d.status + WORD, bit);
   if (!(old & bit) && bit != kStatCapacity) atomicExch(&d.err_info[kErrBadId], info);
   if (!(old & kStatAbortMask)) {
     const long long s = *d.step;
@@ -232,15 +234,20 @@ struct NbrIter {
 };
 
 // True once a kernel before this one reported a failure: the step's state-changing kernels
-// then return at entry.  The flag word is read past L1 (it is written by atomics in L2).  In
-// kernels whose warps cooperate, lane 0's reading is taken by the whole warp.
-__device__ __forceinline__ bool step_aborted(const Dev& d) {
+// then return at entry.  The flag words are read past L1 (they are written by atomics in L2).
+// In kernels whose warps cooperate, lane 0's reading is taken by the whole warp.
+// step_stopped: before this step's hash (see StatusBits).
+__device__ __forceinline__ bool step_stopped(const Dev& d) {
   return (*(volatile const unsigned*)d.status & kStatAbortMask) != 0u;
+}
+__device__ __forceinline__ bool step_aborted(const Dev& d) {
+  const volatile unsigned* s = d.status;
+  return ((s[0] | s[1]) & kStatAbortMask) != 0u;
 }
 __device__ __forceinline__ bool step_aborted_warp(const Dev& d) {
   unsigned v = 0u;
-  if ((threadIdx.x & 31) == 0) v = *(volatile const unsigned*)d.status;
-  return (__shfl_sync(0xffffffffu, v, 0) & kStatAbortMask) != 0u;
+  if ((threadIdx.x & 31) < 2) v = ((volatile const unsigned*)d.status)[threadIdx.x & 31];
+  return __any_sync(0xffffffffu, (v & kStatAbortMask) != 0u);
 }
 
 // A position outside [0, L] along a periodic axis of its box (or not finite).
@@ -249,7 +256,10 @@ __device__ __forceinline__ bool outside_periodic(const BoxParams& p, double x, d
   return !(x >= 0.0 && x <= p.L[0]) || (p.wall == 0 && !(y >= 0.0 && y <= p.L[1])) ||
          (p.dim == 3 && !(z >= 0.0 && z <= p.L[2]));
 }
-__device__ __forceinline__ void mark_outside(const Dev& d) { d.err_info[kPosOutside] = 1; }
+__device__ __forceinline__ void mark_outside(const Dev& d, int parity) {
+  d.err_info[kPosOutside + parity] = 1;
+}
+__device__ __forceinline__ void mark_outside(const Dev& d) { mark_outside(d, d.parity); }
 
 // A particle at least 1.0625 rcut from every periodic face of its box.  While every position
 // lies in [0, L] along the periodic axes (err_info[kPosOutside] clear), the minimum image
@@ -270,7 +280,7 @@ __device__ __forceinline__ bool clear_of_faces(const BoxParams& p, T x, T y, T z
 // reading of the flag is taken by the whole warp.
 __device__ __forceinline__ bool warp_plain_image(const Dev& d, bool clear) {
   int v = 0;
-  if ((threadIdx.x & 31) == 0) v = *(volatile const int*)(d.err_info + kPosOutside);
+  if ((threadIdx.x & 31) == 0) v = *(volatile const int*)(d.err_info + kPosOutside + d.parity);
   v = __shfl_sync(0xffffffffu, v, 0);
   return __all_sync(0xffffffffu, clear) && v == 0;
 }

@@ -18,6 +18,10 @@ constexpr int kTypeBits = 12;
 constexpr int kTypeMask = (1 << kTypeBits) - 1;
 
 // Device error flags (bit set in Dev::status by any kernel that detects the condition).
+// status[1] takes the flags the hash raises: the hash is part of the kernel that moves the
+// particles, which has to finish whatever some particle's position turns out to be, so that
+// kernel and the cell scan look at status[0] alone, every later kernel of the step at both,
+// and the reorder copies status[1] into status[0] for the steps that follow.
 // Once any of them is set, every state-changing kernel of the step returns at entry, so a
 // failure found in step k of a multi-step (graph-replayed) call leaves the state where step
 // k found it; the first report records the step counter and the phase (Dev::err_info).
@@ -37,13 +41,15 @@ enum ErrInfo : int {
   kErrStepLo = 2,    // device step counter (completed steps) at the first report, low word
   kErrStepHi = 3,    // ... high word
   kErrPhase = 4,     // FailPhase of the first report
-  // nonzero when a position may lie outside [0, L] along a periodic axis: cleared before
-  // the hash of each search and set by the hash for every position it finds outside, by the
-  // half-kicks for every position they leave outside, and by any write of positions from
-  // the host.  While it is set the list build places every candidate by its minimum image;
+  // nonzero when a position may lie outside [0, L] along a periodic axis.  Two words, one per
+  // buffer parity (Dev::parity): a search's hash sets the word of the parity that the search
+  // ends with for every position it finds outside and its cell scan clears the other word, for
+  // the next search; the half-kicks set the current word for every position they leave
+  // outside, and so does any write of positions from the host.  While it is set the list build places every candidate by its minimum image;
   // while it is clear the pair passes may drop the minimum image for particles clear of the
   // periodic faces (clear_of_faces).
   kPosOutside = 5,
+  kPosOutside1 = 6,
   kErrInfoLen = 8,
 };
 
@@ -189,11 +195,12 @@ struct Dev {
   int2* nchunk;     // cap x Npad: nchunk[k * Npad + i]
   int* nbr_nch;     // per slot: chunks stored
   int* nbr_cnt;     // per slot: candidates (set bits over the particle's chunks)
-  int* key_by_gid;
-  int* keys;     // sorted keys
+  int* keys;     // sorted keys (global cell of each slot)
   int* vals;     // sorted values (global ids)
-  int* keys_alt;
-  int* vals_alt;
+  int* cell_count;  // Ctot + 1: particles counted per cell by the hash; zero between searches
+  int* scan_sums;   // partial sums of the cell scan
+  int2* moved;      // per slot, by the hash: (cell, place in the cell's count)
+  int2* bucket;     // per new slot: (global id, old slot), unordered within a cell
   int* cell_begin;     // Ctot + 1: first slot of each global cell (current)
   int* cell_start;     // Ctot, reference semantics, box-local slot index
   int* cell_end;       // Ctot
@@ -205,6 +212,8 @@ struct Dev {
   int* wall_chunk;     // nwallchunks + 1 boundaries into walls_list, never across segments
   int* wall_seg_chunk; // nwallseg + 1 boundaries into the chunks
   double* wall_part;   // nwallchunks x 3 partial sums
+  int* wall_of_chunk;  // nwallchunks: the wall of a chunk
+  int* wall_done;      // nwallseg: chunks summed so far; zero between passes
   int nwallchunks;
   // colloids
   int* colloids_list;  // global ids
@@ -225,8 +234,10 @@ struct Dev {
   long long* step;     // device step counter (graph replays)
   unsigned* status;
   int* err_info;       // kErrInfoLen ints, see ErrInfo
+  int parity;          // which buffers hold the state: flips with every reorder
   int grad_all;        // fused pair pass: velocity gradient of every particle, not only fluid
-  int fold_vv2;        // fused pair pass: also the step's second half-kick of fluid particles
+  int fold_vv2;        // fused pair pass: also the step's second half-kick of fluid particles,
+                       // and the step count
   int one_box;         // a single box: its pair constants are in pc
   PairConsts pc;
 };
@@ -261,9 +272,14 @@ inline int& last_launch_error() {
 }
 
 int launch_vv1_particles(const Launch& L);
+// the half-kick and drift of the particles and the hash of the search that follows
+int launch_vv1_hash(const Launch& L);
 int launch_vv1_colloids(const Launch& L);
-int launch_vv2(const Launch& L, bool particles = true);
+int launch_vv2(const Launch& L);
 int launch_hash(const Launch& L);
+// Cell ranges from the hash's counts and the buckets; advance: also the magnetic moment of the
+// step being taken (launch_advance_time with mode 0).
+int launch_cell_sort(const Launch& L, bool advance);
 int launch_reorder(const Launch& L, bool permute_forces);
 int launch_build_lists_dim(const Launch& L, int dim);
 int launch_colloid_cells_n(const Launch& L, int nboxes, int max_coll);
@@ -272,8 +288,10 @@ int launch_pressure(const Launch& L);
 int launch_pairs_dim(const Launch& L, int dim, int mode, int with_ext);
 int launch_ext_force(const Launch& L);
 int launch_dcdt_from_gradv(const Launch& L);
+// Wall forces, and the forces and torques of the colloids (with_pairs: with their repulsion and
+// magnetic forces; kick: and their second half-kick).
 int launch_wall_forces(const Launch& L);
-int launch_colloid_forces(const Launch& L, int with_pairs);
+int launch_colloid_forces(const Launch& L, int with_pairs, int kick = 0);
 int launch_advance_time(const Launch& L, int mode);
 int launch_count_step(const Launch& L);
 int launch_kinetic_energy(const Launch& L, double* partial);
@@ -307,8 +325,7 @@ int launch_init_fill(const Launch& L, const InitBox* boxes, const int* blk_box, 
 int launch_init_scatter(const Launch& L, int n, const int2* meta, const double4* pos,
                         const double4* vel, const double* conf);
 
-// Stable LSD radix sort of the hash keys (sph_sort.cu): keys d.key_by_gid indexed by
-// global id, values = global ids; result in d.keys / d.vals.
+// Stable LSD radix sort (sph_sort.cu) of the allocation-free neighbour search.
 // Geometry of the sort, shared by every user of its histogram buffer: items per tile,
 // buckets per pass (at most 9 key bits per pass) and entries per scan block.
 constexpr int kSortTile = 4096;
@@ -322,12 +339,4 @@ constexpr size_t sort_hist_ints(long long n) {
           kSortScanChunk - 1) / kSortScanChunk +
          32;
 }
-struct SortScratch {
-  int* hist;       // radix histogram / offsets
-  int hist_len;
-  int ntiles;
-};
-size_t sort_hist_len(int n, int key_bits);
-int launch_sort(const Launch& L, int key_bits, const SortScratch& scr);
-
 }  // namespace sph
