@@ -19,6 +19,7 @@
 using namespace sph;
 
 struct sph_ctx {
+  int nsm = 148;  // multiprocessors of the device
   int device = 0, prec = SPH_PREC_FP64, dim = 3, nboxes = 0, use_graph = 1;
   std::vector<HostBox> boxes;
   Dev d{};
@@ -100,6 +101,7 @@ Launch launcher(sph_ctx* c) {
   L.prec = c->prec;
   L.stream = c->stream;
   L.launches = &c->launches;
+  L.nsm = c->nsm;
   L.list_tpc = c->tune.list_threads_per_cell;
   L.density_block = c->tune.density_block;
   return L;
@@ -576,6 +578,7 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
     delete c;
     return SPH_ERR_CUDA;
   }
+  cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
   cudaEventCreate(&c->ev0);
   cudaEventCreate(&c->ev1);
   // ---- lattice boxes built on the device: count the kept and wall sites per block ----

@@ -442,19 +442,23 @@ __global__ void k_reorder(Dev d) {
 // Density contribution of one list entry (kernel_densities.cu:52-163 with kernel_W.cu): the
 // exact distance test, then W(r) with r from one reciprocal square root; the particle itself
 // (r2 = 0) contributes W(0).  FP64: over cw, and rcut_inv is 3 / rcut.  WRAP: see min_image.
-template <typename T, int DIM, bool WRAP = true>
+// SELECT: without a branch.
+template <typename T, int DIM, bool WRAP = true, bool SELECT = false>
 __device__ __forceinline__ T density_term(const typename V4<T>::type& xi,
                                           const typename V4<T>::type& xj, const T L[3],
                                           const T h[3], int wall, T rcutsq, T rcut_inv, T cw) {
   T rx = xi.x - xj.x, ry = xi.y - xj.y, rz = DIM == 3 ? xi.z - xj.z : T(0);
   min_image<T, DIM, WRAP>(rx, ry, rz, L, h, wall);
   const T r2 = norm2(rx, ry, rz, DIM == 3);
-  if (!(r2 < rcutsq)) return T(0);
+  const bool in = r2 < rcutsq;
+  if (!SELECT && !in) return T(0);
+  T w;
   if constexpr (sizeof(T) == 8) {
-    return sph_w(r2 > 0.0 ? xmul(r2, inv_sqrt(r2)) : 0.0, rcut_inv);
+    w = sph_w(r2 > 0.0 ? xmul(r2, inv_sqrt(r2)) : 0.0, rcut_inv);
   } else {
-    return sph_w(r2 > 0.0f ? r2 * rsqrt(r2) : 0.0f, rcut_inv, cw);
+    w = sph_w(r2 > 0.0f ? r2 * rsqrt(r2) : 0.0f, rcut_inv, cw);
   }
+  return in ? w : T(0);
 }
 
 // Density, pressure (kernel_pressures.cu:13-23) and the neighbour record of slot i.
@@ -603,7 +607,7 @@ __device__ __forceinline__ bool stale_cell(const Dev& d, int nc) {
 }
 
 template <int DIM, int TPC>
-__global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d) {
+__global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int split) {
   static_assert(TPC == 32 || TPC == 16, "a warp or a half-warp per cell");
   // candidates staged as three float rows per warp, read four at a time
   __shared__ __align__(16) float stage_x[kListWarps][32];
@@ -622,7 +626,9 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d) {
   float* stx = &stage_x[w][sub * TPC];
   float* sty = &stage_y[w][sub * TPC];
   float* stz = &stage_z[w][sub * TPC];
-  const int cell = (blockIdx.x * kListWarps + w) * (32 / TPC) + sub;
+  // `split` warps per cell, warp `part` of them taking every split-th round of particles
+  const int part = (blockIdx.x * kListWarps + w) % split;
+  const int cell = (blockIdx.x * kListWarps + w) / split * (32 / TPC) + sub;
   // both groups of a warp walk the same loop structure in lockstep (divergent halves would
   // run one after the other): trip counts are warp maxima, a group past its own range idles
   const bool live = cell < d.Ctot;
@@ -686,7 +692,7 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d) {
   // the particle loop, in the cheap form (per-cell shifts) or the minimum-image one
   auto walk = [&](auto mi_tag) {
     constexpr bool kMI = decltype(mi_tag)::value;
-    for (int t0 = 0; t0 < span; t0 += TPC) {
+    for (int t0 = part * TPC; t0 < span; t0 += split * TPC) {
       const int i = beg + t0 + gl;
       const bool active = i < end;
       float xi = 0.f, yi = 0.f, zi = 0.f;
@@ -915,11 +921,10 @@ __global__ void k_colloid_cells(Dev d, int nboxes) {
 // flight per lane the pass waited on memory, 5 long-scoreboard stalls per instruction).
 // Measured at 128^3 (FP64, with the plain separations): 1.16 ms with one entry at a time,
 // 1.10 ms with two, 1.21 and 1.22 ms with three and four (registers, fewer warps).
-template <typename T, int DIM, bool WRAP>
+template <typename T, int DIM, bool WRAP, int kAhead>
 __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>::type* P,
                                               int i, const BoxParams& p) {
   using V = typename V4<T>::type;
-  constexpr int kAhead = 2;
   const T L[3] = {(T)p.L[0], (T)p.L[1], (T)p.L[2]};
   const T h[3] = {(T)p.halfL[0], (T)p.halfL[1], (T)p.halfL[2]};
   const T rcutsq = (T)p.rcutsq;
@@ -936,11 +941,21 @@ __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>
     for (int u = 0; u < kAhead; ++u) j[u] = k + u < n ? it.next() : -1;
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) x[u] = ld_pos<DIM>(P + (j[u] >= 0 ? j[u] : i));
+    if constexpr (kAhead > 2) {
+      // the terms side by side, then their sum in order
+      T w[kAhead];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      if (j[u] < 0) break;
-      const T w = density_term<T, DIM, WRAP>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv, cw);
-      dens = dens + w;
+      for (int u = 0; u < kAhead; ++u)
+        w[u] = density_term<T, DIM, WRAP, true>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv, cw);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) dens = dens + (j[u] >= 0 ? w[u] : T(0));
+    } else {
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        if (j[u] < 0) break;
+        const T w = density_term<T, DIM, WRAP>(xi, x[u], L, h, p.wall, rcutsq, rcut_inv, cw);
+        dens = dens + w;
+      }
     }
   }
   return sizeof(T) == 8 ? __dmul_rn(p.cw, dens) : dens;  // the factor left out of the terms
@@ -948,7 +963,7 @@ __device__ __forceinline__ double density_sum(const Dev& d, const typename V4<T>
 
 // Whole warps (lanes past the end mirror the last slot and store nothing), so that a warp
 // of particles clear of the periodic faces takes the sums without the minimum image.
-template <typename T, int DIM>
+template <typename T, int DIM, int AHEAD>
 __global__ void k_density(Dev d) {
   using V = typename V4<T>::type;
   const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -963,9 +978,9 @@ __global__ void k_density(Dev d) {
   const V xi = ld_pos<DIM>(P + i);
   double dens;
   if (warp_plain_image(d, clear_of_faces<T, DIM>(p, xi.x, xi.y, xi.z)))
-    dens = density_sum<T, DIM, false>(d, P, i, p);
+    dens = density_sum<T, DIM, false, AHEAD>(d, P, i, p);
   else
-    dens = density_sum<T, DIM, true>(d, P, i, p);
+    dens = density_sum<T, DIM, true, AHEAD>(d, P, i, p);
   if (active) density_epilogue<T, DIM>(d, i, p, dens);
 }
 
@@ -1153,7 +1168,7 @@ __global__ void k_pressure(Dev d) {
 //    registers with 32 bytes of spill, but at 16 warps per SM (4 blocks of 4 warps or 8 of
 //    2) it took 4.03 and 3.98 ms: the larger shared-memory carve-out leaves L1 too little
 //    for the record gathers.
-template <typename T, int DIM>
+template <typename T, int DIM, bool WIDE = false>
 struct PairShape {
   using Rec = typename RecFor<T, DIM>::type;
   static constexpr bool kF64 = sizeof(T) == 8;
@@ -1161,8 +1176,8 @@ struct PairShape {
   static constexpr bool kF64_3D = kF64 && DIM == 3;
   // the float 2D pass runs 2-warp blocks (measured 2.29 vs 2.35 ms on the 512-box ensemble;
   // the float 3D pass was slower with them, the FP64 passes unchanged)
-  static constexpr int kWarps = kF2D ? 2 : 4;
-  static constexpr int kMinBlocks = kF2D ? 6 : (kF64_3D ? 3 : (kF64 ? 5 : 4));
+  static constexpr int kWarps = WIDE ? 1 : kF2D ? 2 : 4;
+  static constexpr int kMinBlocks = WIDE ? 1 : kF2D ? 6 : (kF64_3D ? 3 : (kF64 ? 5 : 4));
 };
 
 // The pair constants of a one-box context, viewed as PairParams (same layout).
@@ -1297,15 +1312,68 @@ __device__ __forceinline__ void pair_walk(const PairWalk<T, DIM>& W, NbrIter& it
   }
 }
 
-template <typename T, int DIM, int MODE, bool EXT, bool ONE>
-__global__ void __launch_bounds__(PairShape<T, DIM>::kWarps * 32,
-                                  PairShape<T, DIM>::kMinBlocks)
+// The same, two positions per step, side by side where all partners of the warp are fluid.
+template <typename T, int DIM, bool WRAP, int MODE>
+__device__ __forceinline__ void pair_walk_wide(const PairWalk<T, DIM>& W, NbrIter& it,
+                                               PairAcc<T, DIM>& acc) {
+  using Rec = typename RecFor<T, DIM>::type;
+  using St = PairStage<Rec>;
+  static_assert(DIM == 2, "the type words come from the type array");
+  const int n = W.n, lane = W.lane;
+  int jc[2], tc[2];
+  auto fetch = [&](int k, int buf, int (&j)[2], int (&t)[2]) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      j[u] = k + u < n ? it.next() : -1;
+      if (k + u < W.nmax) stage_records<Rec>(W.sb + (buf * 2 + u) * St::kRows, W.rec, j[u], lane);
+      t[u] = j[u] >= 0 ? __ldg(&W.d.tinfo[j[u]]) : 0;
+    }
+    cp_async_commit();
+  };
+  fetch(0, 0, jc, tc);
+  int buf = 0;
+  for (int k = 0; k < W.nmax; k += 2) {
+    int jn[2], tn[2];
+    fetch(k + 2, buf ^ 1, jn, tn);
+    cp_async_wait_prev();
+    __syncwarp();
+    const int4* row = W.sb + buf * 2 * St::kRows + lane * St::kStride;
+    const StagedRec<T, Rec> R[2] = {StagedRec<T, Rec>(row), StagedRec<T, Rec>(row + St::kRows)};
+    bool valid[2], fluid = W.o.fluid;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      valid[u] = jc[u] >= 0 && jc[u] != W.i;
+      fluid = fluid && (!valid[u] || type_of(tc[u]) == 0);
+    }
+    if (__all_sync(SPH_FULL, fluid)) {
+      pair_fluid_x2<T, DIM, WRAP, MODE>(W.p, W.pp, W.o, R[0].r, R[1].r, valid, acc);
+    } else {
+#pragma unroll 1
+      for (int u = 0; u < 2; ++u) {
+        const StagedRec<T, Rec> Ru(row + u * St::kRows);
+        if (u == 0 ? valid[0] : valid[1])
+          pair_term<T, DIM, WRAP>(W.p, W.pp, W.cv, W.o, Ru.r, type_of(u == 0 ? tc[0] : tc[1]), acc);
+      }
+    }
+    __syncwarp();  // this buffer is refilled by the next step's fetch
+    buf ^= 1;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      jc[u] = jn[u];
+      tc[u] = tn[u];
+    }
+  }
+}
+
+template <typename T, int DIM, int MODE, bool EXT, bool ONE, bool WIDE = false>
+__global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
+                                  PairShape<T, DIM, WIDE>::kMinBlocks)
     k_pairs(const __grid_constant__ Dev d) {
-  using Sh = PairShape<T, DIM>;
+  using Sh = PairShape<T, DIM, WIDE>;
   using Rec = typename Sh::Rec;
   using St = PairStage<Rec>;
   // per warp: a double buffer of staged positions
-  __shared__ int4 stage[Sh::kWarps][2][St::kRows];
+  __shared__ int4 stage[Sh::kWarps][WIDE ? 4 : 2][St::kRows];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wbase = (blockIdx.x * Sh::kWarps + w) * 32;
   if (wbase >= d.Ntot) return;  // whole warps only: the lanes below cooperate
@@ -1336,7 +1404,10 @@ __global__ void __launch_bounds__(PairShape<T, DIM>::kWarps * 32,
   it.init(d, is);
   const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], lane, i, n, nmax, p, pp, cv, o};
   auto walk = [&](auto wrap_tag) {
-    pair_walk<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
+    if constexpr (WIDE)
+      pair_walk_wide<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
+    else
+      pair_walk<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
   };
   // Warps clear of the periodic faces drop the minimum image, in 3D only: the 512-box 2D
   // ensemble's small boxes put both kinds of warp on every SM, and the second copy of the
@@ -1949,14 +2020,20 @@ int launch_reorder(const Launch& L, bool permute_forces) {
 int launch_build_lists_dim(const Launch& L, int dim) {
   if (L.d.Ctot == 0) return 0;
   const bool half = L.list_tpc == 16;
-  const int nb = blocks(L.d.Ctot, kListWarps * (half ? 2 : 1));
+  // Cells of more than 28 particles on average hold more than a warp's 32 here and there, and the
+  // warps of those cells, with a second round, are what a small grid waits for: two warps per
+  // cell, up to 64 cells per SM.  Measured in 3D (ms, one / two): 25 x 25 x 31 sites (4 cells per
+  // SM) 0.062 / 0.038, 56^3 (44) 0.130 / 0.114, 61 x 53 x 67 (51) 0.136 / 0.129; 128^3 (520) 0.856
+  // / 0.895, and 48^3, 27 per cell, 0.069 / 0.075.
+  const int split = L.d.Ntot / 28 > L.d.Ctot && L.d.Ctot <= 64 * L.nsm ? 2 : 1;
+  const int nb = blocks(blocks(L.d.Ctot, half ? 2 : 1) * split, kListWarps);
   constexpr int nt = kListWarps * 32;
   if (dim == 3) {
-    if (half) k_build_lists<3, 16><<<nb, nt, 0, S(L)>>>(L.d);
-    else k_build_lists<3, 32><<<nb, nt, 0, S(L)>>>(L.d);
+    if (half) k_build_lists<3, 16><<<nb, nt, 0, S(L)>>>(L.d, split);
+    else k_build_lists<3, 32><<<nb, nt, 0, S(L)>>>(L.d, split);
   } else {
-    if (half) k_build_lists<2, 16><<<nb, nt, 0, S(L)>>>(L.d);
-    else k_build_lists<2, 32><<<nb, nt, 0, S(L)>>>(L.d);
+    if (half) k_build_lists<2, 16><<<nb, nt, 0, S(L)>>>(L.d, split);
+    else k_build_lists<2, 32><<<nb, nt, 0, S(L)>>>(L.d, split);
   }
   return check(L);
 }
@@ -1965,6 +2042,26 @@ int launch_colloid_cells_n(const Launch& L, int nboxes, int max_coll) {
   if (L.d.ncoll == 0) return 0;
   k_colloid_cells<<<nboxes, 128, sizeof(int) * (max_coll > 0 ? max_coll : 1), S(L)>>>(L.d, nboxes);
   return check(L);
+}
+
+// A context of so few particles that its warps (one per 32) hardly fill the SMs: a pass then
+// takes as long as one warp's walk over its lists, and what shortens the walk is work side by
+// side in the warp (its registers are free), in one-warp blocks spread over all SMs.
+inline bool few_warps(const Launch& L, int per_sm) { return L.d.Ntot <= 32 * per_sm * L.nsm; }
+
+// Up to kFewDensity warps per SM: the terms of eight list entries side by side.  Measured (ms,
+// two at a time / eight): FP64 at 13.5 warps per SM (40 x 40 x 40) 0.062 / 0.056, at 18 0.066 /
+// 0.086; float at 18 0.056 / 0.052, at 26 0.065 / 0.064, at 37 0.087 / 0.090.
+template <typename T>
+constexpr int kFewDensity = sizeof(T) == 8 ? 14 : 24;
+template <typename T, int DIM>
+static void density_launch(const Launch& L) {
+  if (few_warps(L, kFewDensity<T>)) {
+    k_density<T, DIM, 8><<<blocks(L.d.Ntot, 32), 32, 0, S(L)>>>(L.d);
+  } else {
+    const int nt = L.density_block;
+    k_density<T, DIM, 2><<<blocks(L.d.Ntot, nt), nt, 0, S(L)>>>(L.d);
+  }
 }
 
 int launch_density_dim(const Launch& L, int dim) {
@@ -1982,14 +2079,12 @@ int launch_density_dim(const Launch& L, int dim) {
     }
     return check(L);
   }
-  const int nt = L.density_block;
-  const int nb = blocks(L.d.Ntot, nt);
   if (L.prec == SPH_PREC_FP64) {
-    if (dim == 3) k_density<double, 3><<<nb, nt, 0, S(L)>>>(L.d);
-    else k_density<double, 2><<<nb, nt, 0, S(L)>>>(L.d);
+    if (dim == 3) density_launch<double, 3>(L);
+    else density_launch<double, 2>(L);
   } else {
-    if (dim == 3) k_density<float, 3><<<nb, nt, 0, S(L)>>>(L.d);
-    else k_density<float, 2><<<nb, nt, 0, S(L)>>>(L.d);
+    if (dim == 3) density_launch<float, 3>(L);
+    else density_launch<float, 2>(L);
   }
   return check(L);
 }
@@ -2007,6 +2102,18 @@ template <typename T, int DIM, bool ONE>
 static void pairs_launch(const Launch& L, int mode, int with_ext) {
   constexpr int nt = PairShape<T, DIM>::kWarps * 32;
   const int nb = blocks(L.d.Ntot, nt);
+  // FP64 2D, up to kFewPairs warps per SM: two list positions side by side.  Measured (ms, one /
+  // two): 64^2 0.037 / 0.029, 192^2 (8 warps per SM) 0.054 / 0.050, 256^2 (14) 0.065 / 0.076; in
+  // 3D and in float the walk is bound by its instructions (3D FP64 16^3 0.109 / 0.111 ms).
+  constexpr int kFewPairs = 10;
+  if constexpr (sizeof(T) == 8 && DIM == 2) {
+    if (mode == kPairFused && few_warps(L, kFewPairs)) {
+      const int nb1 = blocks(L.d.Ntot, 32);
+      if (with_ext) k_pairs<T, DIM, kPairFused, true, ONE, true><<<nb1, 32, 0, S(L)>>>(L.d);
+      else k_pairs<T, DIM, kPairFused, false, ONE, true><<<nb1, 32, 0, S(L)>>>(L.d);
+      return;
+    }
+  }
   if (mode == kPairGradvAll)
     k_pairs<T, DIM, kPairGradvAll, false, ONE><<<nb, nt, 0, S(L)>>>(L.d);
   else if (mode == kPairForcesOnly)
