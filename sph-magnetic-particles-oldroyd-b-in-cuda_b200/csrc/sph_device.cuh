@@ -57,6 +57,17 @@ __device__ __forceinline__ double inv_sqrt(double x) {
   return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 
+// a / b.  FP64: a times the hardware's reciprocal seed after one third-order step,
+// y (1 + e + e^2) with e = 1 - b y (the series of 1 / (1 - e)), without the library's special
+// cases; b is a distance from a wall or a colloid's surface.
+__device__ __forceinline__ double quotient(double a, double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  const double e = __fma_rn(-b, y, 1.0);
+  return __dmul_rn(a, __fma_rn(y, __fma_rn(e, e, e), y));
+}
+__device__ __forceinline__ float quotient(float a, float b) { return a / b; }
+
 // c where t >= 0, else 0 (a test of the sign bit; the constant's low word is zero)
 template <int C>
 __device__ __forceinline__ double where_pos(double t) {
@@ -331,149 +342,6 @@ struct CollView {
   int nc;
 };
 
-// Morris ghost velocity, fluid particle i next to wall / colloid particle j
-// (kernel_forces.cu:234-318, 590-692; kernel_vel_gradients.cu:162-247, 421-525).
-template <typename T, int DIM>
-__device__ __forceinline__ void ghost_fluid_i(const BoxParams& p, const CollView& cv,
-                                              int tj, int coll0, T xi, T yi, T zi, T yj,
-                                              const T vi[3], const T r[3], const T L[3],
-                                              const T h[3], T v[3]) {
-  const T beta_max = (T)p.beta_max;
-  if (tj == 1 || tj == 2) {
-    T di, dj, Vw;
-    if (tj == 1) {
-      di = yi - (T)p.y_bottom;
-      dj = (T)p.y_bottom - yj;
-      Vw = (T)p.V_bottom;
-    } else {
-      di = (T)p.y_top - yi;
-      dj = yj - (T)p.y_top;
-      Vw = (T)p.V_top;
-    }
-    T beta = T(1) + dj / di;
-    if (beta > beta_max) beta = beta_max;
-    if (di > T(0)) {
-      v[0] = beta * (vi[0] - Vw);
-      v[1] = beta * vi[1];
-      v[2] = beta * vi[2];
-    } else {
-      v[0] = vi[0] - Vw;
-      v[1] = vi[1];
-      v[2] = vi[2];
-    }
-    return;
-  }
-  const int c = coll0 + tj - 3, nc = cv.nc;
-  T rc[3] = {xi - (T)cv.cs[CS_X * nc + c], yi - (T)cv.cs[CS_Y * nc + c],
-             DIM == 3 ? zi - (T)cv.cs[CS_Z * nc + c] : T(0)};
-  min_image<T, DIM>(rc[0], rc[1], rc[2], L, h, p.wall);
-  const T dc = DIM == 3 ? sqrt(rc[0] * rc[0] + rc[1] * rc[1] + rc[2] * rc[2])
-                        : sqrt(rc[0] * rc[0] + rc[1] * rc[1]);
-  const T R = (T)p.coll_R;
-  const T dis = dc - R;
-  const T cvel[3] = {(T)cv.cs[CS_VX * nc + c], (T)cv.cs[CS_VY * nc + c],
-                     DIM == 3 ? (T)cv.cs[CS_VZ * nc + c] : T(0)};
-  if (dis < T(0)) {
-    v[0] = vi[0] - cvel[0];
-    v[1] = vi[1] - cvel[1];
-    v[2] = vi[2] - cvel[2];
-    return;
-  }
-  const T xs = rc[0] / dc * R, ys = rc[1] / dc * R, zs = DIM == 3 ? rc[2] / dc * R : T(0);
-  T vr[3];
-  const T wz = (T)cv.cs[CS_OZ * nc + c];
-  if (DIM == 2) {
-    vr[0] = -wz * ys;
-    vr[1] = wz * xs;
-    vr[2] = T(0);
-  } else {
-    const T wx = (T)cv.cs[CS_OX * nc + c], wy = (T)cv.cs[CS_OY * nc + c];
-    vr[0] = wy * zs - wz * ys;
-    vr[1] = wz * xs - wx * zs;
-    vr[2] = wx * ys - wy * xs;
-  }
-  const T sv0 = rc[0] / dc, sv1 = rc[1] / dc, sv2 = DIM == 3 ? rc[2] / dc : T(0);
-  const T djs = DIM == 3 ? (r[0] * sv0 + r[1] * sv1 + r[2] * sv2) - dis
-                         : (r[0] * sv0 + r[1] * sv1) - dis;
-  T beta = T(1) + djs / dis;
-  if (beta > beta_max) beta = beta_max;
-  v[0] = beta * (vi[0] - cvel[0] - vr[0]);
-  v[1] = beta * (vi[1] - cvel[1] - vr[1]);
-  v[2] = beta * (vi[2] - cvel[2] - vr[2]);
-}
-
-// Morris ghost velocity, wall / colloid particle i next to particle j
-// (kernel_forces.cu:337-418, 721-821; kernel_vel_gradients.cu:249-331, 527-630).
-template <typename T, int DIM>
-__device__ __forceinline__ void ghost_solid_i(const BoxParams& p, const CollView& cv,
-                                              int ti, int coll0, T yi, T xj, T yj, T zj,
-                                              const T vj[3], const T r[3], const T L[3],
-                                              const T h[3], T v[3]) {
-  const T beta_max = (T)p.beta_max;
-  if (ti == 1 || ti == 2) {
-    T di, dj, Vw;
-    if (ti == 1) {
-      di = (T)p.y_bottom - yi;
-      dj = yj - (T)p.y_bottom;
-      Vw = (T)p.V_bottom;
-    } else {
-      di = yi - (T)p.y_top;
-      dj = (T)p.y_top - yj;
-      Vw = (T)p.V_top;
-    }
-    T beta = T(1) + di / dj;
-    if (beta > beta_max) beta = beta_max;
-    if (dj > T(0)) {
-      v[0] = beta * (Vw - vj[0]);
-      v[1] = -beta * vj[1];
-      v[2] = -beta * vj[2];
-    } else {
-      v[0] = Vw - vj[0];
-      v[1] = -vj[1];
-      v[2] = -vj[2];
-    }
-    return;
-  }
-  const int c = coll0 + ti - 3, nc = cv.nc;
-  T rc[3] = {xj - (T)cv.cs[CS_X * nc + c], yj - (T)cv.cs[CS_Y * nc + c],
-             DIM == 3 ? zj - (T)cv.cs[CS_Z * nc + c] : T(0)};
-  min_image<T, DIM>(rc[0], rc[1], rc[2], L, h, p.wall);
-  const T dc = DIM == 3 ? sqrt(rc[0] * rc[0] + rc[1] * rc[1] + rc[2] * rc[2])
-                        : sqrt(rc[0] * rc[0] + rc[1] * rc[1]);
-  const T R = (T)p.coll_R;
-  const T djs = dc - R;
-  const T cvel[3] = {(T)cv.cs[CS_VX * nc + c], (T)cv.cs[CS_VY * nc + c],
-                     DIM == 3 ? (T)cv.cs[CS_VZ * nc + c] : T(0)};
-  if (djs < T(0)) {
-    v[0] = cvel[0] - vj[0];
-    v[1] = cvel[1] - vj[1];
-    v[2] = cvel[2] - vj[2];
-    return;
-  }
-  const T xs = rc[0] / dc * R, ys = rc[1] / dc * R, zs = DIM == 3 ? rc[2] / dc * R : T(0);
-  T vr[3];
-  const T wz = (T)cv.cs[CS_OZ * nc + c];
-  if (DIM == 2) {
-    vr[0] = -wz * ys;
-    vr[1] = wz * xs;
-    vr[2] = T(0);
-  } else {
-    const T wx = (T)cv.cs[CS_OX * nc + c], wy = (T)cv.cs[CS_OY * nc + c];
-    vr[0] = wy * zs - wz * ys;
-    vr[1] = wz * xs - wx * zs;
-    vr[2] = wx * ys - wy * xs;
-  }
-  const T sv0 = rc[0] / dc, sv1 = rc[1] / dc, sv2 = DIM == 3 ? rc[2] / dc : T(0);
-  const T dis = DIM == 3 ? (-r[0] * sv0 - r[1] * sv1 - r[2] * sv2) - djs
-                         : (-r[0] * sv0 - r[1] * sv1) - djs;
-  T beta = T(1) + dis / djs;
-  if (beta > beta_max) beta = beta_max;
-  v[0] = beta * (cvel[0] + vr[0] - vj[0]);
-  v[1] = beta * (cvel[1] + vr[1] - vj[1]);
-  v[2] = beta * (cvel[2] + vr[2] - vj[2]);
-}
-
-
 // ---------------------------------------------------------------------------------
 // Pair pass arithmetic: velocity gradient (kernel_vel_gradients.cu:15-662), forces
 // (kernel_forces.cu:15-865), external force (kernel_ext_force.cu:13-73), dc/dt
@@ -582,6 +450,95 @@ __device__ __forceinline__ T pair_sep(const PairParams<T, DIM>& pp, int wall,
   r[2] = DIM == 3 ? o.z - (T)rec_z<DIM>(rj) : T(0);
   min_image<T, DIM, WRAP>(r[0], r[1], r[2], pp.L, pp.h, wall);
   return norm2(r[0], r[1], r[2], DIM == 3);
+}
+
+// Morris ghost velocity difference of a fluid particle and a wall or colloid particle
+// (kernel_forces.cu:234-418, 590-821; kernel_vel_gradients.cu:162-331, 421-630), seen from the
+// target i: o is the target, rj its partner, r = x_i - x_j.  The fluid particle's velocity
+// relative to the boundary is extrapolated to the solid particle, beta = 1 + (the solid
+// particle's distance from the boundary) / (the fluid one's); whichever of the two the target
+// is, the difference is that of the same two particles, and the lanes of a warp that hold one
+// and the other take the same path.
+template <typename T, int DIM, typename Rec>
+__device__ __forceinline__ void ghost_velocity(const BoxParams& p, const PairParams<T, DIM>& pp,
+                                               const CollView& cv, const PairOwn<T, DIM>& o,
+                                               const Rec& rj, int tj, const T r[3], T v[3]) {
+  const bool own = o.fluid;        // the target is the fluid particle
+  const int ts = own ? tj : o.t;   // the solid particle's type
+  const T vq[3] = {own ? o.v[0] : (T)rj.vx, own ? o.v[1] : (T)rj.vy,
+                   DIM == 3 ? (own ? o.v[2] : (T)rec_vz<DIM>(rj)) : T(0)};
+  const T yq = own ? o.y : (T)rj.y;
+  const T beta_max = (T)p.beta_max;
+  if (ts == 1 || ts == 2) {
+    const T ys = own ? (T)rj.y : o.y;
+    T dq, ds, Vw;
+    if (ts == 1) {
+      dq = yq - (T)p.y_bottom;
+      ds = (T)p.y_bottom - ys;
+      Vw = (T)p.V_bottom;
+    } else {
+      dq = (T)p.y_top - yq;
+      ds = ys - (T)p.y_top;
+      Vw = (T)p.V_top;
+    }
+    T beta = T(1) + quotient(ds, dq);
+    beta = beta <= beta_max ? beta : beta_max;
+    beta = dq > T(0) ? beta : T(1);
+    v[0] = beta * (vq[0] - Vw);
+    v[1] = beta * vq[1];
+    v[2] = beta * vq[2];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] = own ? v[a] : -v[a];
+    return;
+  }
+  const int c = p.coll0 + ts - 3, nc = cv.nc;
+  const T xq = own ? o.x : (T)rj.x, zq = DIM == 3 ? (own ? o.z : (T)rec_z<DIM>(rj)) : T(0);
+  T rc[3] = {xq - (T)cv.cs[CS_X * nc + c], yq - (T)cv.cs[CS_Y * nc + c],
+             DIM == 3 ? zq - (T)cv.cs[CS_Z * nc + c] : T(0)};
+  min_image<T, DIM>(rc[0], rc[1], rc[2], pp.L, pp.h, p.wall);
+  const T d2 = DIM == 3 ? rc[0] * rc[0] + rc[1] * rc[1] + rc[2] * rc[2]
+                        : rc[0] * rc[0] + rc[1] * rc[1];
+  const T R = (T)p.coll_R;
+  T dc, n[3];  // distance from the centre and its direction
+  if constexpr (sizeof(T) == 8) {
+    const T inv = inv_sqrt(d2);
+    dc = d2 * inv;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) n[a] = rc[a] * inv;
+  } else {
+    dc = sqrt(d2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) n[a] = a < DIM ? rc[a] / dc : T(0);
+  }
+  const T dq = dc - R;  // the fluid particle's distance from the surface
+  const T cvel[3] = {(T)cv.cs[CS_VX * nc + c], (T)cv.cs[CS_VY * nc + c],
+                     DIM == 3 ? (T)cv.cs[CS_VZ * nc + c] : T(0)};
+  const T xs = n[0] * R, ys = n[1] * R, zs = n[2] * R;
+  T vr[3];
+  const T wz = (T)cv.cs[CS_OZ * nc + c];
+  if (DIM == 2) {
+    vr[0] = -wz * ys;
+    vr[1] = wz * xs;
+    vr[2] = T(0);
+  } else {
+    const T wx = (T)cv.cs[CS_OX * nc + c], wy = (T)cv.cs[CS_OY * nc + c];
+    vr[0] = wy * zs - wz * ys;
+    vr[1] = wz * xs - wx * zs;
+    vr[2] = wx * ys - wy * xs;
+  }
+  // the separation along the normal, from the solid particle to the fluid one
+  const T along = DIM == 3 ? r[0] * n[0] + r[1] * n[1] + r[2] * n[2] : r[0] * n[0] + r[1] * n[1];
+  const T ds = (own ? along : -along) - dq;
+  T beta = T(1) + quotient(ds, dq);
+  beta = beta <= beta_max ? beta : beta_max;
+  const bool inside = dq < T(0);  // not extrapolated, and without the rotation
+  beta = inside ? T(1) : beta;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const T w = inside ? T(0) : vr[a];
+    // (v_q - V) - w, or (V + w) - v_q
+    v[a] = beta * (own ? (vq[a] - cvel[a]) - w : (cvel[a] + w) - vq[a]);
+  }
 }
 
 // The radial part of a pair's terms.  FP64: 1/|r| and the vector s = (dW/dr / c_gradw) r / |r|,
@@ -713,53 +670,27 @@ __device__ __forceinline__ void pair_term(const BoxParams& p, const PairParams<T
   T r[3];
   const T r2 = pair_sep<T, DIM, WRAP>(pp, p.wall, o, rj, r);
   if (!(r2 < pp.rcutsq)) return;
-  const T vj[3] = {(T)rj.vx, (T)rj.vy, (T)rec_vz<DIM>(rj)};
-  T v[3];
-  if (o.t == tj) {
-    v[0] = o.v[0] - vj[0];
-    v[1] = o.v[1] - vj[1];
-    v[2] = o.v[2] - vj[2];
-  } else if (o.fluid) {
-    ghost_fluid_i<T, DIM>(p, cv, tj, p.coll0, o.x, o.y, o.z, (T)rj.y, o.v, r, pp.L, pp.h, v);
-  } else {
-    ghost_solid_i<T, DIM>(p, cv, o.t, p.coll0, o.y, (T)rj.x, (T)rj.y, (T)rec_z<DIM>(rj), vj, r, pp.L,
-                          pp.h, v);
-  }
+  T v[3] = {o.v[0] - (T)rj.vx, o.v[1] - (T)rj.vy, o.v[2] - (T)rec_vz<DIM>(rj)};
+  if (o.t != tj) ghost_velocity<T, DIM>(p, pp, cv, o, rj, tj, r, v);
   PairRadial<T, DIM> g;
   g.eval(pp, r2, r);
   if (pair_grad) pair_grad_add<DIM>(o, g, v, acc);
   if (pair_force) {
-    T Pi[6], Pj[6], di, dj;
-    if (o.fluid && fluid_j) {
+    // The partner's stress term, by the two particles' kinds: fluid and fluid: its own; fluid i,
+    // solid j: j mirrors i's density and pressure and keeps its own c (kernel_forces.cu:217-233);
+    // solid i: i takes j's density, pressure and c (kernel_forces.cu:320-336; FP64: twice j's
+    // stress, and none of its own at the end of the pass).
+    const bool mirrors = o.fluid && !fluid_j;
+    const T diag = mirrors ? o.press : T(0);
+    const T scale = mirrors ? o.invd * o.invd : (sizeof(T) == 8 && !o.fluid ? T(2) : T(1));
+    T Pi[6], Pj[6];
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        Pi[q] = o.P[q];
-        Pj[q] = rec_P<DIM>(rj, q);
-      }
-      di = o.invd;
-      dj = rj.invd;
-    } else if (o.fluid) {
-      // j mirrors i's density and pressure, keeps its own c (kernel_forces.cu:217-233)
-      const T dsq = o.invd * o.invd;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        Pi[q] = o.P[q];
-        const T diag = (q == 0 || q == 2 || q == 5) ? o.press : T(0);
-        Pj[q] = (diag + rec_P<DIM>(rj, q)) * dsq;
-      }
-      di = o.invd;
-      dj = o.invd;
-    } else {
-      // i takes j's density, pressure and c (kernel_forces.cu:320-336); FP64: twice j's
-      // stress, and none of its own at the end of the pass
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        Pj[q] = (sizeof(T) == 8 ? T(2) : T(1)) * rec_P<DIM>(rj, q);
-        Pi[q] = rec_P<DIM>(rj, q);
-      }
-      di = rj.invd;
-      dj = rj.invd;
+    for (int q = 0; q < 6; ++q) {
+      const T P = rec_P<DIM>(rj, q);
+      Pi[q] = o.fluid ? (T)o.P[q] : P;
+      Pj[q] = ((q == 0 || q == 2 || q == 5) ? diag + P : P) * scale;
     }
+    const T di = o.fluid ? o.invd : (T)rj.invd, dj = fluid_j ? (T)rj.invd : o.invd;
     pair_force_add<DIM>(pp, g, r, v, Pi, Pj, di, dj, acc);
   }
 }
