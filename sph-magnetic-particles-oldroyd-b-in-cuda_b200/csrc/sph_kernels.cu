@@ -8,6 +8,7 @@
 // reference's order (kernel_densities.cu:52-163), so each particle's sums run over the
 // same neighbours in the same order as the reference's gather loops.  All sums are
 // gathers (no atomics), so results are bit-reproducible run to run.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -606,9 +607,338 @@ __device__ __forceinline__ bool stale_cell(const Dev& d, int nc) {
   return d.cell_end[nc] >= d.cell_start[nc] && d.cell_begin[nc] == d.cell_begin[nc + 1];
 }
 
-template <int DIM, int TPC>
+// A particle exactly on the upper box edge: its own neighbour cells, the whole warp testing its
+// candidates.  ti, tb: its slot and box (uniform).  Returns its chunks with hits.
+template <int DIM>
+__device__ __forceinline__ int list_odd_particle(const Dev& d, int ti, int tb) {
+  constexpr int kNZ = DIM == 3 ? 3 : 1;
+  const int lane = threadIdx.x & 31, cap = d.cap;
+  const size_t Np = d.Npad;
+  const BoxParams& tp = d.box[tb];
+  const double4 xt = d.pos[ti];
+  int ax = 0, ay = 0, az = 0;
+  own_cell(tp, xt.x, xt.y, xt.z, ax, ay, az);  // checked above: cannot fail
+  const double tox = ax * tp.cell_size[0];
+  const double toy = ay * tp.cell_size[1] - (tp.wall ? tp.wall_width : 0.0);
+  const double toz = DIM == 3 ? az * tp.cell_size[2] : 0.0;
+  const float tcut2 = (float)tp.list_cut2;
+  const float txi = (float)(xt.x - tox), tyi = (float)(xt.y - toy), tzi = (float)(xt.z - toz);
+  int tcnt = 0, tk = 0;
+  for (int q = 0; q < 9 * kNZ; ++q) {
+    int nc;
+    if (!neighbour_cell<DIM>(tp, ax, ay, az, q, nc)) continue;
+    const int s = d.cell_start[nc] + tp.slot0, e = d.cell_end[nc] + tp.slot0;
+    for (int c0 = s; c0 <= e; c0 += 32) {
+      const int j = c0 + lane;
+      bool hit = false;
+      if (j <= e) {
+        // rare: every candidate at its minimum image about the particle's own cell
+        double4 xj = d.pos[j];
+        const float vx = stale_offset((float)(xj.x - tox), tp.cell_size[0], tp.L[0]);
+        float vy = (float)(xj.y - toy);
+        if (!tp.wall) vy = stale_offset(vy, tp.cell_size[1], tp.L[1]);
+        float vz = (float)(xj.z - toz);
+        if (DIM == 3) vz = stale_offset(vz, tp.cell_size[2], tp.L[2]);
+        const float rx = txi - vx;
+        const float ry = tyi - vy;
+        float r2 = rx * rx + ry * ry;
+        if (DIM == 3) {
+          const float rz = tzi - vz;
+          r2 += rz * rz;
+        }
+        hit = r2 < tcut2;
+      }
+      const unsigned hits = __brev(__ballot_sync(SPH_FULL, hit));
+      if (hits != 0u) {
+        if (lane == 0 && tk < cap) d.nchunk[(size_t)tk * Np + ti] = make_int2(c0, (int)hits);
+        tcnt += __popc(hits);
+        ++tk;
+      }
+    }
+  }
+  if (lane == 0) {
+    d.nbr_cnt[ti] = tcnt;
+    d.nbr_nch[ti] = min(tk, cap);
+  }
+  return tk;
+}
+
+// ---- a warp per cell: the candidate test on the tensor cores ----
+//
+// r_ij^2 - cut^2 = |x_i|^2 - cut^2 + |x_j|^2 - 2 x_i.x_j for a round of 32 particles (rows) and a
+// chunk of 32 candidates (columns) is a matrix product with few terms: mma.m16n8k16, float16
+// operands and float accumulators, the sign of an accumulator being the hit.  Coordinates are
+// offsets from the cell's centre over rcut, each split into two float16 (the second holds what
+// the first rounds away), so that a candidate is eight float16, four words:
+//     (x y) (z n) (x' y') (z' n')         n + n' = |x_j|^2, primes: the second parts
+// A particle's row multiplies them by (-2x -2y) (-2z 1) (-2x -2y) (-2z 1) and, in the upper half
+// of K, the same words once more by (-2x' -2y') (-2z' 0) (-2x' -2y') (-2z' 0); the accumulators
+// start from |x_i|^2 - cut^2.  Offsets are below 2 (cells are at most 4/3 rcut wide), so a split
+// coordinate is within 5e-7 and the square within 1.5e-5 of its value, against the 1e-4 by which
+// list_cut2 exceeds the cutoff that every consumer applies exactly: no neighbour is missed.
+// Candidates further off (minimum-image placement) only have to be outside; their n is held
+// finite.
+//
+// What bounds it: instruction issue, about 165 per chunk against 290 with the packed float test
+// (whose operands and subtractions each lane repeats for every candidate); LIST_FIGURES
+__device__ __forceinline__ unsigned pack_h2(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const unsigned*>(&h);
+}
+__device__ __forceinline__ float2 unpack_h2(unsigned u) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&u));
+}
+__device__ __forceinline__ void mma_16x8x16(unsigned (&d)[4], const unsigned (&a)[4], unsigned b,
+                                            float c01, float c23) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%8}, "
+      "{%9,%9,%10,%10};\n"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b), "f"(c01), "f"(c23));
+}
+// The sign bits of two rows (g and g + 8 of the tile of 16) against TILES tiles of 8 candidates:
+// the lane's candidates 8 u + 2 t and + 1 in bits 31 - 8 u and 30 - 8 u.
+template <int TILES>
+__device__ __forceinline__ void hit_bits(const unsigned (&a)[4], const unsigned (&b)[4], float c01,
+                                         float c23, unsigned& m0, unsigned& m1) {
+  unsigned d[4][4];
+#pragma unroll
+  for (int u = 0; u < TILES; ++u) mma_16x8x16(d[u], a, b[u], c01, c23);
+  unsigned top[4];  // the top bytes of the four tiles' accumulators q, tile 0's first
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const unsigned hi = __byte_perm(d[1][q], d[0][q], 0x7377);  // bytes 3, 2: tiles 0, 1
+    if (TILES == 4) {
+      const unsigned lo = __byte_perm(d[3][q], d[2][q], 0x7773);  // bytes 1, 0 (read below)
+      top[q] = __byte_perm(lo, hi, 0x7610);
+    } else {
+      top[q] = hi;
+    }
+  }
+  constexpr unsigned kKeep = TILES == 4 ? 0x80808080u : 0x80800000u;
+  m0 = (top[0] & kKeep) | ((top[1] & kKeep) >> 1);
+  m1 = (top[2] & kKeep) | ((top[3] & kKeep) >> 1);
+}
+// The four words of a candidate at (x, y, z); keep: it exists.
+__device__ __forceinline__ uint4 candidate_words(float x, float y, float z, bool keep) {
+  constexpr float kFar = 60000.0f;
+  float n = fminf(fmaf(z, z, fmaf(y, y, x * x)), kFar);
+  n = keep ? n : kFar;
+  uint4 w;
+  w.x = pack_h2(x, y);
+  w.y = pack_h2(z, n);
+  const float2 a = unpack_h2(w.x), c = unpack_h2(w.y);
+  w.z = pack_h2(x - a.x, y - a.y);
+  w.w = pack_h2(z - c.x, n - c.y);
+  return w;
+}
+
+template <int DIM>
 __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int split) {
-  static_assert(TPC == 32 || TPC == 16, "a warp or a half-warp per cell");
+  constexpr int kNZ = DIM == 3 ? 3 : 1;
+  __shared__ uint4 stage[kListWarps][32];  // the chunk's candidates, a row of 16 bytes each
+  __shared__ float frame[kListWarps][9];   // lo[3], hi[3], L[3] (frame_offset)
+  // the neighbour cells' candidate ranges and what takes their positions to offsets from this
+  // cell's centre
+  __shared__ int2 range[kListWarps][9 * kNZ];
+  __shared__ double shift[kListWarps][9 * kNZ][DIM];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (step_aborted_warp(d)) return;
+  // a position outside the box (the hash's flag) may be sorted into a cell other than its
+  // own (the linear cell index runs on into the next row): then every candidate is placed
+  // by its minimum image, as in a stale range
+  int out_flag = 0;
+  if (lane == 0) out_flag = *(volatile const int*)(d.err_info + kPosOutside + d.parity);
+  const bool any_out = __shfl_sync(SPH_FULL, out_flag, 0) != 0;
+  // `split` warps per cell, warp `part` of them taking every split-th round of particles
+  const int part = (blockIdx.x * kListWarps + w) % split;
+  const int cell = (blockIdx.x * kListWarps + w) / split;
+  if (cell >= d.Ctot) return;  // whole warps
+  const int b = d.cell_box[cell];
+  const BoxParams& p = d.box[b];
+  const int N0 = p.Ncells[0], N1 = p.Ncells[1], N2 = p.Ncells[2];
+  const int lc = cell - p.cell0;
+  const int cx = lc % N0, cy = (lc / N0) % N1, cz = DIM == 3 ? lc / (N0 * N1) : 0;
+  const int beg = d.cell_begin[cell], end = d.cell_begin[cell + 1];
+  const double ox = cx * p.cell_size[0];
+  const double oy = cy * p.cell_size[1] - (p.wall ? p.wall_width : 0.0);
+  const double oz = DIM == 3 ? cz * p.cell_size[2] : 0.0;
+  // the cell's centre; offsets from it in units of rcut
+  const double mx = ox + 0.5 * p.cell_size[0], my = oy + 0.5 * p.cell_size[1];
+  const double mz = DIM == 3 ? oz + 0.5 * p.cell_size[2] : 0.0;
+  const float inv = (float)p.rcut_inv;
+  const float cut2 = (float)(p.list_cut2 * p.rcut_inv * p.rcut_inv);
+  const int cap = d.cap;  // chunks with hits a particle can store
+  const size_t Np = d.Npad;
+  const int span = end - beg;
+  int maxch = 0;  // the most chunks with hits any particle of this warp had
+  // lane q looks up neighbour cell q (all 3^d loads in flight at once)
+  bool found = false;  // a stale neighbour range
+  if (lane < 9 * kNZ) {
+    int nc, rs = 0, re = -1;
+    if (neighbour_cell<DIM>(p, cx, cy, cz, lane, nc)) {
+      rs = d.cell_start[nc] + p.slot0;
+      re = d.cell_end[nc] + p.slot0;
+      found = stale_cell(d, nc);
+    }
+    range[w][lane] = make_int2(rs, re);
+    const int nx = cx + lane / (3 * kNZ) - 1, ny = cy + (lane / kNZ) % 3 - 1;
+    shift[w][lane][0] = (nx < 0 ? -p.L[0] : nx >= N0 ? p.L[0] : 0.0) - mx;
+    shift[w][lane][1] = (p.wall ? 0.0 : ny < 0 ? -p.L[1] : ny >= N1 ? p.L[1] : 0.0) - my;
+    if (DIM == 3) {
+      const int nz = cz + lane % 3 - 1;
+      shift[w][lane][DIM - 1] = (nz < 0 ? -p.L[2] : nz >= N2 ? p.L[2] : 0.0) - mz;
+    }
+  }
+  // minimum-image placement for the whole warp (see stale_offset)
+  const bool mi = any_out || __any_sync(SPH_FULL, found);
+  if (mi && lane == 0) {
+    for (int q = 0; q < 3; ++q) {
+      const bool wraps = q == 0 || (q == 1 && !p.wall) || (q == 2 && DIM == 3);
+      const float c = (float)(0.5 * p.cell_size[q]), h = (float)(0.5 * p.L[q]);
+      frame[w][q] = wraps ? c - h : -3.0e38f;
+      frame[w][3 + q] = wraps ? c + h : 3.0e38f;
+      frame[w][6 + q] = (float)p.L[q];
+    }
+  }
+  __syncwarp();
+  const float* flo = frame[w];
+  const float* fhi = flo + 3;
+  const float* fL = flo + 6;
+  const int g = lane >> 2, t = lane & 3;  // this lane's part of the fragments
+  const unsigned srow = (unsigned)__cvta_generic_to_shared(&stage[w][lane]);
+  // the particle loop, in the cheap form (per-cell shifts) or the minimum-image one
+  auto walk = [&](auto mi_tag) {
+    constexpr bool kMI = decltype(mi_tag)::value;
+    for (int t0 = part * 32; t0 < span; t0 += split * 32) {
+      // lane 4 g + t holds row g + 8 t: the quad of lanes that gets row g's accumulators in its
+      // four fragments also holds the particles of those four rows
+      const int i = beg + t0 + g + 8 * t;
+      const bool active = i < end;
+      float xi = 0.f, yi = 0.f, zi = 0.f;
+      bool odd = false, lost = false;
+      if (active) {
+        const double4 x = ld_pos<DIM>(d.pos + i);
+        xi = (float)(x.x - mx) * inv;
+        yi = (float)(x.y - my) * inv;
+        zi = DIM == 3 ? (float)(x.z - mz) * inv : 0.f;
+        int ax = 0, ay = 0, az = 0;
+        if (own_cell(p, x.x, x.y, x.z, ax, ay, az)) {
+          odd = (ax != cx) || (ay != cy) || (DIM == 3 && az != cz);
+        } else {
+          // not finite or far outside the box: already reported by the hash; no neighbours
+          lost = true;
+          const bool finite = isfinite(x.x) && isfinite(x.y) && isfinite(x.z);
+          raise_status(d, finite ? kStatCellRange : kStatNaN, d.gid[i], kPhaseLists);
+        }
+      }
+      const bool listed = active && !odd && !lost;
+      // this particle's row: words of the lower and the upper half of K, start value
+      const uint4 cw = candidate_words(xi, yi, zi, true);
+      const float2 h01 = unpack_h2(cw.x), h23 = unpack_h2(cw.y), l01 = unpack_h2(cw.z),
+                   l23 = unpack_h2(cw.w);
+      const float s = listed ? -2.0f : 0.0f;
+      const unsigned lo0 = pack_h2(s * h01.x, s * h01.y), lo1 = pack_h2(s * h23.x, listed ? 1.f : 0.f);
+      const unsigned up0 = pack_h2(s * l01.x, s * l01.y), up1 = pack_h2(s * l23.x, 0.f);
+      const float start = listed ? fmaf(zi, zi, fmaf(yi, yi, xi * xi)) - cut2 : 1.0f;
+      // fragments: word t (of the four) of rows g, g + 8 and of rows g + 16, g + 24
+      unsigned fa[2][4];
+      float fc[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int from = 4 * g + q;  // the lane that holds row g + 8 q
+        const unsigned a0 = __shfl_sync(SPH_FULL, lo0, from), a1 = __shfl_sync(SPH_FULL, lo1, from);
+        const unsigned b0 = __shfl_sync(SPH_FULL, up0, from), b1 = __shfl_sync(SPH_FULL, up1, from);
+        fa[q >> 1][q & 1] = (t & 1) ? a1 : a0;
+        fa[q >> 1][2 + (q & 1)] = (t & 1) ? b1 : b0;
+        fc[q] = __shfl_sync(SPH_FULL, start, from);
+      }
+      const bool two = span - t0 > 16;             // rows 16 .. 31 are in use
+      int2* col = d.nchunk + (listed ? i : 0);     // this particle's chunks, stride Npad
+      int cnt = 0;                                 // its candidates
+      int kc = 0;                                  // its chunks with hits
+      for (int q = 0; q < 9 * kNZ; ++q) {
+        const int cs = range[w][q].x, ce = range[w][q].y;
+        const double sx = shift[w][q][0], sy = shift[w][q][1], sz = shift[w][q][DIM - 1];
+        // (empty ranges and rows beyond a wall have ce < cs)
+        for (int c0 = cs; c0 <= ce; c0 += 32) {
+          const int j = c0 + lane;
+          float vx = 0.f, vy = 0.f, vz = 0.f;
+          if (j <= ce) {
+            const double4 xj = ld_pos<DIM>(d.pos + j);
+            if constexpr (kMI) {
+              vx = frame_offset((float)(xj.x - ox), flo, fhi, fL, 0) - (float)(mx - ox);
+              vy = frame_offset((float)(xj.y - oy), flo, fhi, fL, 1) - (float)(my - oy);
+              if (DIM == 3) vz = frame_offset((float)(xj.z - oz), flo, fhi, fL, 2) - (float)(mz - oz);
+            } else {
+              vx = (float)(xj.x + sx);
+              vy = (float)(xj.y + sy);
+              if (DIM == 3) vz = (float)(xj.z + sz);
+            }
+          }
+          stage[w][lane] = candidate_words(vx * inv, vy * inv, vz * inv, j <= ce);
+          __syncwarp();
+          unsigned fb[4];  // word t of candidates 8 u + g, u = 0 .. 3
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                       : "=r"(fb[0]), "=r"(fb[1]), "=r"(fb[2]), "=r"(fb[3])
+                       : "r"(srow)
+                       : "memory");
+          __syncwarp();  // the stage is refilled by the next chunk
+          // hits of rows g + 8 r
+          unsigned m[4] = {0u, 0u, 0u, 0u};
+          if (ce - c0 >= 16) {
+            hit_bits<4>(fa[0], fb, fc[0], fc[1], m[0], m[1]);
+            if (two) hit_bits<4>(fa[1], fb, fc[2], fc[3], m[2], m[3]);
+          } else {
+            hit_bits<2>(fa[0], fb, fc[0], fc[1], m[0], m[1]);
+            if (two) hit_bits<2>(fa[1], fb, fc[2], fc[3], m[2], m[3]);
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) m[r] >>= 2 * t;
+          // the quad's parts of rows g + 8 r to the lane that holds the row (t = r): bit 31 - k of
+          // `hits` is then candidate k, the consumers' order of leading zeros
+          const bool o1 = (t & 1) != 0, o2 = (t & 2) != 0;
+          const unsigned p0 = (o1 ? m[1] : m[0]) | __shfl_xor_sync(SPH_FULL, o1 ? m[0] : m[1], 1);
+          const unsigned p1 = (o1 ? m[3] : m[2]) | __shfl_xor_sync(SPH_FULL, o1 ? m[2] : m[3], 1);
+          const unsigned hits = (o2 ? p1 : p0) | __shfl_xor_sync(SPH_FULL, o2 ? p0 : p1, 2);
+          if (hits != 0u) {  // a chunk with hits: (first slot, mask) in the next entry
+            if (kc < cap) col[(size_t)kc * Np] = make_int2(c0, (int)hits);
+            cnt += __popc(hits);
+            ++kc;
+          }
+        }
+      }
+      if (active && !odd) {
+        d.nbr_cnt[i] = cnt;
+        d.nbr_nch[i] = min(kc, cap);
+      }
+      maxch = max(maxch, kc);
+      // particles exactly on the upper box edge: their own neighbour cells
+      unsigned odd_mask = __ballot_sync(SPH_FULL, active && odd);
+      while (odd_mask) {
+        const int l = __ffs(odd_mask) - 1;
+        odd_mask &= odd_mask - 1;
+        const int ti = __shfl_sync(SPH_FULL, i, l), tb = __shfl_sync(SPH_FULL, b, l);
+        maxch = max(maxch, list_odd_particle<DIM>(d, ti, tb));
+      }
+    }
+  };
+  if (mi)
+    walk(std::true_type{});
+  else
+    walk(std::false_type{});
+  // warp max of the chunk counts -> capacity check
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) maxch = max(maxch, __shfl_xor_sync(SPH_FULL, maxch, o));
+  if (lane == 0 && maxch > 0) {
+    atomicMax(&d.err_info[kErrMaxCount], maxch);
+    if (maxch > cap) raise_status(d, kStatCapacity, 0, kPhaseLists);
+  }
+}
+
+// ---- a half warp per cell: packed float test ----
+template <int DIM>
+__global__ void __launch_bounds__(kListWarps * 32) k_build_lists_half(Dev d, int split) {
+  constexpr int TPC = 16;
   // candidates staged as three float rows per warp, read four at a time
   __shared__ __align__(16) float stage_x[kListWarps][32];
   __shared__ __align__(16) float stage_y[kListWarps][32];
@@ -653,21 +983,9 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
   };
   const int span = warp_max(end - beg);
   int maxch = 0;  // the most chunks with hits any particle of this warp had
-  // the neighbour cells' candidate ranges: with a warp per cell, lane q loads those of
-  // neighbour cell q up front (all 3^d loads in flight at once) and the loop takes them
-  // by shuffle; a half-warp group loads them as it goes
   constexpr int kNZ = DIM == 3 ? 3 : 1;
-  int rs = 0, re = -1;
   bool found = false;  // a stale neighbour range
-  if (TPC == 32 && live && lane < 9 * kNZ) {
-    int nc;
-    if (neighbour_cell<DIM>(p, cx, cy, cz, lane, nc)) {
-      rs = d.cell_start[nc] + p.slot0;
-      re = d.cell_end[nc] + p.slot0;
-      found = stale_cell(d, nc);
-    }
-  }
-  if (TPC == 16 && live) {
+  if (live) {
     for (int q = gl; q < 9 * kNZ; q += TPC) {
       int nc;
       if (neighbour_cell<DIM>(p, cx, cy, cz, q, nc)) found = found || stale_cell(d, nc);
@@ -735,17 +1053,13 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
             }
             // an empty range where the neighbour row does not exist (walls) or the group idles
             int s = 0, e = -1;
-            if (TPC == 32) {
-              const int q = ((ddx + 1) * 3 + (ddy + 1)) * kNZ + (DIM == 3 ? ddz + 1 : 0);
-              s = __shfl_sync(SPH_FULL, rs, q);
-              e = __shfl_sync(SPH_FULL, re, q);
-            } else if (live && ny >= 0 && ny < N1) {
+            if (live && ny >= 0 && ny < N1) {
               const int nc = p.cell0 + (DIM == 3 ? (nz * N1 + ny) * N0 + nx : ny * N0 + nx);
               s = d.cell_start[nc] + p.slot0;
               e = d.cell_end[nc] + p.slot0;
             }
             const int nch = e >= s ? (e - s + TPC) / TPC : 0;
-            const int nchw = TPC == 32 ? nch : warp_max(nch);
+            const int nchw = warp_max(nch);
             for (int k = 0; k < nchw; ++k) {
               const int c0 = s + k * TPC;
               const int j = c0 + gl;
@@ -767,25 +1081,22 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
               if (DIM == 3) stz[gl] = vz;
               __syncwarp();
               const int n = k < nch ? min(TPC, e - c0 + 1) : 0;
-              // hit mask of this chunk; staged candidate q is slot c0 + q.  A half-warp group
-              // runs a fixed trip count, which keeps both halves on one instruction stream.
-              const int m = TPC == 32 ? (n + 3) & ~3 : TPC;
+              // hit mask of this chunk; staged candidate q is slot c0 + q.  Both halves run a
+              // fixed trip count, which keeps them on one instruction stream.
               unsigned hits = 0u;
-              if (TPC == 16 || listed) {
-  #pragma unroll 1
-                for (int q = 0; q < m; q += 4) {
-                  const ulonglong2 cx4 = *reinterpret_cast<const ulonglong2*>(stx + q);
-                  const ulonglong2 cy4 = *reinterpret_cast<const ulonglong2*>(sty + q);
-                  const ulonglong2 cz4 = DIM == 3 ? *reinterpret_cast<const ulonglong2*>(stz + q)
-                                                  : make_ulonglong2(0ull, 0ull);
-                  hits = list_test2<DIM>(hits, xi2, yi2, zi2, ncut22, cx4.x, cy4.x, cz4.x);
-                  hits = list_test2<DIM>(hits, xi2, yi2, zi2, ncut22, cx4.y, cy4.y, cz4.y);
-                }
-                // first candidate was shifted in first: align it to bit 31 (bit 31 - q is
-                // candidate q, the consumers' order of leading zeros)
-                hits = m > 0 ? hits << (32 - m) : 0u;
-                if (TPC == 16) hits &= (listed && n > 0) ? ~(0xFFFFFFFFu >> n) : 0u;
+#pragma unroll 1
+              for (int q = 0; q < TPC; q += 4) {
+                const ulonglong2 cx4 = *reinterpret_cast<const ulonglong2*>(stx + q);
+                const ulonglong2 cy4 = *reinterpret_cast<const ulonglong2*>(sty + q);
+                const ulonglong2 cz4 = DIM == 3 ? *reinterpret_cast<const ulonglong2*>(stz + q)
+                                                : make_ulonglong2(0ull, 0ull);
+                hits = list_test2<DIM>(hits, xi2, yi2, zi2, ncut22, cx4.x, cy4.x, cz4.x);
+                hits = list_test2<DIM>(hits, xi2, yi2, zi2, ncut22, cx4.y, cy4.y, cz4.y);
               }
+              // first candidate was shifted in first: align it to bit 31 (bit 31 - q is
+              // candidate q, the consumers' order of leading zeros)
+              hits <<= 32 - TPC;
+              hits &= (listed && n > 0) ? ~(0xFFFFFFFFu >> n) : 0u;
               if (hits != 0u) {  // a chunk with hits: (first slot, mask) in the next entry
                 if (kc < cap) col[(size_t)kc * Np] = make_int2(c0, (int)hits);
                 cnt += __popc(hits);
@@ -799,62 +1110,13 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
         d.nbr_nch[i] = min(kc, cap);
       }
       maxch = max(maxch, kc);
-      // particles exactly on the upper box edge: their own neighbour cells, the whole warp
-      // testing one such particle's candidates at a time
+      // particles exactly on the upper box edge: their own neighbour cells
       unsigned odd_mask = __ballot_sync(SPH_FULL, active && odd);
       while (odd_mask) {
         const int l = __ffs(odd_mask) - 1;
         odd_mask &= odd_mask - 1;
-        // the particle and its cell's geometry, from the lane that holds it
-        const int ti = __shfl_sync(SPH_FULL, i, l);
-        const int tb = __shfl_sync(SPH_FULL, b, l);
-        const BoxParams& tp = d.box[tb];
-        const double4 xt = d.pos[ti];
-        int ax = 0, ay = 0, az = 0;
-        own_cell(tp, xt.x, xt.y, xt.z, ax, ay, az);  // checked above: cannot fail
-        const double tox = ax * tp.cell_size[0];
-        const double toy = ay * tp.cell_size[1] - (tp.wall ? tp.wall_width : 0.0);
-        const double toz = DIM == 3 ? az * tp.cell_size[2] : 0.0;
-        const float tcut2 = (float)tp.list_cut2;
-        const float txi = (float)(xt.x - tox), tyi = (float)(xt.y - toy), tzi = (float)(xt.z - toz);
-        int tcnt = 0, tk = 0;
-        for (int q = 0; q < 9 * kNZ; ++q) {
-          int nc;
-          if (!neighbour_cell<DIM>(tp, ax, ay, az, q, nc)) continue;
-          const int s = d.cell_start[nc] + tp.slot0, e = d.cell_end[nc] + tp.slot0;
-          for (int c0 = s; c0 <= e; c0 += 32) {
-            const int j = c0 + lane;
-            bool hit = false;
-            if (j <= e) {
-              // rare: every candidate at its minimum image about the particle's own cell
-              double4 xj = d.pos[j];
-              const float vx = stale_offset((float)(xj.x - tox), tp.cell_size[0], tp.L[0]);
-              float vy = (float)(xj.y - toy);
-              if (!tp.wall) vy = stale_offset(vy, tp.cell_size[1], tp.L[1]);
-              float vz = (float)(xj.z - toz);
-              if (DIM == 3) vz = stale_offset(vz, tp.cell_size[2], tp.L[2]);
-              const float rx = txi - vx;
-              const float ry = tyi - vy;
-              float r2 = rx * rx + ry * ry;
-              if (DIM == 3) {
-                const float rz = tzi - vz;
-                r2 += rz * rz;
-              }
-              hit = r2 < tcut2;
-            }
-            const unsigned hits = __brev(__ballot_sync(SPH_FULL, hit));
-            if (hits != 0u) {
-              if (lane == 0 && tk < cap) d.nchunk[(size_t)tk * Np + ti] = make_int2(c0, (int)hits);
-              tcnt += __popc(hits);
-              ++tk;
-            }
-          }
-        }
-        if (lane == 0) {
-          d.nbr_cnt[ti] = tcnt;
-          d.nbr_nch[ti] = min(tk, cap);
-        }
-        maxch = max(maxch, tk);
+        const int ti = __shfl_sync(SPH_FULL, i, l), tb = __shfl_sync(SPH_FULL, b, l);
+        maxch = max(maxch, list_odd_particle<DIM>(d, ti, tb));
       }
     }
   };
@@ -2029,11 +2291,11 @@ int launch_build_lists_dim(const Launch& L, int dim) {
   const int nb = blocks(blocks(L.d.Ctot, half ? 2 : 1) * split, kListWarps);
   constexpr int nt = kListWarps * 32;
   if (dim == 3) {
-    if (half) k_build_lists<3, 16><<<nb, nt, 0, S(L)>>>(L.d, split);
-    else k_build_lists<3, 32><<<nb, nt, 0, S(L)>>>(L.d, split);
+    if (half) k_build_lists_half<3><<<nb, nt, 0, S(L)>>>(L.d, split);
+    else k_build_lists<3><<<nb, nt, 0, S(L)>>>(L.d, split);
   } else {
-    if (half) k_build_lists<2, 16><<<nb, nt, 0, S(L)>>>(L.d, split);
-    else k_build_lists<2, 32><<<nb, nt, 0, S(L)>>>(L.d, split);
+    if (half) k_build_lists_half<2><<<nb, nt, 0, S(L)>>>(L.d, split);
+    else k_build_lists<2><<<nb, nt, 0, S(L)>>>(L.d, split);
   }
   return check(L);
 }
