@@ -208,7 +208,7 @@ __device__ __forceinline__ void raise_status(const Dev& d, unsigned bit, int inf
 // build writes: nchunk[k * Npad + i] = (first slot, hit mask) of the particle's k-th chunk
 // with hits (nbr_nch[i] of them), bit 31 - q of the mask meaning slot first + q (the first
 // candidate in the highest bit, so that a count of leading zeros gives its offset).  Candidates come
-// chunk by chunk and, inside a chunk, by increasing slot: the reference's candidate order.
+// chunk by chunk and, inside a chunk, by increasing slot.
 // Every stored chunk has a hit, so moving to the next one never loops; its entry is loaded
 // one chunk ahead.  next() gives nbr_cnt[i] candidates, then -1.  It has no branch: the
 // lanes of a warp move to their next chunks at different positions, and a branch taken by

@@ -4,9 +4,9 @@
 // neighbour search, so that every cell's particles are contiguous in HBM.  State is SoA /
 // packed AoS (pos = double4 x,y,z,mass; vel = double4) and is permuted into the new order
 // once per search (k_reorder).  The pair phases read per-particle neighbour lists built by
-// a warp-per-cell kernel (k_build_lists) that walks the 3^d neighbour cells in the
-// reference's order (kernel_densities.cu:52-163), so each particle's sums run over the
-// same neighbours in the same order as the reference's gather loops.  All sums are
+// a warp-per-cell kernel (k_build_lists) that walks the 3^d neighbour cells (y slowest, then
+// z, then x), so each particle's sums run over the same neighbours as the reference's gather
+// loops (kernel_densities.cu:52-163), rows of cells along x one after the other.  All sums are
 // gathers (no atomics), so results are bit-reproducible run to run.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -473,18 +473,18 @@ __device__ __forceinline__ void density_epilogue(const Dev& d, int i, const BoxP
 }
 
 // One warp per cell: the cell's particles (<= 32 per round) test the candidates of the
-// 3^d neighbour cells, staged 32 at a time in shared memory as float offsets from the
-// cell corner.  Candidate ranges come from the reference-semantics cell_start / cell_end,
-// so the candidate set and order are the reference's (kernel_densities.cu:52-163), stale
-// ranges included.  The float test uses a slightly enlarged cutoff; consumers apply the
+// 3^d neighbour cells, staged 32 at a time in shared memory as offsets from the cell.
+// Candidate ranges are those of the reference-semantics cell_start / cell_end, so the
+// candidates are the reference's (kernel_densities.cu:52-163), stale
+// ranges included.  The test uses a slightly enlarged cutoff; consumers apply the
 // exact test.
 //
 // The lists are chunks with hit masks, not indices.  Candidates come in chunks of up to 32
-// consecutive slots of one neighbour cell; for every chunk in which it has a hit, a particle
+// consecutive slots of one range; for every chunk in which it has a hit, a particle
 // stores one 8-byte entry (the chunk's first slot, a 32-bit mask whose bit 31 - q means slot
 // first + q is a candidate), chunk-major: nchunk[k * Npad + i], so that consumers walking
 // their lists in step read neighbouring words.  Decoding the entries in order, bit by bit,
-// gives the neighbours in the order of an index list (the reference's candidate order), at
+// gives the neighbours in the order of an index list (the candidate order), at
 // 8 bytes per chunk with hits (about 20 in 3D) instead of 4 bytes per neighbour (about
 // 108), and the build needs no per-lane append loop: a chunk's hits are one store.
 //
@@ -495,10 +495,9 @@ __device__ __forceinline__ void density_epilogue(const Dev& d, int i, const BoxP
 // separate k_density pass: the per-lane hit loops diverge and the warp runs the FP64
 // kernel evaluation for its busiest lane.)
 //
-// TPC (threads per cell) is 32 or 16.  With 16, each half-warp works on its own cell:
-// 2D cells at overlap 4 hold about 16 particles, so a whole warp per cell leaves half of
-// its lanes idle.  The neighbours are the same either way (same candidates, same order);
-// chunks are then 16 slots long.
+// With 16 threads per cell (k_build_lists_half) each half-warp works on its own cell, chunks are
+// 16 slots long and the test is in packed float.  The neighbours are the same either way (same
+// candidates, same order).
 //
 // Blocks of 4 warps, measured against 8 (128^3 list build 1.66 vs 1.88 ms; 2D ensemble
 // 1.15 vs 1.19 ms, with the test loop not unrolled).
@@ -578,15 +577,16 @@ __device__ __forceinline__ float frame_offset(float v, const float* lo, const fl
   return v < lo[q] ? v + L[q] : v;
 }
 
-// Neighbour cell q (0 .. 3^d - 1, x slowest) of cell (cx, cy, cz) of box p with the
-// periodic wrap; false where the row does not exist (beyond a wall).
+// Neighbour cell q (0 .. 3^d - 1: dy slowest, then dz, then dx) of cell (cx, cy, cz) of box p
+// with the periodic wrap; false where the row does not exist (beyond a wall).  The three cells
+// of a row lie one after the other in memory, up to the wrap.
 template <int DIM>
 __device__ __forceinline__ bool neighbour_cell(const BoxParams& p, int cx, int cy, int cz,
                                                int q, int& nc) {
   constexpr int kNZ = DIM == 3 ? 3 : 1;
   const int N0 = p.Ncells[0], N1 = p.Ncells[1], N2 = p.Ncells[2];
-  int nx = cx + q / (3 * kNZ) - 1, ny = cy + (q / kNZ) % 3 - 1;
-  int nz = DIM == 3 ? cz + q % 3 - 1 : 0;
+  int nx = cx + q % 3 - 1, ny = cy + q / (3 * kNZ) - 1;
+  int nz = DIM == 3 ? cz + (q / 3) % 3 - 1 : 0;
   if (nx < 0) nx += N0;
   if (nx >= N0) nx -= N0;
   if (DIM == 3) {
@@ -676,11 +676,18 @@ __device__ __forceinline__ int list_odd_particle(const Dev& d, int ti, int tb) {
 // start from |x_i|^2 - cut^2.  Offsets are below 2 (cells are at most 4/3 rcut wide), so a split
 // coordinate is within 5e-7 and the square within 1.5e-5 of its value, against the 1e-4 by which
 // list_cut2 exceeds the cutoff that every consumer applies exactly: no neighbour is missed.
-// Candidates further off (minimum-image placement) only have to be outside; their n is held
-// finite.
+// Candidates further off (minimum-image placement) only have to be outside: held within 200 rcut,
+// and n below what a float16 holds.
 //
-// What bounds it: instruction issue, about 165 per chunk against 290 with the packed float test
-// (whose operands and subtractions each lane repeats for every candidate); LIST_FIGURES
+// What bounds it: instruction issue.  The packed float test (k_build_lists_half), whose operands
+// and subtractions each lane repeats for every candidate, took most of a chunk's instructions;
+// with the matrix product they are staging (FP64 positions to four words), eight matrix
+// instructions and the exchange of the masks.  A row of three neighbour cells is one range of
+// slots, since their particles follow one another in memory, so chunks are nearly full: cells of
+// 16 particles took 9 chunks, their rows take 6, and the consumers' lists are shorter as well.
+// Measured (ms; packed float test cell by cell / matrix product cell by cell / by rows): 128^3
+// 0.857 / 0.641 / 0.591, 96^3 with colloids 0.346 / 0.265 / 0.255, 61 x 53 x 67 0.129 / 0.099 / 0.094, 512 2D boxes 0.657 / 0.683 / 0.617, one 64^2
+// box 0.0140 / 0.0127 / 0.0119; the 128^3 step's pair pass went from 2.77 to 2.70 with the shorter lists.
 __device__ __forceinline__ unsigned pack_h2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const unsigned*>(&h);
@@ -737,8 +744,8 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
   constexpr int kNZ = DIM == 3 ? 3 : 1;
   __shared__ uint4 stage[kListWarps][32];  // the chunk's candidates, a row of 16 bytes each
   __shared__ float frame[kListWarps][9];   // lo[3], hi[3], L[3] (frame_offset)
-  // the neighbour cells' candidate ranges and what takes their positions to offsets from this
-  // cell's centre
+  // the candidates as ranges of consecutive slots (a row of three neighbour cells is one, or two
+  // at the periodic wrap), and what takes their positions to offsets from this cell's centre
   __shared__ int2 range[kListWarps][9 * kNZ];
   __shared__ double shift[kListWarps][9 * kNZ][DIM];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -772,25 +779,43 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
   const int span = end - beg;
   int maxch = 0;  // the most chunks with hits any particle of this warp had
   // lane q looks up neighbour cell q (all 3^d loads in flight at once)
-  bool found = false;  // a stale neighbour range
+  int rs = 0, re = -1, nb = 0, ne = -1;  // the recorded range, the range of this search
   if (lane < 9 * kNZ) {
-    int nc, rs = 0, re = -1;
+    int nc;
     if (neighbour_cell<DIM>(p, cx, cy, cz, lane, nc)) {
       rs = d.cell_start[nc] + p.slot0;
       re = d.cell_end[nc] + p.slot0;
-      found = stale_cell(d, nc);
-    }
-    range[w][lane] = make_int2(rs, re);
-    const int nx = cx + lane / (3 * kNZ) - 1, ny = cy + (lane / kNZ) % 3 - 1;
-    shift[w][lane][0] = (nx < 0 ? -p.L[0] : nx >= N0 ? p.L[0] : 0.0) - mx;
-    shift[w][lane][1] = (p.wall ? 0.0 : ny < 0 ? -p.L[1] : ny >= N1 ? p.L[1] : 0.0) - my;
-    if (DIM == 3) {
-      const int nz = cz + lane % 3 - 1;
-      shift[w][lane][DIM - 1] = (nz < 0 ? -p.L[2] : nz >= N2 ? p.L[2] : 0.0) - mz;
+      nb = d.cell_begin[nc];
+      ne = d.cell_begin[nc + 1] - 1;
     }
   }
-  // minimum-image placement for the whole warp (see stale_offset)
-  const bool mi = any_out || __any_sync(SPH_FULL, found);
+  // a stale range, or a position outside the box: minimum-image placement for the whole warp
+  // (see stale_offset)
+  const bool mi = any_out || __any_sync(SPH_FULL, re >= rs && ne < nb);
+  // Otherwise the recorded ranges are this search's, and the cells of a row that follow one
+  // another in x do so in memory: the first of them takes the others' slots.
+  const int ne1 = __shfl_down_sync(SPH_FULL, ne, 1), ne2 = __shfl_down_sync(SPH_FULL, ne, 2);
+  if (!mi) {
+    const int dx = lane % 3;  // cell cx - 1, cx or cx + 1 of the row
+    rs = nb;
+    re = ne;
+    if (dx == 0 && cx > 0) re = cx < N0 - 1 ? ne2 : ne1;
+    if (dx == 1) re = cx == 0 ? ne1 : rs - 1;
+    if (dx == 2 && cx < N0 - 1) re = rs - 1;
+  }
+  const unsigned filled = __ballot_sync(SPH_FULL, lane < 9 * kNZ && re >= rs);
+  const int nseg = __popc(filled);
+  if ((filled >> lane) & 1u) {
+    const int at = __popc(filled & ((1u << lane) - 1u));
+    range[w][at] = make_int2(rs, re);
+    const int nx = cx + lane % 3 - 1, ny = cy + lane / (3 * kNZ) - 1;
+    shift[w][at][0] = (nx < 0 ? -p.L[0] : nx >= N0 ? p.L[0] : 0.0) - mx;
+    shift[w][at][1] = (p.wall ? 0.0 : ny < 0 ? -p.L[1] : ny >= N1 ? p.L[1] : 0.0) - my;
+    if (DIM == 3) {
+      const int nz = cz + (lane / 3) % 3 - 1;
+      shift[w][at][DIM - 1] = (nz < 0 ? -p.L[2] : nz >= N2 ? p.L[2] : 0.0) - mz;
+    }
+  }
   if (mi && lane == 0) {
     for (int q = 0; q < 3; ++q) {
       const bool wraps = q == 0 || (q == 1 && !p.wall) || (q == 2 && DIM == 3);
@@ -856,10 +881,9 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
       int2* col = d.nchunk + (listed ? i : 0);     // this particle's chunks, stride Npad
       int cnt = 0;                                 // its candidates
       int kc = 0;                                  // its chunks with hits
-      for (int q = 0; q < 9 * kNZ; ++q) {
+      for (int q = 0; q < nseg; ++q) {
         const int cs = range[w][q].x, ce = range[w][q].y;
         const double sx = shift[w][q][0], sy = shift[w][q][1], sz = shift[w][q][DIM - 1];
-        // (empty ranges and rows beyond a wall have ce < cs)
         for (int c0 = cs; c0 <= ce; c0 += 32) {
           const int j = c0 + lane;
           float vx = 0.f, vy = 0.f, vz = 0.f;
@@ -875,7 +899,15 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists(Dev d, int spli
               if (DIM == 3) vz = (float)(xj.z + sz);
             }
           }
-          stage[w][lane] = candidate_words(vx * inv, vy * inv, vz * inv, j <= ce);
+          vx *= inv;
+          vy *= inv;
+          vz *= inv;
+          if constexpr (kMI) {  // no further than float16 reaches
+            vx = fminf(fmaxf(vx, -200.f), 200.f);
+            vy = fminf(fmaxf(vy, -200.f), 200.f);
+            vz = fminf(fmaxf(vz, -200.f), 200.f);
+          }
+          stage[w][lane] = candidate_words(vx, vy, vz, j <= ce);
           __syncwarp();
           unsigned fb[4];  // word t of candidates 8 u + g, u = 0 .. 3
           asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -1036,9 +1068,9 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists_half(Dev d, int
       int2* col = d.nchunk + (listed ? i : 0);  // this particle's chunks, stride Npad
       int cnt = 0;                              // this lane's candidates
       int kc = 0;                               // this lane's chunks with hits
-      for (int ddx = -1; ddx <= 1; ++ddx)
-        for (int ddy = -1; ddy <= 1; ++ddy)
-          for (int ddz = (DIM == 3 ? -1 : 0); ddz <= (DIM == 3 ? 1 : 0); ++ddz) {
+      for (int ddy = -1; ddy <= 1; ++ddy)
+        for (int ddz = (DIM == 3 ? -1 : 0); ddz <= (DIM == 3 ? 1 : 0); ++ddz)
+          for (int ddx = -1; ddx <= 1; ++ddx) {
             int nx = cx + ddx, ny = cy + ddy, nz = cz + ddz;
             double sx = 0.0, sy = 0.0, sz = 0.0;
             if (nx < 0) { nx += N0; sx = -p.L[0]; }
@@ -1248,7 +1280,7 @@ __global__ void k_density(Dev d) {
 
 // Density over neighbour-cell tiles: one warp per cell, as the list build.  The positions
 // of the neighbour cells' candidate ranges (the list build's ranges, stale ones included)
-// are staged in shared memory by coalesced copies, in phases of 9 cells (the dx = -1, 0, +1
+// are staged in shared memory by coalesced copies, in phases of 9 cells (the dy = -1, 0, +1
 // planes in 3D; all 9 cells at once in 2D), and every lane walks its own list in order,
 // reading each neighbour from the tile.  The sums are those of k_density term for term:
 // the same list order, the same arithmetic; only where the position is read from differs.
@@ -1281,8 +1313,8 @@ __global__ void __launch_bounds__(kDensWarps * 32) k_density_cells(Dev d) {
   // candidate range of neighbour cell `lane` (the list build's, kernel_densities.cu:52-163)
   int rs = 0, re = -1;
   if (lane < kNR) {
-    const int ddx = lane / (3 * kNZ) - 1, ddy = (lane / kNZ) % 3 - 1;
-    const int ddz = DIM == 3 ? lane % 3 - 1 : 0;
+    const int ddx = lane % 3 - 1, ddy = lane / (3 * kNZ) - 1;
+    const int ddz = DIM == 3 ? (lane / 3) % 3 - 1 : 0;
     int nx = cx + ddx, ny = cy + ddy, nz = cz + ddz;
     if (nx < 0) nx += N0;
     if (nx >= N0) nx -= N0;
