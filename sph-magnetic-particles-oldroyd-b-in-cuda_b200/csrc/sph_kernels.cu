@@ -1448,6 +1448,14 @@ __global__ void k_pressure(Dev d) {
 // while the current ones are evaluated.  Each lane then reads its records
 // from shared memory (row stride padded by one piece: conflict-free).
 //
+// What bounds the 3D FP64 pass is the load/store pipe all of this goes through (79 % busy at 96^3,
+// the FP64 pipe 34 %, issue 49 %): per position of a warp 32 passes for the copies, 32 for the
+// records and one for each shuffle or slot.  There the slots go through shared memory, three
+// passes in place of eight shuffles, and records are read 16 bytes at a time: 128^3 pair pass
+// 2.70 -> 2.51 ms FP64, 2.12 -> 2.06 mixed.  In 2D, with 64- and 32-byte records, the same slots
+// cost more than the four or two shuffles (512 boxes 2.58 -> 2.76 ms FP64, 1.87 -> 1.91 mixed),
+// except in the wide walk (one 64^2 box 28.6 -> 26.6 us).
+//
 // Launch shape of the pair pass per precision and dimension, as measured on B200.  Every pass
 // evaluates one list position per step: with the fluid-fluid form of that walk, evaluating two
 // positions side by side (to overlap their dependency chains) measured slower everywhere
@@ -1510,6 +1518,8 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   else
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+template <typename Rec>
+constexpr bool kThroughL1 = std::is_same<Rec, RecD>::value || std::is_same<Rec, RecF>::value;
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -1517,8 +1527,8 @@ __device__ __forceinline__ void cp_async_wait_prev() {
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
 }
 
-// Lane `lane` copies its piece of the records the warp's lanes list at one position
-// (jn: this lane's neighbour there, -1 for none) into row block `buf`.
+// Copies the records the warp's lanes list at one position into row block `buf`, lane `lane`
+// one 16-byte piece per copy.  jn: this lane's slot, -1 for none; each copy's slots by a shuffle.
 template <typename Rec>
 __device__ __forceinline__ void stage_records(int4* buf, const Rec* __restrict__ rec, int jn,
                                               int lane) {
@@ -1529,19 +1539,69 @@ __device__ __forceinline__ void stage_records(int4* buf, const Rec* __restrict__
     const int r = t * St::kPerCopy + lane / St::kPieces;
     const int jr = __shfl_sync(SPH_FULL, jn, r);
     if (jr >= 0)
-      cp_async16<std::is_same<Rec, RecD>::value || std::is_same<Rec, RecF>::value>(
-          buf + r * St::kStride + piece, reinterpret_cast<const int4*>(rec + jr) + piece);
+      cp_async16<kThroughL1<Rec>>(buf + r * St::kStride + piece,
+                                  reinterpret_cast<const int4*>(rec + jr) + piece);
+  }
+}
+// The same with the lanes' slots in shared memory (idx): the kPieces lanes that move a record
+// move those of kPieces successive rows, whose slots they read in one or two loads.
+template <typename Rec>
+__device__ __forceinline__ void stage_records(int4* buf, const Rec* __restrict__ rec,
+                                              const int* idx, int lane) {
+  using St = PairStage<Rec>;
+  constexpr int kP = St::kPieces;
+  static_assert(kP % 4 == 0, "slots are read four at a time");
+  const int piece = lane % kP, r0 = lane - piece;
+  int j[kP];
+#pragma unroll
+  for (int t = 0; t < kP; t += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(idx + r0 + t);
+    j[t] = v.x;
+    j[t + 1] = v.y;
+    j[t + 2] = v.z;
+    j[t + 3] = v.w;
+  }
+#pragma unroll
+  for (int t = 0; t < kP; ++t) {
+    if (j[t] >= 0)
+      cp_async16<kThroughL1<Rec>>(buf + (r0 + t) * St::kStride + piece,
+                                  reinterpret_cast<const int4*>(rec + j[t]) + piece);
   }
 }
 
-// A lane's view of one staged record: FP64 records are read in place, each field loaded
-// from shared memory where the pair term uses it, which keeps the 128-byte record out of
-// the register file; float records are copied into registers.
+// A lane's view of one staged record.  FP64 2D records are read in place, each field loaded from
+// shared memory where the pair term uses it, which keeps them out of the register file; float
+// records are copied into registers, and so are the FP64 3D ones, 16 bytes a load: the fields
+// read one by one took 11 loads, the 8-byte ones among them with two-way bank conflicts (128^3
+// pair pass 2.59 -> 2.56 ms).
 template <typename T, typename Rec>
 struct StagedRec {
   const Rec& r;
   __device__ __forceinline__ explicit StagedRec(const int4* src)
       : r(*reinterpret_cast<const Rec*>(src)) {}
+};
+template <>
+struct StagedRec<double, RecD> {
+  RecD r;
+  __device__ __forceinline__ explicit StagedRec(const int4* src) {
+    const double2* q = reinterpret_cast<const double2*>(src);
+    const double2 a = q[0], b = q[1], c = q[2], e = q[3], f = q[4], g = q[5];
+    const int4 h = src[6];
+    r.x = a.x;
+    r.y = a.y;
+    r.z = b.x;
+    r.vx = b.y;
+    r.vy = c.x;
+    r.vz = c.y;
+    r.P[0] = e.x;
+    r.P[1] = e.y;
+    r.P[2] = f.x;
+    r.P[3] = f.y;
+    r.P[4] = g.x;
+    r.P[5] = g.y;
+    r.invd = __hiloint2double(h.y, h.x);
+    r.tinfo = h.z;
+  }
 };
 template <typename Rec>
 struct StagedRec<float, Rec> {
@@ -1561,6 +1621,7 @@ struct PairWalk {
   const Dev& d;
   const Rec* __restrict__ rec;
   int4* sb;                      // the warp's staging rows
+  int* idx;                      // slots of two (wide walk: four) positions, 32 each
   int lane, i, n, nmax;
   const BoxParams& p;
   const PairParams<T, DIM>& pp;
@@ -1575,17 +1636,34 @@ __device__ __forceinline__ void pair_walk(const PairWalk<T, DIM>& W, NbrIter& it
                                            PairAcc<T, DIM>& acc) {
   using Rec = typename RecFor<T, DIM>::type;
   using St = PairStage<Rec>;
+  constexpr bool kIdx = DIM == 3;  // slots by way of shared memory, two positions ahead
   const int n = W.n, lane = W.lane;
-  int jc = n > 0 ? it.next() : -1;
+  int jc = n > 0 ? it.next() : -1, jn = -1, j2 = -1;
   // 2D records carry no type word: the neighbour's is read from the type array one
   // position ahead, with its record's copy
   int tc = DIM == 2 && jc >= 0 ? __ldg(&W.d.tinfo[jc]) : 0;
-  stage_records<Rec>(W.sb, W.rec, jc, lane);
+  if constexpr (kIdx) {
+    jn = n > 1 ? it.next() : -1;
+    W.idx[lane] = jc;
+    W.idx[32 + lane] = jn;
+    __syncwarp();
+    stage_records<Rec>(W.sb, W.rec, W.idx, lane);
+    __syncwarp();
+  } else {
+    stage_records<Rec>(W.sb, W.rec, jc, lane);
+  }
   cp_async_commit();
   for (int k = 0; k < W.nmax; ++k) {
     const int k1 = k + 1;
-    const int jn = k1 < n ? it.next() : -1;
-    if (k1 < W.nmax) stage_records<Rec>(W.sb + (k1 & 1) * St::kRows, W.rec, jn, lane);
+    if constexpr (kIdx) {
+      const int b1 = k1 & 1;
+      if (k1 < W.nmax) stage_records<Rec>(W.sb + b1 * St::kRows, W.rec, W.idx + b1 * 32, lane);
+      j2 = k + 2 < n ? it.next() : -1;
+      W.idx[(b1 ^ 1) * 32 + lane] = j2;  // position k's are no longer read, k + 2's after a barrier
+    } else {
+      jn = k1 < n ? it.next() : -1;
+      if (k1 < W.nmax) stage_records<Rec>(W.sb + (k1 & 1) * St::kRows, W.rec, jn, lane);
+    }
     const int tn = DIM == 2 && jn >= 0 ? __ldg(&W.d.tinfo[jn]) : 0;
     cp_async_commit();
     cp_async_wait_prev();  // position k has landed (this lane's copies) ...
@@ -1602,6 +1680,7 @@ __device__ __forceinline__ void pair_walk(const PairWalk<T, DIM>& W, NbrIter& it
       pair_term<T, DIM, WRAP>(W.p, W.pp, W.cv, W.o, R.r, tj, acc);
     __syncwarp();  // buffer k & 1 is refilled at position k + 2
     jc = jn;
+    if constexpr (kIdx) jn = j2;
     tc = tn;
   }
 }
@@ -1619,9 +1698,14 @@ __device__ __forceinline__ void pair_walk_wide(const PairWalk<T, DIM>& W, NbrIte
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       j[u] = k + u < n ? it.next() : -1;
-      if (k + u < W.nmax) stage_records<Rec>(W.sb + (buf * 2 + u) * St::kRows, W.rec, j[u], lane);
+      W.idx[(buf * 2 + u) * 32 + lane] = j[u];
       t[u] = j[u] >= 0 ? __ldg(&W.d.tinfo[j[u]]) : 0;
     }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (k + u < W.nmax)
+        stage_records<Rec>(W.sb + (buf * 2 + u) * St::kRows, W.rec, W.idx + (buf * 2 + u) * 32, lane);
     cp_async_commit();
   };
   fetch(0, 0, jc, tc);
@@ -1668,6 +1752,7 @@ __global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
   using St = PairStage<Rec>;
   // per warp: a double buffer of staged positions
   __shared__ int4 stage[Sh::kWarps][WIDE ? 4 : 2][St::kRows];
+  __shared__ __align__(16) int slots[DIM == 3 || WIDE ? Sh::kWarps : 1][WIDE ? 4 : 2][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wbase = (blockIdx.x * Sh::kWarps + w) * 32;
   if (wbase >= d.Ntot) return;  // whole warps only: the lanes below cooperate
@@ -1696,7 +1781,7 @@ __global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
   for (int s = 16; s > 0; s >>= 1) nmax = max(nmax, __shfl_xor_sync(SPH_FULL, nmax, s));
   NbrIter it;
   it.init(d, is);
-  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], lane, i, n, nmax, p, pp, cv, o};
+  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], &slots[DIM == 3 || WIDE ? w : 0][0][0], lane, i, n, nmax, p, pp, cv, o};
   auto walk = [&](auto wrap_tag) {
     if constexpr (WIDE)
       pair_walk_wide<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
