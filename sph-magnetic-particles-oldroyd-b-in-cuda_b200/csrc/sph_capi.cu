@@ -154,7 +154,9 @@ bool alloc_lists(sph_ctx* c, int cap) {
     *ptr = static_cast<T*>(q);
     return true;
   };
-  if (!replace(&d.nchunk, (size_t)cap * d.Npad)) return false;
+  // one row more than a particle can store: the consumers read an entry ahead (NbrIter)
+  if (!replace(&d.nchunk, ((size_t)cap + 1) * d.Npad)) return false;
+  cudaMemsetAsync(d.nbr_cnt, 0, d.Npad * sizeof(int), c->stream);  // no entries yet
   d.cap = cap;
   return true;
 }
@@ -726,7 +728,7 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
     ok = ok && dalloc(c, &r, Np);
     d.rec = r;
   }
-  ok = ok && dalloc(c, &d.nbr_cnt, Np) && dalloc(c, &d.nbr_nch, Np);
+  ok = ok && dalloc(c, &d.nbr_cnt, Np);
   ok = ok && dalloc(c, &d.keys, Np) && dalloc(c, &d.vals, Np);
   ok = ok && dalloc(c, &d.moved, Np) && dalloc(c, &d.bucket, Np);
   ok = ok && dalloc(c, &d.cell_count, Ctot + 1) && dalloc(c, &d.scan_sums, Ctot / 4096 + 2);
@@ -1123,7 +1125,10 @@ sph_status sph_synchronize(sph_ctx* c) {
     int used = 0;
     cudaMemcpy(&used, c->d.err_info + kErrMaxCount, sizeof(int), cudaMemcpyDeviceToHost);
     // keep headroom: grow the lists (and recapture) once 90% of the capacity is in use
-    if (used > (9 * c->d.cap) / 10) s = grow_capacity(c, used);
+    if (used > (9 * c->d.cap) / 10) {
+      s = grow_capacity(c, used);
+      c->pos_dirty = true;  // the new lists are empty: the next reader searches again
+    }
   }
   return s;
 }

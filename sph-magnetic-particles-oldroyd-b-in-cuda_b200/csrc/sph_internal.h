@@ -192,9 +192,8 @@ struct Dev {
   void* rec;     // RecD or RecF per slot
   // neighbour candidates (k_build_lists): per particle, for every chunk of up to 32
   // consecutive candidate slots in which it has a hit, (first slot, hit mask), chunk-major
-  int2* nchunk;     // cap x Npad: nchunk[k * Npad + i]
-  int* nbr_nch;     // per slot: chunks stored
-  int* nbr_cnt;     // per slot: candidates (set bits over the particle's chunks)
+  int2* nchunk;     // (cap + 1) x Npad: nchunk[k * Npad + i]
+  int* nbr_cnt;     // per slot: candidates (set bits over the particle's chunks; 0: too many chunks)
   int* keys;     // sorted keys (global cell of each slot)
   int* vals;     // sorted values (global ids)
   int* cell_count;  // Ctot + 1: particles counted per cell by the hash; zero between searches

@@ -52,3 +52,27 @@ def test_densities_of_uneven_cells(workdir, dim, N, overlap, wall, tpc):
     assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
     e.close()
     o.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_lists_without_a_spare_entry_and_lists_just_grown(workdir, precision):
+    """A capacity of exactly the entries in use gives the same bits as a larger one; grown for
+    headroom by synchronize(), the emptied lists are built again before they are read."""
+    p = sph_input.write_input(os.path.join(workdir, "input"), N=(24, 20, 28),
+                              L=(24 / 28.0, 20 / 28.0, 1.0), dim=3, overlap=3.0, dt=1e-5)
+    wide = sph_b200.System(p, precision=precision)
+    wide.neighbours_search()
+    wide.calculate_density()
+    used = wide.neighbour_lists()["max_used"]
+    tight = sph_b200.System(p, precision=precision, nbr_capacity=used)
+    tight.neighbours_search()
+    tight.calculate_density()
+    want = wide.field("dens")
+    assert np.array_equal(tight.field("dens"), want)
+    tight.synchronize()
+    lists = tight.neighbour_lists()
+    assert lists["grown"] == 1 and lists["capacity"] > used
+    tight.calculate_density()
+    assert np.array_equal(tight.field("dens"), want)
+    wide.close()
+    tight.close()
