@@ -676,15 +676,22 @@ __device__ __forceinline__ int list_odd_particle(const Dev& d, int ti, int tb) {
 // Candidates further off (minimum-image placement) only have to be outside: held within 200 rcut,
 // and n below what a float16 holds.
 //
-// What bounds it: instruction issue.  The packed float test (k_build_lists_half), whose operands
-// and subtractions each lane repeats for every candidate, took most of a chunk's instructions;
-// with the matrix product they are staging (FP64 positions to four words), eight matrix
-// instructions and the exchange of the masks.  A row of three neighbour cells is one range of
-// slots, since their particles follow one another in memory, so chunks are nearly full: cells of
-// 16 particles took 9 chunks, their rows take 6, and the consumers' lists are shorter as well.
-// Measured (ms; packed float test cell by cell / matrix product cell by cell / by rows): 128^3
-// 0.857 / 0.641 / 0.591, 96^3 with colloids 0.346 / 0.265 / 0.255, 61 x 53 x 67 0.129 / 0.099 / 0.094, 512 2D boxes 0.657 / 0.683 / 0.617, one 64^2
-// box 0.0140 / 0.0127 / 0.0119; the 128^3 step's pair pass went from 2.77 to 2.70 with the shorter lists.
+// What bounds it: instruction issue (67 % at 96^3).  The packed float test (k_build_lists_half),
+// whose operands and subtractions each lane repeats for every candidate, took most of a chunk's
+// instructions; with the matrix product about 110 are left, for staging (FP64 positions to four
+// words), eight matrix instructions and the masks, and as many as 15 chunks take for a cell's
+// ranges and rows.  A row of three neighbour cells is one range of slots, since their particles
+// follow one another in memory, so chunks are nearly full: cells of 16 particles took 9 chunks,
+// their rows take 6, and the consumers' lists are shorter as well.
+// Sign bits are shifted into one byte per row and lane, and two exchanges with byte selections
+// turn a quad's bytes into its rows' masks; candidates are staged in the columns that make their
+// order come out right.  The largest chunk count goes to memory only where it is larger than the
+// one there: an atomic from every cell's warp was what the 2D grids waited for.
+// Measured (ms; packed float test cell by cell / matrix product cell by cell / by rows / and with
+// the byte masks and the filtered count): 128^3 0.857 / 0.641 / 0.599 / 0.564, 96^3 with colloids
+// 0.346 / 0.265 / 0.258 / 0.244, 61 x 53 x 67 0.129 / 0.099 / 0.097 / 0.089, 512 2D boxes 0.657 /
+// 0.683 / 0.616 / 0.447, one 64^2 box 0.0140 / 0.0127 / 0.0119 / 0.0113.  64 rows a round, for
+// cells of more than 32, were slower (128^3 0.577 -> 0.629: registers).
 __device__ __forceinline__ unsigned pack_h2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const unsigned*>(&h);
@@ -692,35 +699,40 @@ __device__ __forceinline__ unsigned pack_h2(float lo, float hi) {
 __device__ __forceinline__ float2 unpack_h2(unsigned u) {
   return __half22float2(*reinterpret_cast<const __half2*>(&u));
 }
-__device__ __forceinline__ void mma_16x8x16(unsigned (&d)[4], const unsigned (&a)[4], unsigned b,
-                                            float c01, float c23) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%8}, "
-      "{%9,%9,%10,%10};\n"
+// B's two registers hold the same word, C's four two start values; they are passed one by one,
+// from loads and shuffles of their own, because the instruction takes them from neighbouring
+// registers and equal ones would be copied there before each.
+__device__ __forceinline__ void mma_16x8x16(unsigned (&d)[4], const unsigned (&a)[4], unsigned b0,
+                                            unsigned b1, const float (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%11,%12,%13};\n"
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b), "f"(c01), "f"(c23));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]),
+        "f"(c[2]), "f"(c[3]));
 }
-// The sign bits of two rows (g and g + 8 of the tile of 16) against TILES tiles of 8 candidates:
-// the lane's candidates 8 u + 2 t and + 1 in bits 31 - 8 u and 30 - 8 u.
+__device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], unsigned at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(at)
+               : "memory");
+}
+// The sign bits of a lane's accumulators against TILES tiles of 8 candidates, one byte (two tiles:
+// nibble) for each of its two rows, g in the upper one: columns 2 t and 2 t + 1 of tile 0 first.
 template <int TILES>
-__device__ __forceinline__ void hit_bits(const unsigned (&a)[4], const unsigned (&b)[4], float c01,
-                                         float c23, unsigned& m0, unsigned& m1) {
-  unsigned d[4][4];
+__device__ __forceinline__ unsigned hit_bits(const unsigned (&a)[4], const unsigned (&b)[8],
+                                             const float (&c)[4]) {
+  unsigned d[TILES][4];
 #pragma unroll
-  for (int u = 0; u < TILES; ++u) mma_16x8x16(d[u], a, b[u], c01, c23);
-  unsigned top[4];  // the top bytes of the four tiles' accumulators q, tile 0's first
+  for (int u = 0; u < TILES; ++u) mma_16x8x16(d[u], a, b[2 * u], b[2 * u + 1], c);
+  unsigned m[2] = {0u, 0u};
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const unsigned hi = __byte_perm(d[1][q], d[0][q], 0x7377);  // bytes 3, 2: tiles 0, 1
-    if (TILES == 4) {
-      const unsigned lo = __byte_perm(d[3][q], d[2][q], 0x7773);  // bytes 1, 0 (read below)
-      top[q] = __byte_perm(lo, hi, 0x7610);
-    } else {
-      top[q] = hi;
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int u = 0; u < TILES; ++u) {
+      m[h] = __funnelshift_l(d[u][2 * h], m[h], 1);
+      m[h] = __funnelshift_l(d[u][2 * h + 1], m[h], 1);
     }
-  }
-  constexpr unsigned kKeep = TILES == 4 ? 0x80808080u : 0x80800000u;
-  m0 = (top[0] & kKeep) | ((top[1] & kKeep) >> 1);
-  m1 = (top[2] & kKeep) | ((top[3] & kKeep) >> 1);
+  return m[0] << 8 | m[1];
 }
 // The four words of a candidate at (x, y, z); keep: it exists.
 __device__ __forceinline__ uint4 candidate_words(float x, float y, float z, bool keep) {
@@ -737,12 +749,14 @@ __device__ __forceinline__ uint4 candidate_words(float x, float y, float z, bool
 }
 
 template <int DIM>
-// Blocks per SM the registers are held to, measured (ms, 7 / 8 / 9): 128^3 0.604 / 0.599 / 0.615,
-// 512 2D boxes 0.611 / 0.616 / 0.623.
-__global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
+// Blocks per SM the registers are held to, measured (ms, 6 / 7 / 8): 128^3 0.596 / 0.574 / 0.564,
+// 512 2D boxes 0.512 / 0.473 / 0.447.
+__global__ void __launch_bounds__(kListWarps * 32, 8)
     k_build_lists(Dev d, int split) {
   constexpr int kNZ = DIM == 3 ? 3 : 1;
-  __shared__ uint4 stage[kListWarps][32];  // the chunk's candidates, a row of 16 bytes each
+  // the chunk's candidates, 16 bytes each, tiles of 8 rows two rows apart (a round of stores then
+  // meets no bank twice)
+  __shared__ uint4 stage[kListWarps][40];
   __shared__ float frame[kListWarps][9];   // lo[3], hi[3], L[3] (frame_offset)
   // the candidates as ranges of consecutive slots (a row of three neighbour cells is one, or two
   // at the periodic wrap), and what takes their positions to offsets from this cell's centre
@@ -764,7 +778,8 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
   const BoxParams& p = d.box[b];
   const int N0 = p.Ncells[0], N1 = p.Ncells[1], N2 = p.Ncells[2];
   const int lc = cell - p.cell0;
-  const int cx = lc % N0, cy = (lc / N0) % N1, cz = DIM == 3 ? lc / (N0 * N1) : 0;
+  const int row = lc / N0, cx = lc - row * N0;
+  const int cz = DIM == 3 ? row / N1 : 0, cy = row - cz * N1;
   const int beg = d.cell_begin[cell], end = d.cell_begin[cell + 1];
   const double ox = cx * p.cell_size[0];
   const double oy = cy * p.cell_size[1] - (p.wall ? p.wall_width : 0.0);
@@ -773,6 +788,10 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
   const double mx = ox + 0.5 * p.cell_size[0], my = oy + 0.5 * p.cell_size[1];
   const double mz = DIM == 3 ? oz + 0.5 * p.cell_size[2] : 0.0;
   const float inv = (float)p.rcut_inv;
+  // offsets up to these are inside the cell whatever the rounding of its bounds
+  constexpr float kIn = 0.5f - 1e-5f;
+  const float inx = kIn * (float)p.cell_size[0] * inv, iny = kIn * (float)p.cell_size[1] * inv;
+  const float inz = kIn * (float)p.cell_size[2] * inv;
   const float cut2 = (float)(p.list_cut2 * p.rcut_inv * p.rcut_inv);
   const int cap = d.cap;  // chunks with hits a particle can store
   const size_t Np = d.Npad;
@@ -830,7 +849,17 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
   const float* fhi = flo + 3;
   const float* fL = flo + 6;
   const int g = lane >> 2, t = lane & 3;  // this lane's part of the fragments
-  const unsigned srow = (unsigned)__cvta_generic_to_shared(&stage[w][lane]);
+  // Candidate k of a chunk is staged in the column whose sign bits end up in bit 31 - k of the
+  // masks: column 2 t + c of tile u for k = 8 t + 2 u + c, in chunks of at most 16 (two tiles)
+  // k = 4 t + 2 u + c.
+  const int col_long = 10 * ((lane >> 1) & 3) + 2 * (lane >> 3) + (lane & 1);
+  const int col_short =
+      lane < 16 ? 10 * ((lane >> 1) & 1) + 2 * (lane >> 2) + (lane & 1) : 20 + (lane & 15);
+  // each tile's rows twice, for the two words of B
+  const unsigned srow =
+      (unsigned)__cvta_generic_to_shared(&stage[w][10 * (lane >> 4) + (lane & 7)]);
+  // byte selectors of the quad's 4 x 4 transposition
+  const unsigned sel1 = (t & 1) ? 0x6240u : 0x3715u, sel2 = (t & 2) ? 0x5410u : 0x3276u;
   // the particle loop, in the cheap form (per-cell shifts) or the minimum-image one
   auto walk = [&](auto mi_tag) {
     constexpr bool kMI = decltype(mi_tag)::value;
@@ -847,7 +876,9 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
         yi = (float)(x.y - my) * inv;
         zi = DIM == 3 ? (float)(x.z - mz) * inv : 0.f;
         int ax = 0, ay = 0, az = 0;
-        if (own_cell(p, x.x, x.y, x.z, ax, ay, az)) {
+        if (fabsf(xi) < inx && fabsf(yi) < iny && (DIM == 2 || fabsf(zi) < inz)) {
+          // inside its sort cell, without own_cell's divisions
+        } else if (own_cell(p, x.x, x.y, x.z, ax, ay, az)) {
           odd = (ax != cx) || (ay != cy) || (DIM == 3 && az != cz);
         } else {
           // not finite or far outside the box: already reported by the hash; no neighbours
@@ -867,7 +898,7 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
       const float start = listed ? fmaf(zi, zi, fmaf(yi, yi, xi * xi)) - cut2 : 1.0f;
       // fragments: word t (of the four) of rows g, g + 8 and of rows g + 16, g + 24
       unsigned fa[2][4];
-      float fc[4];
+      float fc[2][4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int from = 4 * g + q;  // the lane that holds row g + 8 q
@@ -875,7 +906,8 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
         const unsigned b0 = __shfl_sync(SPH_FULL, up0, from), b1 = __shfl_sync(SPH_FULL, up1, from);
         fa[q >> 1][q & 1] = (t & 1) ? a1 : a0;
         fa[q >> 1][2 + (q & 1)] = (t & 1) ? b1 : b0;
-        fc[q] = __shfl_sync(SPH_FULL, start, from);
+        fc[q >> 1][2 * (q & 1)] = __shfl_sync(SPH_FULL, start, from);
+        fc[q >> 1][2 * (q & 1) + 1] = __shfl_sync(SPH_FULL, start, from);
       }
       const bool two = span - t0 > 16;             // rows 16 .. 31 are in use
       int2* col = d.nchunk + (listed ? i : 0);     // this particle's chunks, stride Npad
@@ -907,31 +939,30 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
             vy = fminf(fmaxf(vy, -200.f), 200.f);
             vz = fminf(fmaxf(vz, -200.f), 200.f);
           }
-          stage[w][lane] = candidate_words(vx, vy, vz, j <= ce);
+          const bool wide = ce - c0 >= 16;
+          stage[w][wide ? col_long : col_short] = candidate_words(vx, vy, vz, j <= ce);
           __syncwarp();
-          unsigned fb[4];  // word t of candidates 8 u + g, u = 0 .. 3
-          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                       : "=r"(fb[0]), "=r"(fb[1]), "=r"(fb[2]), "=r"(fb[3])
-                       : "r"(srow)
-                       : "memory");
-          __syncwarp();  // the stage is refilled by the next chunk
-          // hits of rows g + 8 r
-          unsigned m[4] = {0u, 0u, 0u, 0u};
-          if (ce - c0 >= 16) {
-            hit_bits<4>(fa[0], fb, fc[0], fc[1], m[0], m[1]);
-            if (two) hit_bits<4>(fa[1], fb, fc[2], fc[3], m[2], m[3]);
+          unsigned fb[8];  // word t of candidate g of tile u in fb[2 u] and fb[2 u + 1]
+          ldmatrix_x4(*reinterpret_cast<unsigned(*)[4]>(&fb[0]), srow);
+          // rows g and g + 8 in bytes 3 and 2, g + 16 and g + 24 in bytes 1 and 0
+          unsigned m;
+          if (wide) {
+            ldmatrix_x4(*reinterpret_cast<unsigned(*)[4]>(&fb[4]), srow + 20 * 16);
+            __syncwarp();  // the stage is refilled by the next chunk
+            m = hit_bits<4>(fa[0], fb, fc[0]) << 16;
+            if (two) m |= hit_bits<4>(fa[1], fb, fc[1]);
           } else {
-            hit_bits<2>(fa[0], fb, fc[0], fc[1], m[0], m[1]);
-            if (two) hit_bits<2>(fa[1], fb, fc[2], fc[3], m[2], m[3]);
+            __syncwarp();
+            m = hit_bits<2>(fa[0], fb, fc[0]) << 16;
+            if (two) m |= hit_bits<2>(fa[1], fb, fc[1]);
           }
-#pragma unroll
-          for (int r = 0; r < 4; ++r) m[r] >>= 2 * t;
-          // the quad's parts of rows g + 8 r to the lane that holds the row (t = r): bit 31 - k of
-          // `hits` is then candidate k, the consumers' order of leading zeros
-          const bool o1 = (t & 1) != 0, o2 = (t & 2) != 0;
-          const unsigned p0 = (o1 ? m[1] : m[0]) | __shfl_xor_sync(SPH_FULL, o1 ? m[0] : m[1], 1);
-          const unsigned p1 = (o1 ? m[3] : m[2]) | __shfl_xor_sync(SPH_FULL, o1 ? m[2] : m[3], 1);
-          const unsigned hits = (o2 ? p1 : p0) | __shfl_xor_sync(SPH_FULL, o2 ? p0 : p1, 2);
+          // the quad's bytes of row g + 8 r to the lane that holds the row (t = r), t = 0 first: bit
+          // 31 - k of `hits` is then candidate k, the consumers' order of leading zeros
+          m = __byte_perm(m, __shfl_xor_sync(SPH_FULL, m, 1), sel1);
+          unsigned hits = __byte_perm(m, __shfl_xor_sync(SPH_FULL, m, 2), sel2);
+          if (!wide) {  // nibbles: together, and to the top
+            hits = __byte_perm(hits << 4 | hits << 8, 0u, 0x3144u);
+          }
           if (hits != 0u) {  // a chunk with hits: (first slot, mask) in the next entry
             if (kc < cap) col[(size_t)kc * Np] = make_int2(c0, (int)hits);
             cnt += __popc(hits);
@@ -956,10 +987,10 @@ __global__ void __launch_bounds__(kListWarps * 32, DIM == 3 ? 8 : 7)
   else
     walk(std::false_type{});
   // warp max of the chunk counts -> capacity check
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) maxch = max(maxch, __shfl_xor_sync(SPH_FULL, maxch, o));
-  if (lane == 0 && maxch > 0) {
-    atomicMax(&d.err_info[kErrMaxCount], maxch);
+  maxch = __reduce_max_sync(SPH_FULL, maxch);
+  if (lane == 0) {
+    if (maxch > *(volatile const int*)(d.err_info + kErrMaxCount))
+      atomicMax(&d.err_info[kErrMaxCount], maxch);
     if (maxch > cap) raise_status(d, kStatCapacity, 0, kPhaseLists);
   }
 }
@@ -1153,7 +1184,8 @@ __global__ void __launch_bounds__(kListWarps * 32) k_build_lists_half(Dev d, int
   // warp max of the chunk counts -> capacity check
   maxch = warp_max(maxch);
   if (lane == 0 && maxch > 0) {
-    atomicMax(&d.err_info[kErrMaxCount], maxch);
+    if (maxch > *(volatile const int*)(d.err_info + kErrMaxCount))
+      atomicMax(&d.err_info[kErrMaxCount], maxch);
     if (maxch > cap) raise_status(d, kStatCapacity, 0, kPhaseLists);
   }
 }
