@@ -45,6 +45,7 @@ struct sph_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool events_recorded = false;  // ev0/ev1 bracket the last sph_step
   double last_ms = 0.0;
+  int max_coll_particles = 0;  // of the largest colloid
   int max_coll = 0;
   int cap_grown = 0;
   // the last sph_step call, for resuming it after a full neighbour list was found in one of
@@ -104,6 +105,7 @@ Launch launcher(sph_ctx* c) {
   L.nsm = c->nsm;
   L.list_tpc = c->tune.list_threads_per_cell;
   L.density_block = c->tune.density_block;
+  L.coll_particles = c->max_coll_particles;
   return L;
 }
 
@@ -836,6 +838,7 @@ sph_status sph_create_ensemble(int nboxes, const sph_input* inputs,
         xc[2 * (size_t)std::max(nlist, 1) + e] = hb.z_center[q];
       }
       cseg.push_back((int)cl.size());
+      c->max_coll_particles = std::max(c->max_coll_particles, k1 - k0);
       cbox.push_back(b);
       cs[CS_X * ncoll + gc] = hb.coll_x[k];
       cs[CS_Y * ncoll + gc] = hb.coll_y[k];

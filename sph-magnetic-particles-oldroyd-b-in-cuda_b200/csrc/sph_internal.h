@@ -258,6 +258,7 @@ struct Launch {
   long long* launches;
   int list_tpc = 32;        // threads per cell of the list build (32 or 16)
   int nsm = 148;            // multiprocessors of the device
+  int coll_particles = 0;   // of the largest colloid
   int density_block = 128;  // density pass: 0 = neighbour-cell tiles, else threads per block
   // (launch geometry only: results do not depend on it)
 };

@@ -1911,12 +1911,12 @@ __global__ void k_dcdt(Dev d) {
 // ---------------------------------------------------------------------------------
 constexpr int kRedThreads = 256;
 
-template <int NV>
-__device__ __forceinline__ void block_reduce(double (&v)[NV], double (*sh)[kRedThreads]) {
+template <int NV, int NT>
+__device__ __forceinline__ void block_reduce(double (&v)[NV], double (*sh)[NT]) {
 #pragma unroll
   for (int q = 0; q < NV; ++q) sh[q][threadIdx.x] = v[q];
   __syncthreads();
-  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
+  for (int s = NT / 2; s > 0; s >>= 1) {
     if ((int)threadIdx.x < s)
 #pragma unroll
       for (int q = 0; q < NV; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + s];
@@ -2100,10 +2100,12 @@ __device__ __forceinline__ void colloid_pairs(const Dev& d, const BoxParams& p, 
 }
 
 // One block per colloid.  PAIRS: then its repulsion and magnetic forces (first warp).  KICK: then
-// its second half-kick (kernel_move_colloids_VV_part2.cu:14-46).
-template <bool PAIRS, bool KICK>
-__global__ void __launch_bounds__(kRedThreads) k_collect_colloids(Dev d) {
-  __shared__ double sh[6][kRedThreads];
+// its second half-kick (kernel_move_colloids_VV_part2.cu:14-46).  NT threads, no fewer than any
+// colloid has particles or 256: the sums are then the same (the further threads of a larger block
+// would add zeros).
+template <bool PAIRS, bool KICK, int NT>
+__global__ void __launch_bounds__(NT) k_collect_colloids(Dev d) {
+  __shared__ double sh[6][NT];
   const int c = blockIdx.x;
   if (c >= d.ncoll) return;
   if (step_aborted(d)) return;
@@ -2112,7 +2114,7 @@ __global__ void __launch_bounds__(kRedThreads) k_collect_colloids(Dev d) {
   const double cx = d.cs[CS_X * nc + c], cy = d.cs[CS_Y * nc + c], cz = d.cs[CS_Z * nc + c];
   const int j0 = d.coll_seg[c], j1 = d.coll_seg[c + 1];
   double v[6] = {0, 0, 0, 0, 0, 0};  // F x y z, T x y z
-  for (int j = j0 + threadIdx.x; j < j1; j += kRedThreads) {
+  for (int j = j0 + threadIdx.x; j < j1; j += NT) {
     const int s = d.inv[d.colloids_list[j]];
     const double4 x = d.pos[s];
     const double fx = d.f[s], fy = d.f[Np + s], fz = p.dim == 3 ? d.f[2 * Np + s] : 0.0;
@@ -2566,12 +2568,24 @@ int launch_wall_forces(const Launch& L) {
   return check(L);
 }
 
+template <int NT>
+static void collect_colloids_launch(const Launch& L, int with_pairs, int kick) {
+  const int nb = L.d.ncoll;
+  if (with_pairs && kick) k_collect_colloids<true, true, NT><<<nb, NT, 0, S(L)>>>(L.d);
+  else if (with_pairs) k_collect_colloids<true, false, NT><<<nb, NT, 0, S(L)>>>(L.d);
+  else if (kick) k_collect_colloids<false, true, NT><<<nb, NT, 0, S(L)>>>(L.d);
+  else k_collect_colloids<false, false, NT><<<nb, NT, 0, S(L)>>>(L.d);
+}
+
 int launch_colloid_forces(const Launch& L, int with_pairs, int kick) {
   if (L.d.ncoll == 0) return 0;
-  if (with_pairs && kick) k_collect_colloids<true, true><<<L.d.ncoll, kRedThreads, 0, S(L)>>>(L.d);
-  else if (with_pairs) k_collect_colloids<true, false><<<L.d.ncoll, kRedThreads, 0, S(L)>>>(L.d);
-  else if (kick) k_collect_colloids<false, true><<<L.d.ncoll, kRedThreads, 0, S(L)>>>(L.d);
-  else k_collect_colloids<false, false><<<L.d.ncoll, kRedThreads, 0, S(L)>>>(L.d);
+  // The smallest block that gives every particle of the largest colloid its own thread: ensembles
+  // of small colloids are many blocks that each wait on a chain of loads and on the first warp's
+  // pair forces, and more of them fit an SM (12,288 colloids of up to 64 particles: 0.086 ms with
+  // 256 threads, 0.038 with 64).
+  if (L.coll_particles <= 64) collect_colloids_launch<64>(L, with_pairs, kick);
+  else if (L.coll_particles <= 128) collect_colloids_launch<128>(L, with_pairs, kick);
+  else collect_colloids_launch<kRedThreads>(L, with_pairs, kick);
   return check(L);
 }
 

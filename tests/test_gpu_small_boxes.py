@@ -53,3 +53,32 @@ def test_a_box_alone_and_among_many_gives_the_same_bits(workdir, name, copies, p
         assert np.array_equal(a, b[:n]) and np.array_equal(a, b[-n:]), q
     alone.close()
     many.close()
+
+
+def test_colloids_alone_and_beside_larger_ones_give_the_same_bits(workdir):
+    """The colloid pass takes as many threads a block as the largest colloid of the context has
+    particles, up to 256: about 28, 79 and 201 particles (64, 128 and 256 threads)."""
+    paths, alone = [], []
+    for k, R in enumerate((3.0, 5.0, 8.0)):
+        spec = dict(N=(96, 80), L=(1.2, 1.0), dim=2, overlap=3.0, dt=2e-5, N_colloids=2,
+                    coll_R=R / 80, coll_x=((0.3, 0.31), (0.8, 0.6)), coll_repulsion_cuton=0.2 / 80,
+                    F0_repulsion=1e-3, tau_repulsion=10.0, cutoff_magnetic=8.0 / 80,
+                    F0_magnetic=1e-4, omega_magnetic=6.28)
+        paths.append(sph_input.write_input(os.path.join(workdir, "input%d" % k), **spec))
+
+    def run(some):
+        s = sph_b200.System(some)
+        x, y, fluid = s.field("x"), s.field("y"), s.type() == 0
+        s.set_field("vx", np.where(fluid, 0.5 * np.sin(9.0 * x + 14.0 * y), 0.0))
+        s.set_field("vy", np.where(fluid, 0.5 * np.cos(11.0 * x - 8.0 * y), 0.0))
+        s.initial_forces()
+        s.step(3)
+        s.synchronize()
+        out = [s.colloid_field(q) for q in ("fx_colloid", "fy_colloid", "tz_colloid", "coll_x",
+                                            "coll_vx", "coll_omegaz")]
+        s.close()
+        return np.stack(out)
+
+    for n in (1, 2, 3):
+        alone.append(run(paths[n - 1:n]))
+        assert np.array_equal(run(paths[:n]), np.concatenate(alone, axis=1))
