@@ -1474,22 +1474,21 @@ __global__ void k_pressure(Dev d) {
 // while the current ones are evaluated.  Each lane then reads its records
 // from shared memory (row stride padded by one piece: conflict-free).
 //
-// What bounds the 3D FP64 pass is the load/store pipe all of this goes through (79 % busy at 96^3,
-// the FP64 pipe 34 %, issue 49 %): per position of a warp 32 passes for the copies, 32 for the
-// records and one for each shuffle or slot.  There the slots go through shared memory, three
-// passes in place of eight shuffles, and records are read 16 bytes at a time: 128^3 pair pass
-// 2.70 -> 2.51 ms FP64, 2.12 -> 2.06 mixed.  In 2D, with 64- and 32-byte records, the same slots
-// cost more than the four or two shuffles (512 boxes 2.58 -> 2.76 ms FP64, 1.87 -> 1.91 mixed),
-// except in the wide walk (one 64^2 box 28.6 -> 26.6 us).
+// What bounds the FP64 passes is the load/store pipe all of this goes through (3D: 79 % busy at
+// 96^3, the FP64 pipe 34 %, issue 49 %): per position of a warp 32 passes for the copies of a 3D
+// record, 32 to read it and one for each shuffle or slot.  The slots go through shared memory,
+// three passes in place of eight shuffles, and records are read 16 bytes at a time: 128^3 pair
+// pass 2.70 -> 2.51 ms FP64, 2.12 -> 2.06 mixed; 512 2D boxes, FP64, 2.26 -> 2.17.  With the 32-byte
+// float 2D records the slots cost more than two shuffles (512 boxes 1.87 -> 1.91 ms).
 //
 // Launch shape of the pair pass per precision and dimension, as measured on B200.  Every pass
 // evaluates one list position per step: with the fluid-fluid form of that walk, evaluating two
 // positions side by side (to overlap their dependency chains) measured slower everywhere
 // (float 3D at 128^3 2.41 vs 2.38 ms, FP64 2D on the 512-box ensemble 3.63 vs 3.52 ms).
-//  - kWarps: warps per block; kMinBlocks: resident blocks per SM the register allocation
-//    is held to (FP64 3D: 168 registers, which its working set fits without spilling;
-//    float 3D 128; FP64 2D 96, with a few spills: 5 blocks 3.52 ms, 4 blocks 3.58 ms; the
-//    float 2D pass 80, in 2-warp blocks).
+//  - kWarps: warps per block; kMinBlocks: resident blocks per SM the register allocation is held
+//    to.  512 boxes, FP64 2D: 3 / 4 / 5 / 6 blocks 2.29 / 2.26 / 2.47 / 2.90 ms (spills from 5 on).
+//    128^3 float 3D: 3 / 4 / 5 blocks 1.994 / 2.004 / 2.037 ms; FP64 3D: 3 (168 registers).  Float
+//    2D: 2-warp blocks, 5 to 8 the same.
 //  - One-box 3D contexts (k_pairs<..., ONE = true>) read the pair constants from the
 //    constant bank (Dev::pc) instead of registers: 128^3 pair pass 3.59 -> 3.55 ms (FP64)
 //    and 2.43 -> 2.38 ms (mixed) at the same shape.  The FP64 3D pass then fits 128
@@ -1501,11 +1500,10 @@ struct PairShape {
   using Rec = typename RecFor<T, DIM>::type;
   static constexpr bool kF64 = sizeof(T) == 8;
   static constexpr bool kF2D = !kF64 && DIM == 2;
-  static constexpr bool kF64_3D = kF64 && DIM == 3;
   // the float 2D pass runs 2-warp blocks (measured 2.29 vs 2.35 ms on the 512-box ensemble;
   // the float 3D pass was slower with them, the FP64 passes unchanged)
   static constexpr int kWarps = WIDE ? 1 : kF2D ? 2 : 4;
-  static constexpr int kMinBlocks = WIDE ? 1 : kF2D ? 6 : (kF64_3D ? 3 : (kF64 ? 5 : 4));
+  static constexpr int kMinBlocks = WIDE ? 1 : kF2D ? 6 : kF64 && DIM == 2 ? 4 : 3;
 };
 
 // The pair constants of a one-box context, viewed as PairParams (same layout).
@@ -1595,17 +1593,11 @@ __device__ __forceinline__ void stage_records(int4* buf, const Rec* __restrict__
   }
 }
 
-// A lane's view of one staged record.  FP64 2D records are read in place, each field loaded from
-// shared memory where the pair term uses it, which keeps them out of the register file; float
-// records are copied into registers, and so are the FP64 3D ones, 16 bytes a load: the fields
-// read one by one took 11 loads, the 8-byte ones among them with two-way bank conflicts (128^3
-// pair pass 2.59 -> 2.56 ms).
+// A staged record in a lane's registers, read 16 bytes a load.  FP64: field by field the 3D record
+// took 11 loads, the 8-byte ones among them with two-way bank conflicts (pair pass 2.59 -> 2.56 ms
+// at 128^3, 2.22 -> 2.17 on the 512 2D boxes).
 template <typename T, typename Rec>
-struct StagedRec {
-  const Rec& r;
-  __device__ __forceinline__ explicit StagedRec(const int4* src)
-      : r(*reinterpret_cast<const Rec*>(src)) {}
-};
+struct StagedRec;
 template <>
 struct StagedRec<double, RecD> {
   RecD r;
@@ -1627,6 +1619,22 @@ struct StagedRec<double, RecD> {
     r.P[5] = g.y;
     r.invd = __hiloint2double(h.y, h.x);
     r.tinfo = h.z;
+  }
+};
+template <>
+struct StagedRec<double, RecD2> {
+  RecD2 r;
+  __device__ __forceinline__ explicit StagedRec(const int4* src) {
+    const double2* q = reinterpret_cast<const double2*>(src);
+    const double2 a = q[0], b = q[1], c = q[2], e = q[3];
+    r.x = a.x;
+    r.y = a.y;
+    r.vx = b.x;
+    r.vy = b.y;
+    r.P[0] = c.x;
+    r.P[1] = c.y;
+    r.P[2] = e.x;
+    r.invd = e.y;
   }
 };
 template <typename Rec>
@@ -1655,6 +1663,10 @@ struct PairWalk {
   const PairOwn<T, DIM>& o;
 };
 
+// Passes whose slots go through shared memory (see stage_records): all but the float 2D one.
+template <typename T, int DIM>
+constexpr bool kSlots = DIM == 3 || sizeof(T) == 8;
+
 // A lane's walk over its list, one position per step: the copies for position k + 1 are in
 // flight while k is evaluated.  WRAP: see min_image.
 template <typename T, int DIM, bool WRAP, int MODE>
@@ -1662,7 +1674,7 @@ __device__ __forceinline__ void pair_walk(const PairWalk<T, DIM>& W, NbrIter& it
                                            PairAcc<T, DIM>& acc) {
   using Rec = typename RecFor<T, DIM>::type;
   using St = PairStage<Rec>;
-  constexpr bool kIdx = DIM == 3;  // slots by way of shared memory, two positions ahead
+  constexpr bool kIdx = kSlots<T, DIM>;  // slots by way of shared memory, two positions ahead
   const int n = W.n, lane = W.lane;
   int jc = n > 0 ? it.next() : -1, jn = -1, j2 = -1;
   // 2D records carry no type word: the neighbour's is read from the type array one
@@ -1778,7 +1790,7 @@ __global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
   using St = PairStage<Rec>;
   // per warp: a double buffer of staged positions
   __shared__ int4 stage[Sh::kWarps][WIDE ? 4 : 2][St::kRows];
-  __shared__ __align__(16) int slots[DIM == 3 || WIDE ? Sh::kWarps : 1][WIDE ? 4 : 2][32];
+  __shared__ __align__(16) int slots[kSlots<T, DIM> || WIDE ? Sh::kWarps : 1][WIDE ? 4 : 2][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wbase = (blockIdx.x * Sh::kWarps + w) * 32;
   if (wbase >= d.Ntot) return;  // whole warps only: the lanes below cooperate
@@ -1807,7 +1819,7 @@ __global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
   for (int s = 16; s > 0; s >>= 1) nmax = max(nmax, __shfl_xor_sync(SPH_FULL, nmax, s));
   NbrIter it;
   it.init(d, is);
-  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], &slots[DIM == 3 || WIDE ? w : 0][0][0], lane, i, n, nmax, p, pp, cv, o};
+  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], &slots[kSlots<T, DIM> || WIDE ? w : 0][0][0], lane, i, n, nmax, p, pp, cv, o};
   auto walk = [&](auto wrap_tag) {
     if constexpr (WIDE)
       pair_walk_wide<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
