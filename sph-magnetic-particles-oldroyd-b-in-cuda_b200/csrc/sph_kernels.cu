@@ -1530,10 +1530,10 @@ struct PairStage {
   };
 };
 
-// L1: the copy allocates in L1 (.ca) or goes through L2 only (.cg).  The 3D records are
-// staged through L1 (reused by the neighbouring warps of the SM), the 2D records (64 and 32
-// bytes) through L2 only: measured 3.74 vs 3.78 ms (FP64 3D), 2.33 vs 2.44 ms (float 3D),
-// 3.28 vs 3.33 ms (FP64 2D ensemble) and 2.28 vs 2.29 ms (float 2D ensemble).
+// L1: the copy allocates in L1 (.ca) or goes through L2 only (.cg).  Records are staged through
+// L1, where the neighbouring warps of the SM find them again, except the 32-byte float 2D ones:
+// measured, L1 / L2 only, 3.74 / 3.78 ms (FP64 3D), 2.33 / 2.44 (float 3D), 2.14 / 2.17 (FP64 2D,
+// 512 boxes) and 2.29 / 2.28 (float 2D, 512 boxes).
 template <bool L1>
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -1543,7 +1543,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 template <typename Rec>
-constexpr bool kThroughL1 = std::is_same<Rec, RecD>::value || std::is_same<Rec, RecF>::value;
+constexpr bool kThroughL1 = !std::is_same<Rec, RecF2>::value;
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -1826,11 +1826,12 @@ __global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
     else
       pair_walk<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
   };
-  // Warps clear of the periodic faces drop the minimum image, in 3D only: the 512-box 2D
-  // ensemble's small boxes put both kinds of warp on every SM, and the second copy of the
-  // walk cost more in instruction fetch than the shorter separations saved (FP64 2D pair
-  // pass 3.52 -> 3.54 ms, float 2D 2.23 -> 2.38 ms); the 3D passes gain 5 %.
-  if constexpr (DIM == 3) {
+  // Warps clear of the periodic faces drop the minimum image.  Not in float 2D, where the second
+  // copy of the walk cost more in instruction fetch than the shorter separations saved (small
+  // boxes put both kinds of warp on every SM: 512 boxes 2.23 -> 2.38 ms), nor in the wide walk
+  // (one 64^2 box 25.6 -> 27.7 us); FP64 2D 2.17 -> 2.09 ms on the 512 boxes, the 3D passes gain
+  // 5 %.
+  if constexpr (DIM == 3 || (sizeof(T) == 8 && !WIDE)) {
     if (warp_plain_image(d, clear_of_faces<T, DIM>(p, o.x, o.y, o.z)))
       walk(std::false_type{});
     else
