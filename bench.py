@@ -77,10 +77,9 @@ B_ALG_STEP = {"fp64": (10 * 3 + 5 * 6 + 4) * 8 + 28, "mixed": 380}
 B_ALG_PAIRS = {"fp64": (6 + 6 + 1 + 1 + 6 + 1 + 3 + 6) * 8 + 4,
                "mixed": (6 + 6 + 1) * 4 + (1 + 6 + 1 + 3 + 6) * 8 + 4}
 # FP64 floating-point operations per particle of one launch of the FP64 pair kernel, counted
-# by ncu on the 96^3 case of this workload (same lattice, same neighbours per particle):
-# DADD + DMUL + 2 DFMA thread instructions (each per-cycle rate times the SM sub-partition's
-# elapsed cycles) / particles (profiles/k_pairs_couette96_fp64.md).
-FP64_PAIR_FLOP = 11626.9
+# by ncu on 96 x 90 x 96 sites of this workload (same lattice, same neighbours per particle):
+# DADD + DMUL + 2 DFMA thread instructions / particles (profiles/k_pairs_couette96_fp64.md).
+FP64_PAIR_FLOP = 10737.0
 # FP64 peak of the B200: 148 SMs x 64 FP64 FMA lanes (ncu's dfma peak_sustained, 9,472 per
 # cycle) x 2 FLOP x the SM clock.
 FP64_LANES = 9472
@@ -771,9 +770,9 @@ def main():
             args.no_cpu_baseline = True
     if (args.pairs_traffic is None and args.workload == "couette3d" and args.lattice == 128
             and args.precision in (None, "fp64")):
-        # dram__bytes_read.sum + dram__bytes_write.sum of one k_pairs launch at 96^3
-        # (940,032 particles), scaled to the 2,195,456 particles of the benchmark
-        args.pairs_traffic = (386.815232e6 + 118.972928e6) * 2195456 / 940032
+        # dram__bytes_read.sum + dram__bytes_write.sum of one k_pairs launch at 96 x 90 x 96
+        # sites (884,736 particles), scaled to the 2,195,456 particles of the benchmark
+        args.pairs_traffic = (351.652352e6 + 106.985728e6) * 2195456 / 884736
     if args.precision is None:
         args.precision = "mixed" if args.workload == "sweep" else "fp64"
     if args.warmup < 3:
