@@ -730,45 +730,6 @@ __device__ __forceinline__ void pair_fluid_x1(const BoxParams& p, const PairPara
   }
 }
 
-// Two list positions of a fluid particle at once, both partners fluid or absent: the terms of
-// pair_fluid_x1 evaluated side by side in one block of straight code, so that their dependency
-// chains overlap, and added in list order.  A position without a partner inside the cutoff takes
-// part with zeros in place of the partner's velocity, stress and density, and adds zeros.
-template <typename T, int DIM, bool WRAP, int MODE, typename Rec>
-__device__ __forceinline__ void pair_fluid_x2(const BoxParams& p, const PairParams<T, DIM>& pp,
-                                              const PairOwn<T, DIM>& o, const Rec& ra,
-                                              const Rec& rb, const bool (&valid)[2],
-                                              PairAcc<T, DIM>& acc) {
-  T r[2][3], r2[2];
-  r2[0] = pair_sep<T, DIM, WRAP>(pp, p.wall, o, ra, r[0]);
-  r2[1] = pair_sep<T, DIM, WRAP>(pp, p.wall, o, rb, r[1]);
-  const bool in[2] = {valid[0] && r2[0] < pp.rcutsq, valid[1] && r2[1] < pp.rcutsq};
-  if (!(in[0] || in[1])) return;
-  PairRadial<T, DIM> g[2];
-  T v[2][3], Pi[6], Pj[2][6], dj[2];
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const Rec& rj = u == 0 ? ra : rb;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) r[u][a] = in[u] ? r[u][a] : T(0);
-    g[u].eval(pp, in[u] ? r2[u] : T(1), r[u]);
-    v[u][0] = in[u] ? o.v[0] - (T)rj.vx : T(0);
-    v[u][1] = in[u] ? o.v[1] - (T)rj.vy : T(0);
-    v[u][2] = in[u] ? o.v[2] - (T)rec_vz<DIM>(rj) : T(0);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) Pj[u][q] = in[u] ? rec_P<DIM>(rj, q) : T(0);
-    dj[u] = in[u] ? (T)rj.invd : T(0);
-  }
-#pragma unroll
-  for (int q = 0; q < 6; ++q) Pi[q] = o.P[q];
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    if constexpr (FluidTerms<MODE>::kGrad) pair_grad_add<DIM>(o, g[u], v[u], acc);
-    if constexpr (FluidTerms<MODE>::kForce)
-      pair_force_add<DIM>(pp, g[u], r[u], v[u], Pi, Pj[u], o.invd, dj[u], acc);
-  }
-}
-
 // Second half-kick of a fluid particle's velocity, v += (dt / 2) f / m
 // (kernel_move_sys_VV_part2.cu:13-58), as explicit fused multiply-adds so that the step's
 // fused form and the standalone V_Verlet_step2 give the same bits.

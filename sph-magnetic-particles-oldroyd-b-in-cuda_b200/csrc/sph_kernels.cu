@@ -1484,7 +1484,8 @@ __global__ void k_pressure(Dev d) {
 // Launch shape of the pair pass per precision and dimension, as measured on B200.  Every pass
 // evaluates one list position per step: with the fluid-fluid form of that walk, evaluating two
 // positions side by side (to overlap their dependency chains) measured slower everywhere
-// (float 3D at 128^3 2.41 vs 2.38 ms, FP64 2D on the 512-box ensemble 3.63 vs 3.52 ms).
+// (float 3D at 128^3 2.41 vs 2.38 ms, FP64 2D on the 512-box ensemble 3.63 vs 3.52 ms, and on one
+// 64^2 box, two warps per SM, 31.5 vs 27.9 us).
 //  - kWarps: warps per block; kMinBlocks: resident blocks per SM the register allocation is held
 //    to.  512 boxes, FP64 2D: 3 / 4 / 5 / 6 blocks 2.29 / 2.26 / 2.47 / 2.90 ms (spills from 5 on).
 //    128^3 float 3D: 3 / 4 / 5 blocks 1.994 / 2.004 / 2.037 ms; FP64 3D: 3 (168 registers).  Float
@@ -1495,15 +1496,15 @@ __global__ void k_pressure(Dev d) {
 //    registers with 32 bytes of spill, but at 16 warps per SM (4 blocks of 4 warps or 8 of
 //    2) it took 4.03 and 3.98 ms: the larger shared-memory carve-out leaves L1 too little
 //    for the record gathers.
-template <typename T, int DIM, bool WIDE = false>
+template <typename T, int DIM>
 struct PairShape {
   using Rec = typename RecFor<T, DIM>::type;
   static constexpr bool kF64 = sizeof(T) == 8;
   static constexpr bool kF2D = !kF64 && DIM == 2;
   // the float 2D pass runs 2-warp blocks (measured 2.29 vs 2.35 ms on the 512-box ensemble;
   // the float 3D pass was slower with them, the FP64 passes unchanged)
-  static constexpr int kWarps = WIDE ? 1 : kF2D ? 2 : 4;
-  static constexpr int kMinBlocks = WIDE ? 1 : kF2D ? 6 : kF64 && DIM == 2 ? 4 : 3;
+  static constexpr int kWarps = kF2D ? 2 : 4;
+  static constexpr int kMinBlocks = kF2D ? 6 : kF64 && DIM == 2 ? 4 : 3;
 };
 
 // The pair constants of a one-box context, viewed as PairParams (same layout).
@@ -1655,7 +1656,7 @@ struct PairWalk {
   const Dev& d;
   const Rec* __restrict__ rec;
   int4* sb;                      // the warp's staging rows
-  int* idx;                      // slots of two (wide walk: four) positions, 32 each
+  int* idx;                      // slots of two positions, 32 each
   int lane, i, n, nmax;
   const BoxParams& p;
   const PairParams<T, DIM>& pp;
@@ -1723,74 +1724,16 @@ __device__ __forceinline__ void pair_walk(const PairWalk<T, DIM>& W, NbrIter& it
   }
 }
 
-// The same, two positions per step, side by side where all partners of the warp are fluid.
-template <typename T, int DIM, bool WRAP, int MODE>
-__device__ __forceinline__ void pair_walk_wide(const PairWalk<T, DIM>& W, NbrIter& it,
-                                               PairAcc<T, DIM>& acc) {
-  using Rec = typename RecFor<T, DIM>::type;
-  using St = PairStage<Rec>;
-  static_assert(DIM == 2, "the type words come from the type array");
-  const int n = W.n, lane = W.lane;
-  int jc[2], tc[2];
-  auto fetch = [&](int k, int buf, int (&j)[2], int (&t)[2]) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      j[u] = k + u < n ? it.next() : -1;
-      W.idx[(buf * 2 + u) * 32 + lane] = j[u];
-      t[u] = j[u] >= 0 ? __ldg(&W.d.tinfo[j[u]]) : 0;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      if (k + u < W.nmax)
-        stage_records<Rec>(W.sb + (buf * 2 + u) * St::kRows, W.rec, W.idx + (buf * 2 + u) * 32, lane);
-    cp_async_commit();
-  };
-  fetch(0, 0, jc, tc);
-  int buf = 0;
-  for (int k = 0; k < W.nmax; k += 2) {
-    int jn[2], tn[2];
-    fetch(k + 2, buf ^ 1, jn, tn);
-    cp_async_wait_prev();
-    __syncwarp();
-    const int4* row = W.sb + buf * 2 * St::kRows + lane * St::kStride;
-    const StagedRec<T, Rec> R[2] = {StagedRec<T, Rec>(row), StagedRec<T, Rec>(row + St::kRows)};
-    bool valid[2], fluid = W.o.fluid;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      valid[u] = jc[u] >= 0 && jc[u] != W.i;
-      fluid = fluid && (!valid[u] || type_of(tc[u]) == 0);
-    }
-    if (__all_sync(SPH_FULL, fluid)) {
-      pair_fluid_x2<T, DIM, WRAP, MODE>(W.p, W.pp, W.o, R[0].r, R[1].r, valid, acc);
-    } else {
-#pragma unroll 1
-      for (int u = 0; u < 2; ++u) {
-        const StagedRec<T, Rec> Ru(row + u * St::kRows);
-        if (u == 0 ? valid[0] : valid[1])
-          pair_term<T, DIM, WRAP>(W.p, W.pp, W.cv, W.o, Ru.r, type_of(u == 0 ? tc[0] : tc[1]), acc);
-      }
-    }
-    __syncwarp();  // this buffer is refilled by the next step's fetch
-    buf ^= 1;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      jc[u] = jn[u];
-      tc[u] = tn[u];
-    }
-  }
-}
-
-template <typename T, int DIM, int MODE, bool EXT, bool ONE, bool WIDE = false>
-__global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
-                                  PairShape<T, DIM, WIDE>::kMinBlocks)
+template <typename T, int DIM, int MODE, bool EXT, bool ONE>
+__global__ void __launch_bounds__(PairShape<T, DIM>::kWarps * 32,
+                                  PairShape<T, DIM>::kMinBlocks)
     k_pairs(const __grid_constant__ Dev d) {
-  using Sh = PairShape<T, DIM, WIDE>;
+  using Sh = PairShape<T, DIM>;
   using Rec = typename Sh::Rec;
   using St = PairStage<Rec>;
   // per warp: a double buffer of staged positions
-  __shared__ int4 stage[Sh::kWarps][WIDE ? 4 : 2][St::kRows];
-  __shared__ __align__(16) int slots[kSlots<T, DIM> || WIDE ? Sh::kWarps : 1][WIDE ? 4 : 2][32];
+  __shared__ int4 stage[Sh::kWarps][2][St::kRows];
+  __shared__ __align__(16) int slots[kSlots<T, DIM> ? Sh::kWarps : 1][2][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wbase = (blockIdx.x * Sh::kWarps + w) * 32;
   if (wbase >= d.Ntot) return;  // whole warps only: the lanes below cooperate
@@ -1819,19 +1762,15 @@ __global__ void __launch_bounds__(PairShape<T, DIM, WIDE>::kWarps * 32,
   for (int s = 16; s > 0; s >>= 1) nmax = max(nmax, __shfl_xor_sync(SPH_FULL, nmax, s));
   NbrIter it;
   it.init(d, is);
-  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], &slots[kSlots<T, DIM> || WIDE ? w : 0][0][0], lane, i, n, nmax, p, pp, cv, o};
+  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], &slots[kSlots<T, DIM> ? w : 0][0][0], lane, i, n, nmax, p, pp, cv, o};
   auto walk = [&](auto wrap_tag) {
-    if constexpr (WIDE)
-      pair_walk_wide<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
-    else
-      pair_walk<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
+    pair_walk<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
   };
   // Warps clear of the periodic faces drop the minimum image.  Not in float 2D, where the second
   // copy of the walk cost more in instruction fetch than the shorter separations saved (small
-  // boxes put both kinds of warp on every SM: 512 boxes 2.23 -> 2.38 ms), nor in the wide walk
-  // (one 64^2 box 25.6 -> 27.7 us); FP64 2D 2.17 -> 2.09 ms on the 512 boxes, the 3D passes gain
+  // boxes put both kinds of warp on every SM: 512 boxes 2.23 -> 2.38 ms); FP64 2D 2.17 -> 2.09 ms on the 512 boxes, the 3D passes gain
   // 5 %.
-  if constexpr (DIM == 3 || (sizeof(T) == 8 && !WIDE)) {
+  if constexpr (DIM == 3 || sizeof(T) == 8) {
     if (warp_plain_image(d, clear_of_faces<T, DIM>(p, o.x, o.y, o.z)))
       walk(std::false_type{});
     else
@@ -2522,18 +2461,6 @@ template <typename T, int DIM, bool ONE>
 static void pairs_launch(const Launch& L, int mode, int with_ext) {
   constexpr int nt = PairShape<T, DIM>::kWarps * 32;
   const int nb = blocks(L.d.Ntot, nt);
-  // FP64 2D, up to kFewPairs warps per SM: two list positions side by side.  Measured (ms, one /
-  // two): 64^2 0.037 / 0.029, 192^2 (8 warps per SM) 0.054 / 0.050, 256^2 (14) 0.065 / 0.076; in
-  // 3D and in float the walk is bound by its instructions (3D FP64 16^3 0.109 / 0.111 ms).
-  constexpr int kFewPairs = 10;
-  if constexpr (sizeof(T) == 8 && DIM == 2) {
-    if (mode == kPairFused && few_warps(L, kFewPairs)) {
-      const int nb1 = blocks(L.d.Ntot, 32);
-      if (with_ext) k_pairs<T, DIM, kPairFused, true, ONE, true><<<nb1, 32, 0, S(L)>>>(L.d);
-      else k_pairs<T, DIM, kPairFused, false, ONE, true><<<nb1, 32, 0, S(L)>>>(L.d);
-      return;
-    }
-  }
   if (mode == kPairGradvAll)
     k_pairs<T, DIM, kPairGradvAll, false, ONE><<<nb, nt, 0, S(L)>>>(L.d);
   else if (mode == kPairForcesOnly)

@@ -1,6 +1,5 @@
-"""Contexts of few particles take other forms of the list build (two warps per cell), the density
-pass (eight entries side by side) and the FP64 2D pair pass (two positions side by side) than
-large ones.  The sums are the same, term for term: a box alone gives the bits it gives among
+"""Contexts of few particles take other forms of the list build (two warps per cell) and the density
+pass (eight entries side by side) than large ones.  The sums are the same, term for term: a box alone gives the bits it gives among
 enough copies of itself to take the forms for many particles."""
 import os
 
