@@ -49,12 +49,17 @@ __device__ __forceinline__ double xfma(double a, double b, double c) { return __
 // 1 / sqrt(x) of a positive normal x.  FP64: the hardware's seed and one third-order
 // Householder step, y (1 + e (1/2 + 3/8 e)) with e = 1 - x y^2 (the Taylor series of
 // (1 - e)^(-1/2) to second order: the error is 5/16 e^3), without the special cases of the
-// library function, which no pair of distinct particles meets.
+// library function: below the smallest normal number the result is not a number.
 __device__ __forceinline__ double inv_sqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
   return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
+}
+// sqrt(x) as x times that; 0 below the smallest normal number, where the seed has no value (a
+// particle in the centre of a colloid).
+__device__ __forceinline__ double length_of(double x, double inv) {
+  return x >= 0x1p-1022 ? __dmul_rn(x, inv) : 0.0;
 }
 
 // a / b.  FP64: a times the hardware's reciprocal seed after one third-order step,
@@ -503,10 +508,10 @@ __device__ __forceinline__ void ghost_velocity(const BoxParams& p, const PairPar
   const T d2 = DIM == 3 ? rc[0] * rc[0] + rc[1] * rc[1] + rc[2] * rc[2]
                         : rc[0] * rc[0] + rc[1] * rc[1];
   const T R = (T)p.coll_R;
-  T dc, n[3];  // distance from the centre and its direction
+  T dc, n[3];  // distance from the centre and its direction (in the centre none, and not used)
   if constexpr (sizeof(T) == 8) {
     const T inv = inv_sqrt(d2);
-    dc = d2 * inv;
+    dc = length_of(d2, inv);
 #pragma unroll
     for (int a = 0; a < 3; ++a) n[a] = rc[a] * inv;
   } else {
