@@ -57,7 +57,7 @@ __device__ __forceinline__ double inv_sqrt(double x) {
   return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 // sqrt(x) as x times that; 0 below the smallest normal number, where the seed has no value (a
-// particle in the centre of a colloid).
+// particle's own density term, a particle in the centre of a colloid).
 __device__ __forceinline__ double length_of(double x, double inv) {
   return x >= 0x1p-1022 ? __dmul_rn(x, inv) : 0.0;
 }

@@ -455,7 +455,7 @@ __device__ __forceinline__ T density_term(const typename V4<T>::type& xi,
   if (!SELECT && !in) return T(0);
   T w;
   if constexpr (sizeof(T) == 8) {
-    w = sph_w(r2 > 0.0 ? xmul(r2, inv_sqrt(r2)) : 0.0, rcut_inv);
+    w = sph_w(length_of(r2, inv_sqrt(r2)), rcut_inv);
   } else {
     w = sph_w(r2 > 0.0f ? r2 * rsqrt(r2) : 0.0f, rcut_inv, cw);
   }

@@ -1,9 +1,11 @@
-"""Distances of zero: a fluid particle exactly in the centre of a colloid, which has a finite force
-in the reference's formulas (a fluid particle inside a colloid takes the plain velocity difference).
+"""Distances of zero in FP64: a fluid particle exactly in the centre of a colloid, and two fluid
+particles whose distance squared is below the smallest normal number.  Both have finite values in
+the reference's formulas (a fluid particle inside a colloid takes the plain velocity difference; the
+kernel at zero distance is W(0)).
 
 Against the FP64 oracle: forces within 1e-11 of the group's scale (some 30 pairs of a few dozen
 rounded operations each, 1e-14, with a margin for the cancellation of the pressure terms, a factor
-of 100 here)."""
+of 100 here), densities within 1e-13 (a few ulps a term)."""
 import os
 
 import numpy as np
@@ -55,5 +57,24 @@ def test_fluid_particle_in_the_centre_of_a_colloid(workdir, dim, precision):
         assert all(np.isfinite(e.field(f)).all() for f in fields), name
         if precision == "fp64":
             assert group_error(e.field, o.field, fields, "max", dim) <= 1e-11, name
+    e.close()
+    o.close()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_density_of_two_particles_at_one_point(workdir, dim):
+    e, o, fluid = _pair(workdir, dim)
+    a, b = fluid[3], fluid[40]
+    for q in "xyz"[:dim]:
+        x = e.field(q)
+        x[a], x[b] = (0.0, 1e-160) if q == "x" else (2.3 / N, 2.3 / N)
+        for s in (e, o):
+            s.set_field(q, x)
+    for s in (e, o):
+        s.neighbours_search()
+        s.calculate_density()
+    want, got = o.field("dens"), e.field("dens")
+    assert np.isfinite(want).all() and want[a] > 1.2 * np.median(want)
+    assert np.abs(got - want).max() <= 1e-13 * want.max()
     e.close()
     o.close()
