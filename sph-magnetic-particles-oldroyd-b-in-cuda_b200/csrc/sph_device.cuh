@@ -49,7 +49,7 @@ __device__ __forceinline__ double xfma(double a, double b, double c) { return __
 // 1 / sqrt(x) of a positive normal x.  FP64: the hardware's seed and one third-order
 // Householder step, y (1 + e (1/2 + 3/8 e)) with e = 1 - x y^2 (the Taylor series of
 // (1 - e)^(-1/2) to second order: the error is 5/16 e^3), without the special cases of the
-// library function: below the smallest normal number the result is not a number.
+// library function: below the smallest normal number the result is not finite.
 __device__ __forceinline__ double inv_sqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
