@@ -56,10 +56,10 @@ __device__ __forceinline__ double inv_sqrt(double x) {
   const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
   return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
-// sqrt(x) as x times that; 0 below the smallest normal number, where the seed has no value (a
-// particle's own density term, a particle in the centre of a colloid).
+constexpr double kMinNormal = 0x1p-1022;
+// sqrt(x) of x >= 0 as x times that; 0 below the smallest normal number.
 __device__ __forceinline__ double length_of(double x, double inv) {
-  return x >= 0x1p-1022 ? __dmul_rn(x, inv) : 0.0;
+  return x >= kMinNormal ? __dmul_rn(x, inv) : 0.0;
 }
 
 // a / b.  FP64: a times the hardware's reciprocal seed after one third-order step,
@@ -508,10 +508,10 @@ __device__ __forceinline__ void ghost_velocity(const BoxParams& p, const PairPar
   const T d2 = DIM == 3 ? rc[0] * rc[0] + rc[1] * rc[1] + rc[2] * rc[2]
                         : rc[0] * rc[0] + rc[1] * rc[1];
   const T R = (T)p.coll_R;
-  T dc, n[3];  // distance from the centre and its direction (in the centre none, and not used)
+  T dc, n[3];  // distance from the centre and its direction
   if constexpr (sizeof(T) == 8) {
     const T inv = inv_sqrt(d2);
-    dc = length_of(d2, inv);
+    dc = d2 * inv;
 #pragma unroll
     for (int a = 0; a < 3; ++a) n[a] = rc[a] * inv;
   } else {
@@ -540,7 +540,11 @@ __device__ __forceinline__ void ghost_velocity(const BoxParams& p, const PairPar
   const T ds = (own ? along : -along) - dq;
   T beta = T(1) + quotient(ds, dq);
   beta = beta <= beta_max ? beta : beta_max;
-  const bool inside = dq < T(0);  // not extrapolated, and without the rotation
+  // Inside the colloid: not extrapolated, and without the rotation.  A particle in the centre
+  // (FP64: d2 is no normal number, and dc has no value) is inside too; the test of the exponent
+  // bits costs nothing measurable (512 boxes 2.073 / 2.060 ms without / with it).
+  bool inside = dq < T(0);
+  if constexpr (sizeof(T) == 8) inside = inside || __double2hiint(d2) < 0x00100000;
   beta = inside ? T(1) : beta;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
