@@ -170,6 +170,10 @@ __device__ __forceinline__ void net_columns(uint32_t tm, F use) {
   }
 }
 
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
 struct NetArgs {
   const float* x;       // n x IN
   const float* y;       // targets (training)
@@ -230,7 +234,11 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_forward(NetArgs a) {
     }
     const size_t gbase = ((size_t)t * 64 + 16 * grp) * kS + row;          // slopes, float4
     const size_t tbase = ((size_t)head * HID + 64 * grp) * a.n + b;       // transposed
-    float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    // Output sums of a prediction: 16 columns in order, then pairs of such sums, pairs of pairs
+    // and so on.  The tree is the same for every R, so that a point's outputs do not depend on
+    // how many others are predicted with it.
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 o4 = zero4, pair4 = zero4, half4 = zero4;
     // 8 neurons: pre-activations z -> activations into the A operand (and the backward
     // pass's arrays); last: the output layer's sums instead of an operand
     auto activate = [&](const float (&z)[8], int k, float* g, __nv_bfloat16* ht, bool last) {
@@ -298,6 +306,16 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_forward(NetArgs a) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) z[q] = v[q] + s->b3[64 * grp + 8 * (sub8 + k) + q];
       activate(z, k, a.g3, a.t3, true);
+      if (!TRAIN && (k & 1)) {  // the 16 columns of group k / 2 are done
+        const int g = k >> 1;
+        if (g & 1) o4 = add4(pair4, o4);
+        if (g == 3) o4 = add4(half4, o4);
+        if (g == 1) half4 = o4;
+        if (g + 1 < 4 / R) {
+          pair4 = o4;
+          o4 = zero4;
+        }
+      }
     });
     const size_t at = (size_t)head * a.n + b;
     if (!TRAIN) {
@@ -308,11 +326,9 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_forward(NetArgs a) {
 #pragma unroll
         for (int c = 0; c < kNetChunks; ++c) {
           g4[c] = s->red[c][row];
-#pragma unroll
-          for (int d = 1; d < R; ++d) {
-            const float4 u = s->red[c][row + d * kS];
-            g4[c] = make_float4(g4[c].x + u.x, g4[c].y + u.y, g4[c].z + u.z, g4[c].w + u.w);
-          }
+          if (R > 1) g4[c] = add4(g4[c], s->red[c][row + kS]);
+          if (R == 4)
+            g4[c] = add4(g4[c], add4(s->red[c][row + 2 * kS], s->red[c][row + 3 * kS]));
         }
         float* o = a.out + at * OUT;  // any float alignment
         o[0] = ((g4[0].x + g4[1].x) + (g4[2].x + g4[3].x)) + s->b4[0];
