@@ -136,16 +136,21 @@ __device__ __forceinline__ void net_close(NetSmall* s, bool ok, int* err) {
   }
 }
 
-// Stores 8 activations of a sample, columns 8 k8 .. + 7 of chunk c, into its rows of the A
-// operand.
+// 8 activations of a sample, moved 16 bytes at a time.
+struct __align__(16) Act8 {
+  __nv_bfloat16 v[8];
+  __device__ __forceinline__ __nv_bfloat16& operator[](int q) { return v[q]; }
+};
+static_assert(sizeof(Act8) == sizeof(uint4) && alignof(Act8) == alignof(uint4), "one 16-byte move");
+
+// Stores them, columns 8 k8 .. + 7 of chunk c, into the sample's rows of the A operand.
 template <int R>
-__device__ __forceinline__ void net_store8(uint8_t* smem, int c, int sample, int k8,
-                                           const __nv_bfloat16 (&h)[8]) {
+__device__ __forceinline__ void net_store8(uint8_t* smem, int c, int sample, int k8, const Act8& h) {
 #pragma unroll
   for (int d = 0; d < R; ++d)
     *reinterpret_cast<uint4*>(smem + c * kNetChunkA +
                               tc::core_offset(sample + d * (tc::kTileM / R), k8)) =
-        *reinterpret_cast<const uint4*>(h);
+        *reinterpret_cast<const uint4*>(&h);
 }
 
 // Reads this thread's 64 / R accumulator columns 16 at a time, the next 16 in flight while
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_forward(NetArgs a) {
     // pass's arrays); last: the output layer's sums instead of an operand
     auto activate = [&](const float (&z)[8], int k, float* g, __nv_bfloat16* ht, bool last) {
       const int k8 = sub8 + k;
-      __nv_bfloat16 h[8];
+      Act8 h;
       float sl[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -398,7 +403,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_backward(NetArgs a) {
     const float4* gp = reinterpret_cast<const float4*>(g) + gbase + (size_t)(2 * k8) * kS;
     const float4 u = gp[0], w = gp[kS];
     const float sl[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-    __nv_bfloat16 h[8];
+    Act8 h;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       h[q] = __float2bfloat16(v[q] * sl[q]);
