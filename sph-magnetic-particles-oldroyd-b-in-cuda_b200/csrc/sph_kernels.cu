@@ -678,8 +678,10 @@ __device__ __forceinline__ int list_odd_particle(const Dev& d, int ti, int tb) {
 // A particle's row multiplies them by (-2x -2y) (-2z 1) (-2x -2y) (-2z 1) and, in the upper half
 // of K, the same words once more by (-2x' -2y') (-2z' 0) (-2x' -2y') (-2z' 0); the accumulators
 // start from |x_i|^2 - cut^2.  Offsets are below 2 (cells are at most 4/3 rcut wide), so a split
-// coordinate is within 5e-7 and the square within 1.5e-5 of its value, against the 1e-4 by which
-// list_cut2 exceeds the cutoff that every consumer applies exactly: no neighbour is missed.
+// coordinate is within 5e-7 and the square within 1.5e-5 of its value.  The products are exact.
+// Their sum, if the matrix unit cuts each of the 17 addends to 24 bits of the largest (below 8 for
+// a pair within reach: n, (1.16 + 1)^2 at most), is off by 17 x 2^-21, 1e-5, at most.  list_cut2
+// exceeds the cutoff that every consumer applies exactly by 1e-4: no neighbour is missed.
 // Candidates further off (minimum-image placement) only have to be outside: held within 200 rcut,
 // and n below what a float16 holds.
 //
@@ -895,6 +897,9 @@ __global__ void __launch_bounds__(kListWarps * 32, 8)
         }
       }
       const bool listed = active && !odd && !lost;
+      // A row without a particle is zero but for its start value, and has no hits; a position
+      // too far out for a float16 would make it infinities times zero.
+      if (!listed) xi = yi = zi = 0.f;
       // this particle's row: words of the lower and the upper half of K, start value
       const uint4 cw = candidate_words(xi, yi, zi, true);
       const float2 h01 = unpack_h2(cw.x), h23 = unpack_h2(cw.y), l01 = unpack_h2(cw.z),
