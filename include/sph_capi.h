@@ -285,13 +285,16 @@ sph_status sph_reset_observables(sph_ctx* ctx);
                             cell (2D cells at overlap 4 hold about 16 particles)
      density_block          0: the density pass over neighbour-cell tiles (a warp per cell,
                             the cells' positions staged in shared memory); 64, 128 or 256:
-                            threads per block of the per-particle density pass
+                            threads per block of the per-particle density pass.  A context
+                            of few particles (up to 448 per multiprocessor in FP64, 768 in
+                            mixed precision; 66,304 and 113,664 on a B200) takes that pass
+                            in blocks of one warp for all three
    sph_set_tuning applies a geometry (captured step graphs are rebuilt).  sph_autotune
    times the candidates on the context's current state -- the timed passes recompute the
    same lists and densities, so the simulation is unchanged -- and keeps the fastest.
-   With cache_path it first looks for an entry keyed by GPU name, dimension, overlap and
-   particle count (rounded to a power of two) in that JSON file, and records its choice
-   there otherwise.  The cell size stays the reference's (rcut): its cell grid carries the
+   With cache_path it first looks for an entry keyed by GPU name, dimension, precision,
+   overlap, particle count (rounded to a power of two) and form of the density pass in that
+   JSON file, and records its choice there otherwise.  The cell size stays the reference's (rcut): its cell grid carries the
    stale-range semantics of the exported cell arrays. */
 typedef struct sph_tuning {
   int list_threads_per_cell;

@@ -1517,9 +1517,10 @@ bool tuning_ok(const sph_tuning& t) {
           t.density_block == 256);
 }
 
-// Cache key: GPU name, dimension, overlap of the first box, total particles rounded to a
-// power of two.
-std::string tune_key(const sph_ctx* c) {
+// Cache key: GPU name, dimension, precision, overlap of the first box, total particles rounded
+// to a power of two, and whether they take the density pass in one form (the line between lies
+// inside such a range of particle counts).
+std::string tune_key(sph_ctx* c) {
   cudaDeviceProp prop;
   std::string name = cudaGetDeviceProperties(&prop, c->device) == cudaSuccess ? prop.name : "gpu";
   for (char& ch : name)
@@ -1528,8 +1529,10 @@ std::string tune_key(const sph_ctx* c) {
   while ((1ll << (lg + 1)) <= (long long)std::max(c->d.Ntot, 1)) ++lg;
   if ((1ll << (lg + 1)) - c->d.Ntot < c->d.Ntot - (1ll << lg)) ++lg;
   char buf[320];
-  std::snprintf(buf, sizeof(buf), "%s|dim=%d|overlap=%g|N=2^%d", name.c_str(), c->dim,
-                c->boxes.empty() ? 0.0 : c->boxes[0].in.overlap, lg);
+  std::snprintf(buf, sizeof(buf), "%s|dim=%d|%s|overlap=%g|N=2^%d%s", name.c_str(), c->dim,
+                c->prec == SPH_PREC_FP64 ? "fp64" : "mixed",
+                c->boxes.empty() ? 0.0 : c->boxes[0].in.overlap, lg,
+                density_one_form(launcher(c)) ? "|one-warp blocks" : "");
   return buf;
 }
 
@@ -1652,7 +1655,9 @@ sph_status sph_autotune(sph_ctx* c, const char* cache_path, sph_tuning* chosen) 
       best.list_threads_per_cell = tpc;
     }
   }
-  for (int nt : {0, 64, 128, 256}) {  // 0: neighbour-cell tiles
+  const bool one_form = density_one_form(launcher(c));  // then 128 stands for 64 and 256 too
+  for (int nt : {0, 64, 128, 256}) {                    // 0: neighbour-cell tiles
+    if (one_form && (nt == 64 || nt == 256)) continue;
     Launch L = launcher(c);
     L.density_block = nt;
     const double ms = time_phase(c, reps, [&] { return launch_density_dim(L, c->dim); }, &bad);

@@ -2420,14 +2420,17 @@ int launch_colloid_cells_n(const Launch& L, int nboxes, int max_coll) {
 // side in the warp (its registers are free), in one-warp blocks spread over all SMs.
 inline bool few_warps(const Launch& L, int per_sm) { return L.d.Ntot <= 32 * per_sm * L.nsm; }
 
-// Up to kFewDensity warps per SM: the terms of eight list entries side by side.  Measured (ms,
+// Up to few_density warps per SM: the terms of eight list entries side by side.  Measured (ms,
 // two at a time / eight): FP64 at 13.5 warps per SM (40 x 40 x 40) 0.062 / 0.056, at 18 0.066 /
 // 0.086; float at 18 0.056 / 0.052, at 26 0.065 / 0.064, at 37 0.087 / 0.090.
-template <typename T>
-constexpr int kFewDensity = sizeof(T) == 8 ? 14 : 24;
+// density_block 64, 128 and 256 are then one form (density_one_form).
+constexpr int few_density(bool fp64) { return fp64 ? 14 : 24; }
+bool density_one_form(const Launch& L) {
+  return few_warps(L, few_density(L.prec == SPH_PREC_FP64));
+}
 template <typename T, int DIM>
 static void density_launch(const Launch& L) {
-  if (few_warps(L, kFewDensity<T>)) {
+  if (density_one_form(L)) {
     k_density<T, DIM, 8><<<blocks(L.d.Ntot, 32), 32, 0, S(L)>>>(L.d);
   } else {
     const int nt = L.density_block;

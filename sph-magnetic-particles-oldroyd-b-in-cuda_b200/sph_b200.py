@@ -495,8 +495,9 @@ class System:
         self._ok(lib().sph_set_tuning(self._h, ctypes.byref(t)))
 
     def autotune(self, cache_path=None):
-        """Pick the fastest launch geometry (cached per GPU, dim, overlap and size when a
-        cache file is given); returns it.  The simulation state is not changed."""
+        """Pick the fastest launch geometry (cached per GPU, dim, precision, overlap, size and
+        form of the density pass when a cache file is given); returns it.  The simulation
+        state is not changed."""
         t = SphTuning()
         self._ok(lib().sph_autotune(self._h, os.fsencode(cache_path) if cache_path else None,
                                     ctypes.byref(t)))
