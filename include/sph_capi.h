@@ -286,9 +286,9 @@ sph_status sph_reset_observables(sph_ctx* ctx);
      density_block          0: the density pass over neighbour-cell tiles (a warp per cell,
                             the cells' positions staged in shared memory); 64, 128 or 256:
                             threads per block of the per-particle density pass.  A context
-                            of few particles (up to 448 per multiprocessor in FP64, 768 in
-                            mixed precision; 66,304 and 113,664 on a B200) takes that pass
-                            in blocks of one warp for all three
+                            of few particles (per multiprocessor up to 448 in FP64, 576 in 2D
+                            and 768 in 3D in mixed precision; 66,304, 85,248 and 113,664 on
+                            a B200) takes that pass in blocks of one warp for all three
    sph_set_tuning applies a geometry (captured step graphs are rebuilt).  sph_autotune
    times the candidates on the context's current state -- the timed passes recompute the
    same lists and densities, so the simulation is unchanged -- and keeps the fastest.

@@ -1532,7 +1532,7 @@ std::string tune_key(sph_ctx* c) {
   std::snprintf(buf, sizeof(buf), "%s|dim=%d|%s|overlap=%g|N=2^%d%s", name.c_str(), c->dim,
                 c->prec == SPH_PREC_FP64 ? "fp64" : "mixed",
                 c->boxes.empty() ? 0.0 : c->boxes[0].in.overlap, lg,
-                density_one_form(launcher(c)) ? "|one-warp blocks" : "");
+                density_one_form(launcher(c), c->dim) ? "|one-warp blocks" : "");
   return buf;
 }
 
@@ -1655,8 +1655,8 @@ sph_status sph_autotune(sph_ctx* c, const char* cache_path, sph_tuning* chosen) 
       best.list_threads_per_cell = tpc;
     }
   }
-  const bool one_form = density_one_form(launcher(c));  // then 128 stands for 64 and 256 too
-  for (int nt : {0, 64, 128, 256}) {                    // 0: neighbour-cell tiles
+  const bool one_form = density_one_form(launcher(c), c->dim);  // 128 stands for 64 and 256 too
+  for (int nt : {0, 64, 128, 256}) {  // 0: neighbour-cell tiles
     if (one_form && (nt == 64 || nt == 256)) continue;
     Launch L = launcher(c);
     L.density_block = nt;

@@ -286,7 +286,7 @@ int launch_build_lists_dim(const Launch& L, int dim);
 int launch_colloid_cells_n(const Launch& L, int nboxes, int max_coll);
 int launch_density_dim(const Launch& L, int dim);
 // The particle count takes the per-particle density pass in one form, whatever density_block > 0.
-bool density_one_form(const Launch& L);
+bool density_one_form(const Launch& L, int dim);
 int launch_pressure(const Launch& L);
 int launch_pairs_dim(const Launch& L, int dim, int mode, int with_ext);
 int launch_ext_force(const Launch& L);

@@ -504,7 +504,10 @@ __device__ __forceinline__ void density_epilogue(const Dev& d, int i, const BoxP
 //
 // With 16 threads per cell (k_build_lists_half) each half-warp works on its own cell, chunks are
 // 16 slots long and the test is in packed float.  The neighbours are the same either way (same
-// candidates, same order).
+// candidates, same order).  It is a choice of the tuning, the faster build of large 2D boxes with
+// 16 particles a cell only.  Measured (us, a warp per cell / a half): 2D, overlap 4, 64^2 12.0 /
+// 14.8, 256^2 16.2 / 17.1, 512^2 35.0 / 34.8, 600^2 46.8 / 44.0 (its pair pass 151.6 / 155.1, over
+// longer lists); overlap 3, 512^2 45.2 / 53.2; 512 boxes 446 / 660; 3D, 48^3 40.6 / 98.3.
 //
 // Blocks of 4 warps, measured against 8 (128^3 list build 1.66 vs 1.88 ms; 2D ensemble
 // 1.15 vs 1.19 ms, with the test loop not unrolled).
@@ -520,11 +523,6 @@ __device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
 __device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
   f32x2 d;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
@@ -2393,9 +2391,9 @@ int launch_build_lists_dim(const Launch& L, int dim) {
   const bool half = L.list_tpc == 16;
   // Cells of more than 28 particles on average hold more than a warp's 32 here and there, and the
   // warps of those cells, with a second round, are what a small grid waits for: two warps per
-  // cell, up to 64 cells per SM.  Measured in 3D (ms, one / two): 25 x 25 x 31 sites (4 cells per
-  // SM) 0.062 / 0.038, 56^3 (44) 0.130 / 0.114, 61 x 53 x 67 (51) 0.136 / 0.129; 128^3 (520) 0.856
-  // / 0.895, and 48^3, 27 per cell, 0.069 / 0.075.
+  // cell, up to 64 cells per SM.  Measured in 3D (us, one / two): 4 cells per SM 41.5 / 27.9, 39
+  // 82.0 / 74.6, 56 93.6 / 90.4, 60 105.0 / 99.4; 82 112.8 / 114.6, 106 134.0 / 138.8, 501 520 /
+  // 566; and, with 27 per cell, 28 cells per SM, 40.9 / 50.3.
   const int split = L.d.Ntot / 28 > L.d.Ctot && L.d.Ctot <= 64 * L.nsm ? 2 : 1;
   const int nb = blocks(blocks(L.d.Ctot, half ? 2 : 1) * split, kListWarps);
   constexpr int nt = kListWarps * 32;
@@ -2420,17 +2418,20 @@ int launch_colloid_cells_n(const Launch& L, int nboxes, int max_coll) {
 // side in the warp (its registers are free), in one-warp blocks spread over all SMs.
 inline bool few_warps(const Launch& L, int per_sm) { return L.d.Ntot <= 32 * per_sm * L.nsm; }
 
-// Up to few_density warps per SM: the terms of eight list entries side by side.  Measured (ms,
-// two at a time / eight): FP64 at 13.5 warps per SM (40 x 40 x 40) 0.062 / 0.056, at 18 0.066 /
-// 0.086; float at 18 0.056 / 0.052, at 26 0.065 / 0.064, at 37 0.087 / 0.090.
+// Up to few_density warps per SM: the terms of eight list entries side by side.  Measured (us,
+// two at a time / eight), FP64: 3D at 13.5 warps per SM 53.5 / 49.5, at 15.6 53.5 / 51.5, at 16.8
+// 57.4 / 78.7; 2D (overlap 4) at 13.8 23.7 / 22.8, at 15.4 22.8 / 22.8, at 16.6 24.9 / 31.6 (an SM
+// holds 16 of its warps).  Float: 3D at 13.5 45.2 / 39.2, at 18.0 47.4 / 45.4, at 20.6 49.5 / 50.3
+// (the whole step 282 / 280), at 23.4 the step 277 / 275; 2D at 15.4 20.8 / 18.9, at 17.8 20.8 /
+// 21.2, at 20.3 21.6 / 22.8 (the step 123.1 / 124.1).
 // density_block 64, 128 and 256 are then one form (density_one_form).
-constexpr int few_density(bool fp64) { return fp64 ? 14 : 24; }
-bool density_one_form(const Launch& L) {
-  return few_warps(L, few_density(L.prec == SPH_PREC_FP64));
+constexpr int few_density(bool fp64, int dim) { return fp64 ? 14 : dim == 3 ? 24 : 18; }
+bool density_one_form(const Launch& L, int dim) {
+  return few_warps(L, few_density(L.prec == SPH_PREC_FP64, dim));
 }
 template <typename T, int DIM>
 static void density_launch(const Launch& L) {
-  if (density_one_form(L)) {
+  if (density_one_form(L, DIM)) {
     k_density<T, DIM, 8><<<blocks(L.d.Ntot, 32), 32, 0, S(L)>>>(L.d);
   } else {
     const int nt = L.density_block;
