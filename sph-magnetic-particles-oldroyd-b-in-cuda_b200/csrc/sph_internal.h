@@ -45,9 +45,9 @@ enum ErrInfo : int {
   // buffer parity (Dev::parity): a search's hash sets the word of the parity that the search
   // ends with for every position it finds outside and its cell scan clears the other word, for
   // the next search; the half-kicks set the current word for every position they leave
-  // outside, and so does any write of positions from the host.  While it is set the list build places every candidate by its minimum image;
-  // while it is clear the pair passes may drop the minimum image for particles clear of the
-  // periodic faces (clear_of_faces).
+  // outside, and so does any write of positions from the host.  While it is set the list build
+  // places every candidate by its minimum image; while it is clear the pair passes may drop the
+  // minimum image for particles clear of the periodic faces (clear_of_faces).
   kPosOutside = 5,
   kPosOutside1 = 6,
   kErrInfoLen = 8,

@@ -1772,14 +1772,15 @@ __global__ void __launch_bounds__(PairShape<T, DIM>::kWarps * 32,
   for (int s = 16; s > 0; s >>= 1) nmax = max(nmax, __shfl_xor_sync(SPH_FULL, nmax, s));
   NbrIter it;
   it.init(d, is);
-  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], &slots[kSlots<T, DIM> ? w : 0][0][0], lane, i, n, nmax, p, pp, cv, o};
+  int* const idx = &slots[kSlots<T, DIM> ? w : 0][0][0];
+  const PairWalk<T, DIM> W{d, rec, &stage[w][0][0], idx, lane, i, n, nmax, p, pp, cv, o};
   auto walk = [&](auto wrap_tag) {
     pair_walk<T, DIM, decltype(wrap_tag)::value, MODE>(W, it, acc);
   };
   // Warps clear of the periodic faces drop the minimum image.  Not in float 2D, where the second
   // copy of the walk cost more in instruction fetch than the shorter separations saved (small
-  // boxes put both kinds of warp on every SM: 512 boxes 2.23 -> 2.38 ms); FP64 2D 2.17 -> 2.09 ms on the 512 boxes, the 3D passes gain
-  // 5 %.
+  // boxes put both kinds of warp on every SM: 512 boxes 2.23 -> 2.38 ms); FP64 2D 2.17 -> 2.09 ms
+  // on the 512 boxes, the 3D passes gain 5 %.
   if constexpr (DIM == 3 || sizeof(T) == 8) {
     if (warp_plain_image(d, clear_of_faces<T, DIM>(p, o.x, o.y, o.z)))
       walk(std::false_type{});

@@ -346,22 +346,23 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_forward(NetArgs a) {
       __syncthreads();
       float* red = reinterpret_cast<float*>(s->red);
       if (arow < kS) {
-      float acc = 0.0f;
-      for (int c = 0; c < kNetChunks; ++c)
+        float acc = 0.0f;
+        for (int c = 0; c < kNetChunks; ++c)
 #pragma unroll 2
-        for (int k8 = 0; k8 < 8; ++k8) {
-          const uint4 u = *reinterpret_cast<const uint4*>(smem + c * kNetChunkA + tc::core_offset(row, k8));
-          const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+          for (int k8 = 0; k8 < 8; ++k8) {
+            const uint4 u = *reinterpret_cast<const uint4*>(smem + c * kNetChunkA +
+                                                            tc::core_offset(row, k8));
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float2 h = __bfloat1622float2(h2[q]);
-            acc = fmaf(s->w4[64 * c + 8 * k8 + 2 * q][grp], h.x, acc);
-            acc = fmaf(s->w4[64 * c + 8 * k8 + 2 * q + 1][grp], h.y, acc);
+            for (int q = 0; q < 4; ++q) {
+              const float2 h = __bfloat1622float2(h2[q]);
+              acc = fmaf(s->w4[64 * c + 8 * k8 + 2 * q][grp], h.x, acc);
+              acc = fmaf(s->w4[64 * c + 8 * k8 + 2 * q + 1][grp], h.y, acc);
+            }
           }
-        }
-      const float r = acc + s->b4[grp], e = r - a.y[(size_t)b * OUT + grp];
-      a.dout[at * OUT + grp] = 2.0f * e / (float)(a.n * OUT);
-      red[4 * row + grp] = e;
+        const float r = acc + s->b4[grp], e = r - a.y[(size_t)b * OUT + grp];
+        a.dout[at * OUT + grp] = 2.0f * e / (float)(a.n * OUT);
+        red[4 * row + grp] = e;
       }
       __syncthreads();
       if (grp == 0 && arow < kS) {
@@ -657,7 +658,8 @@ __global__ void __launch_bounds__(256) k_update(UpdateArgs a) {
     // the parameters in order, without W2 and W3
     const int off = k < OFF_W2 ? k : k < OFF_W2 + HID ? k + HID * HID : k + 2 * HID * HID;
     const size_t t = base + off;
-    const float p = ADAM ? adam(a.params, a.m, a.v, t, a.grads[t], a.adam) : CAST ? a.params[t] : 0.0f;
+    const float p =
+        ADAM ? adam(a.params, a.m, a.v, t, a.grads[t], a.adam) : CAST ? a.params[t] : 0.0f;
     if (CAST) {
       if (off < OFF_B1) a.w1b[(size_t)head * HID * IN + off] = __float2bfloat16(p);
       if (off >= OFF_W4 && off < OFF_B4)
