@@ -169,7 +169,7 @@ const char* sph_status_string(sph_status s);
 /* ----------------------------------------------- step methods of class_system */
 
 /* class_system::neighbours_search (src/system_neighbours_search.cu:19-110): cell hash,
-   stable (cell, id) radix sort, cell ranges, colloid coarse grid; also builds the
+   stable (cell, id) counting sort, cell ranges, colloid coarse grid; also builds the
    neighbour lists the pair kernels read. */
 sph_status sph_neighbours_search(sph_ctx* ctx);
 
@@ -348,7 +348,11 @@ sph_status sph_neighbours_search_noalloc(const double* x, const double* y, const
 #define SPH_NUM_PHASES 11
 sph_status sph_profile_phases(sph_ctx* ctx, int nsteps, double* ms);
 /* Name of phase k ("vv1", "hash", "sort", "reorder", "lists", "colloid_cells",
-   "density", "pairs", "walls", "colloids", "vv2"). */
+   "density", "pairs", "walls", "colloids", "vv2").  A step's kernels hold more than one of its
+   parts: "vv1" is the first half-kick of the colloids alone, "hash" also the particles' half-kick
+   and drift, "sort" also the magnetic moments, "pairs" also the fluid's second half-kick and
+   "colloids" their own; "vv2" brackets no kernel, and two events without one between them read
+   about 3 us. */
 const char* sph_phase_name(int k);
 
 #ifdef __cplusplus

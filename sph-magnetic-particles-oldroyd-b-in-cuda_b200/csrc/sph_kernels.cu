@@ -1484,12 +1484,13 @@ __global__ void k_pressure(Dev d) {
 // while the current ones are evaluated.  Each lane then reads its records
 // from shared memory (row stride padded by one piece: conflict-free).
 //
-// What bounds the FP64 passes is the load/store pipe all of this goes through (3D: 79 % busy at
-// 96^3, the FP64 pipe 34 %, issue 49 %): per position of a warp 32 passes for the copies of a 3D
-// record, 32 to read it and one for each shuffle or slot.  The slots go through shared memory,
-// three passes in place of eight shuffles, and records are read 16 bytes at a time: 128^3 pair
-// pass 2.70 -> 2.51 ms FP64, 2.12 -> 2.06 mixed; 512 2D boxes, FP64, 2.26 -> 2.17.  With the 32-byte
-// float 2D records the slots cost more than two shuffles (512 boxes 1.87 -> 1.91 ms).
+// What bounds the FP64 3D pass is the load/store pipe all of this goes through (81 % busy at 96^3,
+// the FP64 pipe 37 %, issue 51 %): per position of a warp 32 passes for the copies of a record, 28 to
+// read it and one for each shuffle or slot.  (FP64 2D, where the general pair term's chains are
+// waited for: 65 %, 35 % and 54 %.)  The slots go through shared memory, three passes in place of
+// eight shuffles, and records are read 16 bytes at a time: 128^3 pair pass 2.70 -> 2.51 ms FP64,
+// 2.12 -> 2.06 mixed; 512 2D boxes, FP64, 2.26 -> 2.17.  With the 32-byte float 2D records the slots
+// cost more than two shuffles (512 boxes 1.87 -> 1.91 ms).
 //
 // Launch shape of the pair pass per precision and dimension, as measured on B200.  Every pass
 // evaluates one list position per step: with the fluid-fluid form of that walk, evaluating two

@@ -59,7 +59,7 @@ static_assert(NPARAM == SPH_MLP_NPARAMS, "parameter count");
 // cycles), and the weights each tile reads from L2 (256 KB).  Measured there, prediction by
 // all heads: 2.29 ms with a kernel per layer, the activations in memory between them and 1024
 // samples per pass, 0.18 ms so.  A training step (5 heads, batch 1024): 373 us in 15 launches,
-// 115 us in 5.
+// 107 us in 5.
 constexpr int kNetThreads = 512;
 constexpr int kNetA = tc::kTileM * HID * 2;       // bytes of the activations
 constexpr int kNetChunkA = tc::kTileM * tc::kChunkK * 2;
